@@ -284,8 +284,8 @@ __device__ __forceinline__ void src_to_prim(const StageArgs& A, const RowSrc<R>&
                      cs);
     }
   }
-  u = flipx ? -u : u;
-  v = s.flipy ? -v : v;
+  u = flipx ? rneg(u) : u;
+  v = s.flipy ? rneg(v) : v;
   if (xmode == 1) outlet_ghost<R>(g, R(A.bc_p), r, u, v, p);
   out[0] = r;
   out[1] = u;
@@ -481,7 +481,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, const FluxConsts<
         if constexpr (Prec<R>::kind == 0) {
           double u, v, p, cs;
           prim_from_cons(A.gamma, A.gamma - 1.0, un[0], un[1], un[2], un[3], u, v, p, cs);
-          double d = div_rn(A.cfl, div_rn(fabs(u) + cs, cg.dx) + div_rn(fabs(v) + cs, cg.dy));
+          double d = div_rn(A.cfl, div_rn(rabs(u) + cs, cg.dx) + div_rn(rabs(v) + cs, cg.dy));
           if (d_less(d, dt_loc)) dt_loc = d;
           if (d_isnan(un[0]) || d_isnan(u) || d_isnan(v) || d_isnan(p)) st_loc |= ST_NAN;
           if (lt0(un[0])) st_loc |= ST_NEG_DENSITY;
