@@ -56,6 +56,13 @@ static __device__ __noinline__ double mul_rn(double a, double b) {
   return ok ? intdiv::double_of(r) : mul_hw(a, b);
 }
 
+// RN(a / b) with the part that depends on b alone given (intdiv::recip62 of b's bits)
+static __device__ __noinline__ double quot_rn(double a, double b, uint64_t y62) {
+  bool ok;
+  const uint64_t q = intdiv::quot_bits(intdiv::bits_of(a), intdiv::bits_of(b), y62, ok);
+  return ok ? intdiv::double_of(q) : div_hw(a, b);
+}
+
 enum { FLUX_AUSMPW = 0, FLUX_SLAU = 1, FLUX_SLAU2 = 2, FLUX_SD_SLAU = 3, FLUX_SD_SLAU2 = 4,
        FLUX_ROE = 5, FLUX_AUSM_UP = 6, FLUX_HLLC = 7, FLUX_M_AUSMPW = 8 };
 enum { LIM_MINMOD = 0, LIM_SUPERBEE = 1, LIM_VANLEER = 2, LIM_MLP3 = 3, LIM_MLP5 = 4 };
@@ -89,9 +96,34 @@ template <> struct Num<double> {
     if ((intdiv::bits_of(a) << 1) == 0ULL) return a;
     return sqrt_rn(a);
   }
-  // a * b on the integer pipe (mul_rn)
+#ifdef CATO_F64_MUL_INT
   static __device__ __forceinline__ double mul(double a, double b) { return mul_rn(a, b); }
+#else
+  static __device__ __forceinline__ double mul(double a, double b) { return a * b; }
+#endif
 };
+
+// A divisor of several quotients: div_by(a, Rcp(b)) is Num<R>::div(a, b).  FP64 shares the
+// divisor's reciprocal (a third of a division's ~120 instructions).
+template <typename R> struct Rcp {
+  R b;
+  __device__ __forceinline__ explicit Rcp(R x) : b(x) {}
+};
+template <> struct Rcp<double> {
+  double b;
+  uint64_t y;
+  __device__ __forceinline__ explicit Rcp(double x)
+      : b(x), y(intdiv::recip62(intdiv::bits_of(x))) {}
+  // a divisor whose reciprocal is known
+  __device__ __forceinline__ Rcp(double x, uint64_t y62) : b(x), y(y62) {}
+};
+template <typename R> __device__ __forceinline__ R div_by(R a, const Rcp<R>& c);
+template <> __device__ __forceinline__ double div_by<double>(double a, const Rcp<double>& c) {
+  const uint64_t ua = intdiv::bits_of(a), ub = intdiv::bits_of(c.b);
+  if ((ua << 1) == 0ULL && (ub << 1) != 0ULL && ((ub >> 52) & 0x7ffULL) != 0x7ffULL)
+    return intdiv::double_of((ua ^ ub) & 0x8000000000000000ULL);
+  return quot_rn(a, c.b, c.y);
+}
 
 template <> struct Num<float> {
   static constexpr float eps = 2.220446049250313080847263336181640625e-16f;
@@ -108,6 +140,13 @@ template <> struct Num<df> {
   static __device__ __forceinline__ df sqrt(df a) { return df_sqrt(a); }
   static __device__ __forceinline__ df mul(df a, df b) { return a * b; }
 };
+
+template <> __device__ __forceinline__ float div_by<float>(float a, const Rcp<float>& c) {
+  return Num<float>::div(a, c.b);
+}
+template <> __device__ __forceinline__ df div_by<df>(df a, const Rcp<df>& c) {
+  return df_div(a, c.b);
+}
 
 // FP64: the reference's MAX/MIN as compare-and-select (identical signed-zero behaviour to the
 // CPU restatement).  FP32 (mixed path): single-instruction min/max.
@@ -211,6 +250,21 @@ template <> __device__ __forceinline__ double eighth<double>(double x) {
 }
 template <> __device__ __forceinline__ double twice<double>(double x) { return intdiv::scale_up1(x); }
 
+// a / twice(b) by the reciprocal of b.  FP64: half the quotient, exactly, unless that leaves the
+// normal range.
+template <typename R> __device__ __forceinline__ R div_by_twice(R a, const Rcp<R>& c) {
+  return Num<R>::div(a, twice(c.b));
+}
+template <>
+__device__ __forceinline__ double div_by_twice<double>(double a, const Rcp<double>& c) {
+  const double q = div_by(a, c);
+  const uint64_t u = intdiv::bits_of(q);
+  const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
+  if (e > 1u && e < 2046u && (mag_bits(c.b) >> 52) < 2046u)
+    return intdiv::double_of(u - (1ULL << 52));
+  return Num<double>::div(a, twice(c.b));
+}
+
 // a + b * R(0): the reference's products with the zero component of an axis-aligned unit normal.
 // FP64 on the integer pipe: b * 0 is the zero with the sign of b when b is finite (NaN
 // otherwise), and a + (+-0) is a unless a is a zero, where -0 results only from -0 + -0.
@@ -238,7 +292,10 @@ __device__ __forceinline__ double add_zeros<double>(double x, double a, double b
 // |x| < c for c > 0 without an FP compare: bit patterns of non-negative IEEE values order like
 // unsigned integers and NaN compares false, as the reference's ABS(x) < c does.
 __device__ __forceinline__ bool abs_lt(double x, double c) {
-  return mag_bits(x) < (uint64_t)__double_as_longlong(c);
+  const uint64_t cb = (uint64_t)__double_as_longlong(c);
+  if ((uint32_t)cb == 0u)  // c is a constant: for a power of two the high word decides
+    return (uint32_t)(mag_bits(x) >> 32) < (uint32_t)(cb >> 32);
+  return mag_bits(x) < cb;
 }
 __device__ __forceinline__ bool abs_lt(float x, float c) { return fabsf(x) < c; }
 __device__ __forceinline__ bool abs_lt(df x, df c) { return df_abs(x) < c; }
@@ -322,9 +379,10 @@ __device__ __forceinline__ void prim_from_cons(double g, double g1, double r, do
                                                double rv, double rE, double& u, double& v,
                                                double& p, double& cs) {
   const double EPS = Num<double>::eps, TINY = Num<double>::tiny;
-  u = abs_lt(ru, TINY) ? 0.0 : div_rn(ru, r);
-  v = abs_lt(rv, TINY) ? 0.0 : div_rn(rv, r);
-  double e = abs_lt(rE, TINY) ? 0.0 : div_rn(rE, r);
+  const uint64_t ry = intdiv::recip62(intdiv::bits_of(r));  // shared by the four quotients
+  u = abs_lt(ru, TINY) ? 0.0 : quot_rn(ru, r, ry);
+  v = abs_lt(rv, TINY) ? 0.0 : quot_rn(rv, r, ry);
+  double e = abs_lt(rE, TINY) ? 0.0 : quot_rn(rE, r, ry);
   // explicitly rounded: identical in translation units built with FMA contraction
   double s = __dadd_rn(__dmul_rn(u, u), __dmul_rn(v, v));
   if (abs_lt(s, EPS)) s = 0.0;
@@ -332,7 +390,7 @@ __device__ __forceinline__ void prim_from_cons(double g, double g1, double r, do
   double dd = e - h;
   if (abs_lt(dd, EPS)) dd = 0.0;
   p = (r * g1) * dd;
-  double pr = abs_lt(p, TINY) ? 0.0 : div_rn(p, r);
+  double pr = abs_lt(p, TINY) ? 0.0 : quot_rn(p, r, ry);
   cs = Num<double>::sqrt(pr * g);
   // mach_u = u / cs, mach_v = v / cs, then |mach| < 1e-13 zeroes the velocity
   if (mach_below_1e13(u, cs)) u = 0.0;  // each test reads only its own component and cs
@@ -781,7 +839,15 @@ template <typename R> struct FluxConsts {
   R gamma, g_over_gm1, gm1, two_gm1_over_gp1, gamma_factor, hllc_gf, harten_delta;
   R ausm_beta, ausm_kp, ausm_ku, ausm_sigma;
   int low_mach_fix, harten;
+  uint64_t gm1_y62;  // FP64: recip62 of gm1
 };
+// gamma - 1 as a divisor
+template <typename R> __device__ __forceinline__ Rcp<R> gm1_of(const FluxConsts<R>& K) {
+  return Rcp<R>(K.gm1);
+}
+template <> __device__ __forceinline__ Rcp<double> gm1_of<double>(const FluxConsts<double>& K) {
+  return Rcp<double>(K.gm1, K.gm1_y62);
+}
 
 // The FP64 constants carried to another compute type (host side).
 template <typename R> inline FluxConsts<R> convert_consts(const FluxConsts<double>& K) {
@@ -824,6 +890,41 @@ template <typename R> __device__ __forceinline__ R aw_m_minus(R M) {
   return -quarter((M - R(1)) * (M - R(1)));
 }
 
+// Whether the Mach number sqrt(u^2 + v^2) / sqrt(g p / rho) is certainly at least 0.1 (LOW_MACH
+// takes those below): from FP32 estimates with a margin of 1 %, far above their error and the
+// exact value's.  Then the two quotients and two square roots that only the test reads are left
+// out.  The FP32 path forms the numbers themselves.
+template <typename R>
+__device__ __forceinline__ bool above_low_mach(R, R, R, R, R) { return false; }
+template <>
+__device__ __forceinline__ bool above_low_mach<double>(double u, double v, double g, double p,
+                                                       double r) {
+  // finite values d2f_fast takes; p and r not negative
+  const uint32_t most = max(max((uint32_t)(mag_bits(u) >> 32), (uint32_t)(mag_bits(v) >> 32)),
+                            max((uint32_t)(intdiv::bits_of(p) >> 32),
+                                (uint32_t)(intdiv::bits_of(r) >> 32)));
+  if (most >= 0x42000000u) return false;  // 2^33
+  const float uf = d2f_fast(u), vf = d2f_fast(v), pf = d2f_fast(p), rf = d2f_fast(r);
+  const float q2 = (uf * uf + vf * vf) * rf, lim = 0.0102f * (d2f_fast(g) * pf);
+  return rf > 1e-15f && pf > 1e-15f && q2 > lim && q2 < 1e15f;
+}
+template <>
+__device__ __forceinline__ bool above_low_mach<df>(df u, df v, df g, df p, df r) {
+  const float q2 = (u.hi * u.hi + v.hi * v.hi) * r.hi, lim = 0.0102f * (g.hi * p.hi);
+  return r.hi > 1e-15f && p.hi > 1e-15f && q2 > lim && q2 < 1e15f;
+}
+// min(a / b, b / a).  FP64: of two positive finite operands only the quotient of the smaller by
+// the larger can be the minimum (rounding is monotone and 1 is exact).
+template <typename R> __device__ __forceinline__ R least_ratio(R a, R b) {
+  return rmin(Num<R>::div(a, b), Num<R>::div(b, a));
+}
+template <> __device__ __forceinline__ double least_ratio<double>(double a, double b) {
+  const uint64_t ua = intdiv::bits_of(a), ub = intdiv::bits_of(b);
+  if (ua - 1ULL < kInfBits - 1ULL && ub - 1ULL < kInfBits - 1ULL)
+    return ua < ub ? Num<double>::div(a, b) : Num<double>::div(b, a);
+  return rmin(Num<double>::div(a, b), Num<double>::div(b, a));
+}
+
 // AUSMPW+, ausmpw_plus_solver.fypp:336-459.  pc[4] = p1_L, p1_R, p2_L, p2_R (:430-442).
 template <typename R, int DIR>
 __device__ __forceinline__ void flux_ausmpw(const FluxConsts<R>& K, const Prim<R>& A,
@@ -833,34 +934,39 @@ __device__ __forceinline__ void flux_ausmpw(const FluxConsts<R>& K, const Prim<R
   R rho_R = B.r, u_RHS = B.u, v_RHS = B.v, p_R = B.p;
   const R U_L = DIR == 0 ? u_LHS : v_LHS, U_R = DIR == 0 ? u_RHS : v_RHS;
   const R V_L = DIR == 0 ? v_LHS : u_LHS, V_R = DIR == 0 ? v_RHS : u_RHS;
-  R cs_L = Num<R>::sqrt(Num<R>::div(g * p_L, rho_L));
-  R cs_R = Num<R>::sqrt(Num<R>::div(g * p_R, rho_R));
-  R M_LHS = Num<R>::div(Num<R>::sqrt(u_LHS * u_LHS + v_LHS * v_LHS), cs_L);
-  R M_RHS = Num<R>::div(Num<R>::sqrt(u_RHS * u_RHS + v_RHS * v_RHS), cs_R);
-  if (K.low_mach_fix && (abs_lt(M_LHS, R(0.1)) || abs_lt(M_RHS, R(0.1)))) {  // LOW_MACH
-    R f_M = rmin(R(1), rmax(M_LHS, M_RHS));
-    R uLf = half(u_LHS + u_RHS) + half(f_M) * (u_LHS - u_RHS);
-    R uRf = half(u_LHS + u_RHS) - half(f_M) * (u_LHS - u_RHS);
-    R vLf = half(v_LHS + v_RHS) + half(f_M) * (v_LHS - v_RHS);
-    R vRf = half(v_LHS + v_RHS) - half(f_M) * (v_LHS - v_RHS);
-    u_LHS = uLf; u_RHS = uRf; v_LHS = vLf; v_RHS = vRf;
+  const Rcp<R> rc_L(rho_L), rc_R(rho_R);
+  if (K.low_mach_fix && !(above_low_mach(u_LHS, v_LHS, g, p_L, rho_L) &&
+                          above_low_mach(u_RHS, v_RHS, g, p_R, rho_R))) {
+    R cs_L = Num<R>::sqrt(div_by(g * p_L, rc_L));
+    R cs_R = Num<R>::sqrt(div_by(g * p_R, rc_R));
+    R M_LHS = Num<R>::div(Num<R>::sqrt(u_LHS * u_LHS + v_LHS * v_LHS), cs_L);
+    R M_RHS = Num<R>::div(Num<R>::sqrt(u_RHS * u_RHS + v_RHS * v_RHS), cs_R);
+    if (abs_lt(M_LHS, R(0.1)) || abs_lt(M_RHS, R(0.1))) {  // LOW_MACH
+      R f_M = rmin(R(1), rmax(M_LHS, M_RHS));
+      R uLf = half(u_LHS + u_RHS) + half(f_M) * (u_LHS - u_RHS);
+      R uRf = half(u_LHS + u_RHS) - half(f_M) * (u_LHS - u_RHS);
+      R vLf = half(v_LHS + v_RHS) + half(f_M) * (v_LHS - v_RHS);
+      R vRf = half(v_LHS + v_RHS) - half(f_M) * (v_LHS - v_RHS);
+      u_LHS = uLf; u_RHS = uRf; v_LHS = vLf; v_RHS = vRf;
+    }
   }
   const R gg = R(K.g_over_gm1);
-  R H_L = gg * Num<R>::div(p_L, rho_L) + half(u_LHS * u_LHS + v_LHS * v_LHS);
-  R H_R = gg * Num<R>::div(p_R, rho_R) + half(u_RHS * u_RHS + v_RHS * v_RHS);
+  R H_L = gg * div_by(p_L, rc_L) + half(u_LHS * u_LHS + v_LHS * v_LHS);
+  R H_R = gg * div_by(p_R, rc_R) + half(u_RHS * u_RHS + v_RHS * v_RHS);
   R H_normal = rmin(H_L - half(V_L * V_L), H_R - half(V_R * V_R));
   R c_s = Num<R>::sqrt(R(K.two_gm1_over_gp1) * H_normal);
   R c_half;
   if (lt0(half(U_L + U_R))) c_half = Num<R>::div(c_s * c_s, rmax(rabs(U_R), c_s));
   else c_half = Num<R>::div(c_s * c_s, rmax(rabs(U_L), c_s));
-  R M_L = Num<R>::div(U_L, c_half);
-  R M_R = Num<R>::div(U_R, c_half);
+  const Rcp<R> rc_c(c_half);
+  R M_L = div_by(U_L, rc_c);
+  R M_R = div_by(U_R, rc_c);
   R M_L_plus = aw_m_plus(M_L);
   R M_R_minus = aw_m_minus(M_R);
   R P_R_minus = aw_p_minus(M_R);
   R P_L_plus = aw_p_plus(M_L);
   R p_s = p_L * P_L_plus + p_R * P_R_minus;
-  R mt = rmin(Num<R>::div(p_L, p_R), Num<R>::div(p_R, p_L));
+  R mt = least_ratio(p_L, p_R);
   R w = R(1) - mt * mt * mt;
   R f_L, f_R;
   if (abs_lt(p_s, Num<R>::tiny)) {
@@ -869,8 +975,9 @@ __device__ __forceinline__ void flux_ausmpw(const FluxConsts<R>& K, const Prim<R
   } else {
     R t = rmin(R(1), Num<R>::div(rmin(rmin(rmin(pc[0], pc[1]), pc[2]), pc[3]), rmin(p_L, p_R)));
     R min_term = t * t;
-    f_L = (Num<R>::div(p_L, p_s) - R(1)) * min_term;
-    f_R = (Num<R>::div(p_R, p_s) - R(1)) * min_term;
+    const Rcp<R> rc_s(p_s);
+    f_L = (div_by(p_L, rc_s) - R(1)) * min_term;
+    f_R = (div_by(p_R, rc_s) - R(1)) * min_term;
   }
   R Mb_L, Mb_R;
   if (lt0(M_L_plus + M_R_minus)) {
@@ -934,34 +1041,39 @@ __device__ __forceinline__ void flux_mausmpw(const FluxConsts<R>& K, const Prim<
   R rho_R = B.r, u_RHS = B.u, v_RHS = B.v, p_R = B.p;
   const R U_L = DIR == 0 ? u_LHS : v_LHS, U_R = DIR == 0 ? u_RHS : v_RHS;
   const R V_L = DIR == 0 ? v_LHS : u_LHS, V_R = DIR == 0 ? v_RHS : u_RHS;
-  R cs_L = Num<R>::sqrt(Num<R>::div(g * p_L, rho_L));
-  R cs_R = Num<R>::sqrt(Num<R>::div(g * p_R, rho_R));
-  R M_LHS = Num<R>::div(Num<R>::sqrt(u_LHS * u_LHS + v_LHS * v_LHS), cs_L);
-  R M_RHS = Num<R>::div(Num<R>::sqrt(u_RHS * u_RHS + v_RHS * v_RHS), cs_R);
-  if (K.low_mach_fix && (abs_lt(M_LHS, R(0.1)) || abs_lt(M_RHS, R(0.1)))) {  // LOW_MACH
-    R f_M = rmin(R(1), rmax(M_LHS, M_RHS));
-    R uLf = half(u_LHS + u_RHS) + half(f_M) * (u_LHS - u_RHS);
-    R uRf = half(u_LHS + u_RHS) - half(f_M) * (u_LHS - u_RHS);
-    R vLf = half(v_LHS + v_RHS) + half(f_M) * (v_LHS - v_RHS);
-    R vRf = half(v_LHS + v_RHS) - half(f_M) * (v_LHS - v_RHS);
-    u_LHS = uLf; u_RHS = uRf; v_LHS = vLf; v_RHS = vRf;
+  const Rcp<R> rc_L(rho_L), rc_R(rho_R);
+  if (K.low_mach_fix && !(above_low_mach(u_LHS, v_LHS, g, p_L, rho_L) &&
+                          above_low_mach(u_RHS, v_RHS, g, p_R, rho_R))) {
+    R cs_L = Num<R>::sqrt(div_by(g * p_L, rc_L));
+    R cs_R = Num<R>::sqrt(div_by(g * p_R, rc_R));
+    R M_LHS = Num<R>::div(Num<R>::sqrt(u_LHS * u_LHS + v_LHS * v_LHS), cs_L);
+    R M_RHS = Num<R>::div(Num<R>::sqrt(u_RHS * u_RHS + v_RHS * v_RHS), cs_R);
+    if (abs_lt(M_LHS, R(0.1)) || abs_lt(M_RHS, R(0.1))) {  // LOW_MACH
+      R f_M = rmin(R(1), rmax(M_LHS, M_RHS));
+      R uLf = half(u_LHS + u_RHS) + half(f_M) * (u_LHS - u_RHS);
+      R uRf = half(u_LHS + u_RHS) - half(f_M) * (u_LHS - u_RHS);
+      R vLf = half(v_LHS + v_RHS) + half(f_M) * (v_LHS - v_RHS);
+      R vRf = half(v_LHS + v_RHS) - half(f_M) * (v_LHS - v_RHS);
+      u_LHS = uLf; u_RHS = uRf; v_LHS = vLf; v_RHS = vRf;
+    }
   }
   const R gg = R(K.g_over_gm1);
-  R H_L = gg * Num<R>::div(p_L, rho_L) + half(u_LHS * u_LHS + v_LHS * v_LHS);
-  R H_R = gg * Num<R>::div(p_R, rho_R) + half(u_RHS * u_RHS + v_RHS * v_RHS);
+  R H_L = gg * div_by(p_L, rc_L) + half(u_LHS * u_LHS + v_LHS * v_LHS);
+  R H_R = gg * div_by(p_R, rc_R) + half(u_RHS * u_RHS + v_RHS * v_RHS);
   R H_normal = rmin(H_L - half(V_L * V_L), H_R - half(V_R * V_R));
   R c_s = Num<R>::sqrt(R(K.two_gm1_over_gp1) * H_normal);
   R c_half;
   if (lt0(half(U_L + U_R))) c_half = Num<R>::div(c_s * c_s, rmax(rabs(U_R), c_s));
   else c_half = Num<R>::div(c_s * c_s, rmax(rabs(U_L), c_s));
-  R M_L = Num<R>::div(U_L, c_half);
-  R M_R = Num<R>::div(U_R, c_half);
+  const Rcp<R> rc_c(c_half);
+  R M_L = div_by(U_L, rc_c);
+  R M_R = div_by(U_R, rc_c);
   R M_L_plus = aw_m_plus(M_L);
   R M_R_minus = aw_m_minus(M_R);
   R P_R_minus = mausm_p_minus(M_R);
   R P_L_plus = mausm_p_plus(M_L);
   R p_s = p_L * P_L_plus + p_R * P_R_minus;
-  R mt = rmin(Num<R>::div(p_L, p_R), Num<R>::div(p_R, p_L));
+  R mt = least_ratio(p_L, p_R);
   R w = R(1) - (mt * mt * mt);
   R f_L, f_R;
   if (abs_lt(p_s, Num<R>::tiny)) {
@@ -971,10 +1083,11 @@ __device__ __forceinline__ void flux_mausmpw(const FluxConsts<R>& K, const Prim<
     R t = rmin(R(1), Num<R>::div(rmin(rmin(rmin(pc[0], pc[1]), pc[2]), pc[3]), rmin(p_L, p_R)));
     R min_term = t * t;
     if (abs_lt(R(1) - min_term, CUT)) min_term = R(1);
-    R fl = Num<R>::div(p_L, p_s) - R(1);
+    const Rcp<R> rc_s(p_s);
+    R fl = div_by(p_L, rc_s) - R(1);
     if (abs_lt(fl, CUT)) fl = R(0);
     f_L = fl * min_term;
-    R fr = Num<R>::div(p_R, p_s) - R(1);
+    R fr = div_by(p_R, rc_s) - R(1);
     if (abs_lt(fr, CUT)) fr = R(0);
     f_R = fr * min_term;
   }
@@ -1021,15 +1134,16 @@ __device__ __forceinline__ void flux_slau(const FluxConsts<R>& K, const Prim<R>&
   // V_n = u*n_x + v*n_y with an exact unit normal
   R Vp = DIR == 0 ? add_mul0(u_L, v_L) : add_mul0(v_L, u_L);
   R Vm = DIR == 0 ? add_mul0(u_R, v_R) : add_mul0(v_R, u_R);
-  R c_plus = Num<R>::sqrt(Num<R>::div(g * p_L, rho_L));
-  R c_minus = Num<R>::sqrt(Num<R>::div(g * p_R, rho_R));
+  const Rcp<R> rc_L(rho_L), rc_R(rho_R);
+  R c_plus = Num<R>::sqrt(div_by(g * p_L, rc_L));
+  R c_minus = Num<R>::sqrt(div_by(g * p_R, rc_R));
   R c_bar = half(c_plus + c_minus);
+  const Rcp<R> rc_c(c_bar);
   R V_n_bar = Num<R>::div(rho_L * rabs(Vp) + rho_R * rabs(Vm), rho_L + rho_R);
   R vel2 = half(u_L * u_L + v_L * v_L + u_R * u_R + v_R * v_R);
-  R M_hat = rmin(R(1), Num<R>::div(Num<R>::sqrt(vel2), c_bar));
-  R M_bar = Num<R>::div(V_n_bar, c_bar);
-  R M_plus = Num<R>::div(Vp, c_bar);
-  R M_minus = Num<R>::div(Vm, c_bar);
+  R M_hat = rmin(R(1), div_by(Num<R>::sqrt(vel2), rc_c));
+  R M_plus = div_by(Vp, rc_c);
+  R M_minus = div_by(Vm, rc_c);
   R Chi = (R(1) - M_hat) * (R(1) - M_hat);
   R p_bar = half(p_L + p_R);
   R rho_bar = half(rho_L + rho_R);
@@ -1060,7 +1174,7 @@ __device__ __forceinline__ void flux_slau(const FluxConsts<R>& K, const Prim<R>&
     R dp_max = rmax(rabs(delta_p), m6);
     R ratio = Num<R>::div(Num<R>::div(C_SD1 * rabs(delta_p), p_bar) + C_SD1,
                           Num<R>::div(dp_max, p_bar) + C_SD1);
-    theta = rmin(R(1), ratio * ratio) * rmax(R(0), R(1) - rabs(M_bar));
+    theta = rmin(R(1), ratio * ratio) * rmax(R(0), R(1) - rabs(div_by(V_n_bar, rc_c)));
   }
   R p_tilde;
   if (VARIANT == FLUX_SLAU || VARIANT == FLUX_SD_SLAU)
@@ -1071,12 +1185,12 @@ __device__ __forceinline__ void flux_slau(const FluxConsts<R>& K, const Prim<R>&
   R gg = -(rmax(rmin(M_plus, R(0)), R(-1)) * rmin(rmax(M_minus, R(0)), R(1)));
   R diss = (VARIANT == FLUX_SLAU || VARIANT == FLUX_SLAU2) ? Chi : theta;
   R mf = half((rho_L * Vp) + (rho_R * Vm) - rabs(V_n_bar) * delta_rho) * (R(1) - gg) -
-         (Num<R>::div(diss, twice(c_bar)) * delta_p);
+         (div_by_twice(diss, rc_c) * delta_p);
   R mL = half(mf + rabs(mf));
   R mR = half(mf - rabs(mf));
   const R gq = R(K.g_over_gm1);
-  R H_L = gq * Num<R>::div(p_L, rho_L) + half(u_L * u_L + v_L * v_L);
-  R H_R = gq * Num<R>::div(p_R, rho_R) + half(u_R * u_R + v_R * v_R);
+  R H_L = gq * div_by(p_L, rc_L) + half(u_L * u_L + v_L * v_L);
+  R H_R = gq * div_by(p_R, rc_R) + half(u_R * u_R + v_R * v_R);
   F[0] = mL + mR;
   if (DIR == 0) {
     F[1] = (mL * u_L) + (mR * u_R) + p_tilde;
@@ -1086,6 +1200,53 @@ __device__ __forceinline__ void flux_slau(const FluxConsts<R>& K, const Prim<R>&
     F[2] = (mL * v_L) + (mR * v_R) + p_tilde;
   }
   F[3] = (mL * H_L) + (mR * H_R);
+}
+
+// One pair of the Roe pressure sensor, |b - a| / (min(b, a) + 1e-16) >= 1 (or NaN).  With
+// 0 < min <= max < 2 min the difference is below min, so the quotient is below 1 (FP64: the
+// difference is exact by Sterbenz's lemma and the rounded quotient of x < y is below 1; the
+// other types keep a margin for their rounding): five divisions per edge are left out.
+template <typename R> __device__ __forceinline__ bool roe_sensor_slow(R a, R b) {
+  const R ratio = Num<R>::div(rabs(b - a), rmin(b, a) + R(1e-16));
+  return !lt(ratio, R(1));
+}
+static __device__ __noinline__ bool roe_sensor_f64(double a, double b) {
+  return roe_sensor_slow<double>(a, b);
+}
+template <typename R> __device__ __forceinline__ bool roe_sensor(R a, R b);
+template <> __device__ __forceinline__ bool roe_sensor<double>(double a, double b) {
+  const uint64_t ua = intdiv::bits_of(a), ub = intdiv::bits_of(b);
+  const uint64_t lo = ua < ub ? ua : ub, hi = ua < ub ? ub : ua;
+  // positive (the smaller pattern is normal), the larger finite and below twice the smaller
+  if (lo - 0x0010000000000000ULL < 0x7fd0000000000000ULL && hi < lo + (1ULL << 52)) return false;
+  return roe_sensor_f64(a, b);
+}
+template <> __device__ __forceinline__ bool roe_sensor<float>(float a, float b) {
+  const float lo = fminf(a, b), hi = fmaxf(a, b);
+  if (lo > 1e-25f && hi < 1.99f * lo) return false;
+  return roe_sensor_slow<float>(a, b);
+}
+template <> __device__ __forceinline__ bool roe_sensor<df>(df a, df b) {
+  const float lo = fminf(a.hi, b.hi), hi = fmaxf(a.hi, b.hi);
+  if (lo > 1e-25f && hi < 1.99f * lo) return false;
+  return roe_sensor_slow<df>(a, b);
+}
+// whether the correction of a quiet sensor, 0 rav cav (...), is a zero that leaves F1 and F2 alone
+__device__ __forceinline__ bool roe_quiet(double F1, double F2, double rav, double cav, double du,
+                                          double dut, double cl, double cr) {
+  // non-zero fluxes; finite factors; sound speeds positive, so that their ratio is finite
+  return mag_bits(F1) != 0ULL && mag_bits(F2) != 0ULL && d_finite(rav) && d_finite(cav) &&
+         d_finite(du) && d_finite(dut) && intdiv::bits_of(cl) - 1ULL < kInfBits - 1ULL &&
+         intdiv::bits_of(cr) - 1ULL < kInfBits - 1ULL;
+}
+__device__ __forceinline__ bool roe_quiet(float F1, float F2, float rav, float cav, float du,
+                                          float dut, float cl, float cr) {
+  return F1 != 0.0f && F2 != 0.0f && fminf(cl, cr) > 0.0f &&
+         fabsf(rav) + fabsf(cav) + fabsf(du) + fabsf(dut) + cl + cr < 1e30f;
+}
+__device__ __forceinline__ bool roe_quiet(df F1, df F2, df rav, df cav, df du, df dut, df cl,
+                                          df cr) {
+  return roe_quiet(F1.hi, F2.hi, rav.hi, cav.hi, du.hi, dut.hi, cl.hi, cr.hi);
 }
 
 // Roe with the reference's wave-speed bounds and pressure-sensor shear correction,
@@ -1101,9 +1262,10 @@ __device__ __forceinline__ void flux_roe(const FluxConsts<R>& K, const Prim<R>& 
   R rr = rabs(B.r), ur = B.u, vr = B.v, pr = rabs(B.p);
   const R gq = R(K.g_over_gm1);
   R rav = Num<R>::sqrt(m(rl, rr));
-  R q_pl = Num<R>::div(pl, rl), q_rav = Num<R>::div(rav, rl), q_gpl = Num<R>::div(m(g, pl), rl);
+  const Rcp<R> rc_l(rl), rc_r(rr);
+  R q_pl = div_by(pl, rc_l), q_rav = div_by(rav, rc_l), q_gpl = div_by(m(g, pl), rc_l);
   R hl = m(gq, q_pl) + half(m(ul, ul) + m(vl, vl));
-  R hr = m(gq, Num<R>::div(pr, rr)) + half(m(ur, ur) + m(vr, vr));
+  R hr = m(gq, div_by(pr, rc_r)) + half(m(ur, ur) + m(vr, vr));
   R gam1 = R(K.gm1);
   R dd = q_rav;
   R dd1 = Num<R>::div(R(1), R(1) + dd);
@@ -1118,7 +1280,7 @@ __device__ __forceinline__ void flux_roe(const FluxConsts<R>& K, const Prim<R>& 
   R uv = dotn(uav, vav);
   R du = dotn(ur - ul, vr - vl);
   R du_trans = DIR == 0 ? add_mul0(vr - vl, rneg(ur - ul)) : add_mul0(rneg(ur - ul), vr - vl);
-  R cs_R = Num<R>::sqrt(Num<R>::div(m(g, pr), rr));
+  R cs_R = Num<R>::sqrt(div_by(m(g, pr), rc_r));
   R cs_L = Num<R>::sqrt(q_gpl);
   R h1 = rabs(rmin(uv - cav, dotn(ul, vl) - cs_L));
   R h2 = rabs(uv);
@@ -1131,11 +1293,11 @@ __device__ __forceinline__ void flux_roe(const FluxConsts<R>& K, const Prim<R>& 
     e4 = lt(delta, h4) ? h4 : Num<R>::div(half(m(h4, h4) + m(delta, delta)), delta);
   }
   h1 = m(m(rav, cav), du);
-  h2 = Num<R>::div(m(e1, pr - pl - h1), twice(c2a));
-  R h3 = m(e2, rr - rl - Num<R>::div(pr - pl, c2a));
+  const Rcp<R> rc_c2(c2a);
+  h2 = div_by_twice(m(e1, pr - pl - h1), rc_c2);
+  R h3 = m(e2, rr - rl - div_by(pr - pl, rc_c2));
   h4 = m(e2, rav);
-  R h5 = Num<R>::div(m(e4, pr - pl + h1), twice(c2a));
-  R psi = Num<R>::div(rabs(cs_R - cs_L), rmax(cs_R, cs_L));
+  R h5 = div_by_twice(m(e4, pr - pl + h1), rc_c2);
   // the normal-direction terms carry the exact 1, the tangential ones the exact 0
   auto on = [](bool axis, R a, R b) { return axis ? a + b : add_mul0(a, b); };
   R FR0 = m(rr, uv), FR1 = on(DIR == 0, m(m(rr, ur), uv), pr), FR2 = on(DIR == 1, m(m(rr, vr), uv), pr);
@@ -1153,12 +1315,14 @@ __device__ __forceinline__ void flux_roe(const FluxConsts<R>& K, const Prim<R>& 
   F[1] = half(FR1 + FL1 - m1);
   F[2] = half(FR2 + FL2 - m2);
   F[3] = half(FR3 + FL3 - m3);
-  R fmax = R(0);
+  // the shear correction: nothing where the pressure sensor is quiet (a zero product leaves the
+  // flux as it is; roe_quiet: unless a zero's sign or a NaN would come of it)
+  bool fires = false;
 #pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    R ratio = Num<R>::div(rabs(fb[k] - fa[k]), rmin(fb[k], fa[k]) + R(1e-16));
-    fmax = rmax(fmax, lt(ratio, R(1)) ? R(0) : R(1));
-  }
+  for (int k = 0; k < 5; ++k) fires = fires || roe_sensor(fa[k], fb[k]);
+  if (!fires && roe_quiet(F[1], F[2], rav, cav, du, du_trans, cs_L, cs_R)) return;
+  const R fmax = fires ? R(1) : R(0);
+  R psi = Num<R>::div(rabs(cs_R - cs_L), rmax(cs_R, cs_L));
   // -(du_trans n_y) + psi du n_x and du_trans n_x + psi du n_y
   const R c1 = DIR == 0 ? add_mul0(m(psi, du), rneg(du_trans)) : add_mul0(rneg(du_trans), m(psi, du));
   const R c2 = DIR == 0 ? add_mul0(du_trans, m(psi, du)) : add_mul0(m(psi, du), du_trans);
@@ -1188,8 +1352,9 @@ __device__ __forceinline__ void flux_ausm_up(const FluxConsts<R>& K, const Prim<
   R a_circ_L = Num<R>::div(a_crit_L * a_crit_L, rmax(a_crit_L, vel_L));
   R a_circ_R = Num<R>::div(a_crit_R * a_crit_R, rmax(a_crit_R, -vel_R));
   R a_half = rmin(a_circ_L, a_circ_R);
-  R M_L = Num<R>::div(vel_L, a_half);
-  R M_R = Num<R>::div(vel_R, a_half);
+  const Rcp<R> rc_a(a_half);
+  R M_L = div_by(vel_L, rc_a);
+  R M_R = div_by(vel_R, rc_a);
   R M_bar_sq = half(M_L + M_R);  // as written at ausm_plus_solver.f90:585
   const R beta = R(K.ausm_beta);
   R M_plus = (abs_ge(M_L, R(1))) ? up_m1p(M_L) : up_m2p(M_L) * (R(1) - R(16) * beta * up_m2m(M_L));
@@ -1246,7 +1411,7 @@ __device__ __forceinline__ void flux_hllc(const FluxConsts<R>& K, const Prim<R>&
   else SR = qnR + m(cR, Num<R>::sqrt(R(1) + m(gf, Num<R>::div(p_star, B.p) - R(1))));
   // the total energy of the side the flux is taken from (only that one is needed)
   auto energy = [&](const Prim<R>& S) {
-    return Num<R>::div(S.p, R(K.gm1)) + m(half(S.r), m(S.u, S.u) + m(S.v, S.v));
+    return div_by(S.p, gm1_of(K)) + m(half(S.r), m(S.u, S.u) + m(S.v, S.v));
   };
   R S_star = Num<R>::div(B.p - A.p + m(m(A.r, qnL), SL - qnL) - m(m(B.r, qnR), SR - qnR),
                          m(A.r, SL - qnL) - m(B.r, SR - qnR));
@@ -1288,6 +1453,7 @@ constexpr int kNotPow2 = 1 << 20;
 struct Geom {
   double vol, l1, l2, l3, l4;  // volume, edge lengths (bottom, right, top, left)
   double dx, dy;               // min_dx / min_dy for the CFL step
+  uint64_t vol_y62;            // recip62 of vol (uniform grid)
   double inv_vol;              // 1/vol when vol is a power of two (x/vol == x*inv_vol exactly), else 0
   // base-2 exponents of l1..l4 and inv_vol when they are powers of two, else kNotPow2: the
   // products with them are exponent steps
@@ -1320,6 +1486,7 @@ __device__ __forceinline__ Geom cell_geom(const Geom& G, int i, int j) {
   c.vol = dx * dy - 0.0 * 0.0;
   c.dx = dx;
   c.dy = dy;
+  c.vol_y62 = intdiv::recip62(intdiv::bits_of(c.vol));
   c.inv_vol = 0.0;
   c.k1 = c.k2 = c.k3 = c.k4 = c.kinv = kNotPow2;
   return c;
@@ -1340,6 +1507,7 @@ inline Geom uniform_geom(double dx, double dy) {
   G.dy = dy;
   // a division by a power of two is the multiplication by its reciprocal, which is exactly
   // representable: both round the same real number (power-of-two grids, e.g. 4096^2 on [0,1]^2)
+  G.vol_y62 = intdiv::recip62(intdiv::bits_of(G.vol));
   int e = 0;
   const double m = std::frexp(G.vol, &e);
   G.inv_vol = (m == 0.5 && e > -1020 && e < 1020) ? 1.0 / G.vol : 0.0;
@@ -1370,36 +1538,34 @@ __device__ __forceinline__ double mul_pow2(double x, double p, int k) {
   return x * p;
 }
 
-__device__ __forceinline__ double divergence_fp64(double Fi, double Fim, double Fj, double Fjm,
-                                                  const Geom& G) {
+// one direction's difference: (F l - Fm lm), the fluxes scaled by the larger of them and 1
+__device__ __forceinline__ double scaled_difference(double F, double Fm, double l, int k, double lm,
+                                                    int km) {
   const double REL_TOL = 1e-14;
-  const double NEAR0 = 5.0 * Num<double>::tiny;  // near_zero, flux_solver.f90:461-474
-  double mi = rmax(rmax(rabs(Fi), rabs(Fim)), 1.0);
-  double mj = rmax(rmax(rabs(Fj), rabs(Fjm)), 1.0);
-  // x / 1.0 is exact: skip the division when the scale is 1
-  double a, b;
-  // (the scale is 1 or above; compares on the integer pipe, mi * REL_TOL = REL_TOL for mi = 1)
-  using N = Num<double>;
-  const long long ONE = 0x3ff0000000000000LL;
-  // products with the edge lengths: exponent steps when those are powers of two; x * 1.0 (the
-  // scale is 1) is x itself
-  if ((long long)intdiv::bits_of(mi) == ONE) {
-    a = mul_pow2(Fi, G.l2, G.k2) + (-mul_pow2(Fim, G.l4, G.k4));
+  const uint64_t ONE = 0x3ff0000000000000ULL;
+  // max(|F|, |Fm|, 1) by magnitude bits; with a NaN among them the scale and the result are NaN
+  uint64_t m = mag_bits(F), mm = mag_bits(Fm);
+  m = m > mm ? m : mm;
+  double a;
+  if (m <= ONE) {  // the scale is 1: x / 1 and x * 1 are x itself
+    a = mul_pow2(F, l, k) - mul_pow2(Fm, lm, km);
     if (abs_lt(a, REL_TOL)) a = 0.0;
-  } else {
-    a = (mul_pow2(N::div(Fi, mi), G.l2, G.k2) + (-mul_pow2(N::div(Fim, mi), G.l4, G.k4))) * mi;
-    if (abs_lt(a, mi * REL_TOL)) a = 0.0;
+    return a;
   }
-  if ((long long)intdiv::bits_of(mj) == ONE) {
-    b = mul_pow2(Fj, G.l3, G.k3) + (-mul_pow2(Fjm, G.l1, G.k1));
-    if (abs_lt(b, REL_TOL)) b = 0.0;
-  } else {
-    b = (mul_pow2(N::div(Fj, mj), G.l3, G.k3) + (-mul_pow2(N::div(Fjm, mj), G.l1, G.k1))) * mj;
-    if (abs_lt(b, mj * REL_TOL)) b = 0.0;
-  }
-  double s = a + b;
+  const double s = intdiv::double_of(m);
+  const Rcp<double> rs(s);
+  a = (mul_pow2(div_by(F, rs), l, k) - mul_pow2(div_by(Fm, rs), lm, km)) * s;
+  if (mag_bits(a) < intdiv::bits_of(s * REL_TOL)) a = 0.0;
+  return a;
+}
+
+__device__ __forceinline__ double divergence_fp64(double Fi, double Fim, double Fj, double Fjm,
+                                                  const Geom& G, const Rcp<double>& vol) {
+  const double NEAR0 = 5.0 * Num<double>::tiny;  // near_zero, flux_solver.f90:461-474
+  double s = scaled_difference(Fi, Fim, G.l2, G.k2, G.l4, G.k4) +
+             scaled_difference(Fj, Fjm, G.l3, G.k3, G.l1, G.k1);
   if (abs_lt(s, NEAR0)) s = 0.0;
-  return G.inv_vol != 0.0 ? mul_pow2(rneg(s), G.inv_vol, G.kinv) : N::div(rneg(s), G.vol);
+  return G.inv_vol != 0.0 ? mul_pow2(rneg(s), G.inv_vol, G.kinv) : div_by(rneg(s), vol);
 }
 
 }  // namespace cato

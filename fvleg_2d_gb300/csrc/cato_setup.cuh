@@ -25,6 +25,7 @@ inline FluxConsts<double> flux_consts_of(const cato_config& c) {
   K.ausm_ku = c.ausm_ku;
   K.ausm_sigma = c.ausm_sigma;
   K.low_mach_fix = c.apply_low_mach_fix ? 1 : 0;
+  K.gm1_y62 = intdiv::recip62(intdiv::bits_of(K.gm1));
   K.harten = c.roe_entropy_fix == CATO_ROE_HARTEN ? 1 : 0;
   return K;
 }

@@ -411,6 +411,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, const FluxConsts<
         if (A.G.rdyc) dy_inv = to_df(A.G.rdyc[j]);
       }
       if constexpr (Prec<R>::kind != 1) {
+        [[maybe_unused]] const Rcp<double> vol(cg.vol, cg.vol_y62);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const R Fi = sfi[k * T + t], Fim = sfi[k * T + t - 1];
@@ -418,7 +419,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, const FluxConsts<
           const R Fjm = sfj[(((j - 1) & 1) * 4 + k) * T + t];
           double r;
           if constexpr (Prec<R>::kind == 0) {
-            double L = divergence_fp64(Fi, Fim, Fj, Fjm, cg);
+            double L = divergence_fp64(Fi, Fim, Fj, Fjm, cg, vol);
             if (k == 3 && A.src_q) L = L + A.src_q[cidx];
             if (A.kind == 2) {
               r = L;
