@@ -158,6 +158,13 @@ static void drop_graph(cato_batch* b) {
   b->graph_steps = 0;
 }
 
+// columns of a work item's tile incl. the halo
+static int tile_columns(const cato_batch* b) {
+  if (b->prec == CATO_FP64) return batch_shape<double>(b->threads).columns;
+  if (b->prec == CATO_MIXED_DF) return batch_shape<df>(b->threads).columns;
+  return b->threads;
+}
+
 // Rebuild the per-group work lists (instance, tile x, tile y), largest instances first so the
 // dynamic queue ends on small items.
 static int rebuild(cato_batch* b) {
@@ -180,7 +187,7 @@ static int rebuild(cato_batch* b) {
     long long n = 0;
     for (int i : order) {
       const InstDesc& d = b->h_descs[i];
-      const int W = b->threads - 2 * d.ng, rr = std::min(r, d.nj);
+      const int W = tile_columns(b) - 2 * d.ng, rr = std::min(r, d.nj);
       n += (long long)((d.ni + W - 1) / W) * ((d.nj + rr - 1) / rr);
     }
     return n;
@@ -190,7 +197,7 @@ static int rebuild(cato_batch* b) {
   b->tile_rows = tile_rows;
   for (int i : order) {
     const InstDesc& d = b->h_descs[i];
-    const int W = b->threads - 2 * d.ng;
+    const int W = tile_columns(b) - 2 * d.ng;
     const int rows = std::min(tile_rows, d.nj);
     const int tx = (d.ni + W - 1) / W, ty = (d.nj + rows - 1) / rows;
     auto& L = lists[{d.flux, d.recon}];

@@ -78,14 +78,15 @@ __device__ __forceinline__ void batch_stage_args(InstDesc* d, const BatchStageAr
   }
 }
 
-template <typename R, int NG, int FLUX, int RECON>
-__global__ void __launch_bounds__(256, batch_min_blocks<R, FLUX>())
-    batch_stage_kernel(const BatchStageArgs B) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+// The persistent loop of a batch kernel: every CTA pulls (instance, tile) items from the queue and
+// hands them to tile(A, descriptor, tile x, tile y).
+template <typename R, typename Tile>
+__device__ __forceinline__ void batch_loop(const BatchStageArgs& B, Tile tile) {
   __shared__ int s_item;
+  const bool first = threadIdx.x == 0 && threadIdx.y == 0;
   for (;;) {
     __syncthreads();  // the previous tile is done with shared memory and s_item
-    if (threadIdx.x == 0) s_item = atomicAdd(B.counter, 1);
+    if (first) s_item = atomicAdd(B.counter, 1);
     __syncthreads();
     const int it = s_item;
     if (it >= B.n_items) break;
@@ -95,14 +96,30 @@ __global__ void __launch_bounds__(256, batch_min_blocks<R, FLUX>())
     StageArgs A;
     batch_stage_args<R>(d, B, A);
     A.rows_per_cta = w.w;
-    if constexpr (Prec<R>::kind == 0)
-      stage_tile<R, NG, FLUX, RECON, true>(A, d->K64, w.y, w.z, smem_raw);
-    else if constexpr (Prec<R>::kind == 1)
-      // no rectilinear grid, source or pressure input in a batch: the lean FP32 kernel
-      stage_tile<R, NG, FLUX, RECON, false>(A, d->K32, w.y, w.z, smem_raw);
-    else
-      stage_tile<R, NG, FLUX, RECON, true>(A, d->Kdf, w.y, w.z, smem_raw);
+    tile(A, d, w.y, w.z);
   }
+}
+
+// FP32; no rectilinear grid, source or pressure input in a batch: the lean tile
+template <int NG, int FLUX, int RECON>
+__global__ void __launch_bounds__(256, batch_tvd_tile_of(FLUX, RECON)
+                                           ? CATO_F32_BATCH_TVD_MIN_BLOCKS
+                                           : CATO_F32_BATCH_MIN_BLOCKS)
+    batch_stage_kernel(const BatchStageArgs B) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  batch_loop<float>(B, [&](const StageArgs& A, const InstDesc* d, int bx, int by) {
+    tile_of<NG, FLUX, RECON, false, batch_tvd_tile_of(FLUX, RECON)>(A, d->K32, bx, by, smem_raw);
+  });
+}
+
+// FP64 and double-float
+template <typename R, int NG, int FLUX, int RECON>
+__global__ void __maxnreg__(edge_regs(0)) batch_edge_kernel(const BatchStageArgs B) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  batch_loop<R>(B, [&](const StageArgs& A, const InstDesc* d, int bx, int by) {
+    if constexpr (Prec<R>::kind == 0) edge_tile<R, NG, FLUX, RECON>(A, d->K64, bx, by, smem_raw);
+    else edge_tile<R, NG, FLUX, RECON>(A, d->Kdf, bx, by, smem_raw);
+  });
 }
 
 }  // namespace cato

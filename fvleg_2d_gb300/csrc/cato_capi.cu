@@ -27,12 +27,6 @@ using namespace cato;
 
 namespace {
 
-struct Plan {
-  int threads = 128;       // CTA width incl. halo
-  int rows_per_cta = 64;   // rows marched per CTA
-  int variant = 0;         // FP64 stage kernel register budget (launch_stage_one)
-};
-
 struct Stage {
   int kind;     // StageArgs::kind
   double a, b;  // combine coefficients (kind 1 / mixed b)
@@ -91,7 +85,7 @@ struct cato_handle {
   double* src_field = nullptr;
   int* src_dep = nullptr;
   int src_parity = 0;
-  Plan plan;
+  StageShape plan;
   FluxConsts<double> K64{};
   FluxConsts<float> K32{};
   FluxConsts<df> Kdf{};
@@ -164,11 +158,7 @@ static void fill_consts(cato_handle* h) {
 }
 
 static void default_plan(cato_handle* h) {
-  const LaunchShape d = default_shape(h->ni, h->nj, h->ng);
-  Plan p;
-  p.threads = d.threads;
-  p.rows_per_cta = d.rows_per_cta;
-  h->plan = p;
+  h->plan = default_shape(h->ni, h->nj, h->ng, h->cfg.precision);
 }
 
 static StageArgs base_args(cato_handle* h) {
@@ -179,7 +169,7 @@ static StageArgs base_args(cato_handle* h) {
   A.pitch = h->pitch;
   for (int s = 0; s < 4; ++s) A.bc[s] = h->cfg.bc[s];
   A.limiter = h->cfg.limiter;
-  A.rows_per_cta = h->plan.rows_per_cta;
+  A.rows_per_cta = h->plan.rows;
   A.dt = &h->ctl->dt;
   A.active = &h->ctl->active;
   A.dt_min = &h->ctl->dt_min;
@@ -191,17 +181,13 @@ static StageArgs base_args(cato_handle* h) {
   return A;
 }
 
-static cudaError_t launch(cato_handle* h, const StageArgs& A) {
-  const int T = h->plan.threads;
-  const int W = T - 2 * h->ng;
-  dim3 grid((h->ni + W - 1) / W, (h->nj + A.rows_per_cta - 1) / A.rows_per_cta);
+static cudaError_t launch(cato_handle* h, const StageArgs& A, bool warm = false) {
   const int recon = recon_of(h->cfg.limiter);
   if (h->cfg.precision == CATO_FP64)
-    return launch_stage<double>(h->cfg.flux, recon, grid, T, h->stream, A, h->K64,
-                                h->plan.variant);
+    return launch_stage<double>(h->cfg.flux, recon, h->plan, warm, h->stream, A, h->K64);
   if (h->cfg.precision == CATO_MIXED_DF)
-    return launch_stage<df>(h->cfg.flux, recon, grid, T, h->stream, A, h->Kdf);
-  return launch_stage<float>(h->cfg.flux, recon, grid, T, h->stream, A, h->K32);
+    return launch_stage<df>(h->cfg.flux, recon, h->plan, warm, h->stream, A, h->Kdf);
+  return launch_stage<float>(h->cfg.flux, recon, h->plan, warm, h->stream, A, h->K32);
 }
 
 static bool has_pbc(const cato_handle* h) {
@@ -642,15 +628,8 @@ int cato_gpu_create(const cato_config* cfg, cato_handle** out) {
   h->ctl_host->max_iter = (1LL << 62);
   if (cudaMemcpy(h->ctl, h->ctl_host, sizeof(StepCtl), cudaMemcpyHostToDevice) != cudaSuccess)
     return cleanup(CATO_ERR_CUDA);
-  // prepare the kernel's shared-memory attribute outside any stream capture
-  StageArgs A = base_args(h);
-  const int rc0 = recon_of(cfg->limiter);
-  cudaError_t ee =
-      cfg->precision == CATO_FP64
-          ? launch_stage<double>(cfg->flux, rc0, dim3(0, 0), 64, h->stream, A, h->K64)
-      : cfg->precision == CATO_MIXED_DF
-          ? launch_stage<df>(cfg->flux, rc0, dim3(0, 0), 64, h->stream, A, h->Kdf)
-          : launch_stage<float>(cfg->flux, rc0, dim3(0, 0), 64, h->stream, A, h->K32);
+  // prepare the kernels' shared-memory attributes outside any stream capture
+  const cudaError_t ee = launch(h, base_args(h), true);
   if (ee != cudaSuccess) return cleanup(CATO_ERR_CUDA);
   *out = h;
   return CATO_OK;
@@ -1213,13 +1192,26 @@ int cato_gpu_run_timed(cato_handle* h, int64_t n_steps, float* total_ms, float* 
   return status_code(h->ctl_host->status);
 }
 
+// The launch shape of a plan (CTA width incl. the halo, rows per CTA).  The edge-parallel kernels
+// take half the width in columns (32 .. 128) and march in blocks of up to 4 rows.
+static StageShape plan_of(const cato_handle* h, int threads, int rows, int variant) {
+  StageShape s;
+  s.variant = variant;
+  s.rows = rows;
+  s.width = s.threads = threads;
+  if (h->cfg.precision != CATO_MIXED) {
+    s.threads = threads / 64 * 32;
+    s.block = std::min(rows, s.threads > 64 ? 3 : 4);
+  }
+  return s;
+}
+
 int cato_gpu_set_plan(cato_handle* h, int32_t threads, int32_t rows_per_cta) {
   if (!h) return CATO_ERR_ARG;
   if (threads < 64 || threads > 256 || threads % 32 != 0 || rows_per_cta < 1 ||
       threads - 2 * h->ng < 1)
     return fail(h, CATO_ERR_ARG, "invalid plan");
-  h->plan.threads = threads;
-  h->plan.rows_per_cta = rows_per_cta;
+  h->plan = plan_of(h, threads, rows_per_cta, h->plan.variant);
   return CATO_OK;
 }
 
@@ -1241,30 +1233,30 @@ int cato_gpu_tune(cato_handle* h, int32_t steps, int32_t* steps_taken, float* be
   if (steps_taken) *steps_taken = 0;
   if (!h->uploaded) return fail(h, CATO_ERR_STATE, "no state uploaded");
   if (h->exchange) return refuse_exchange(h, "cato_gpu_tune");
-  // candidates: the default plan and 256-wide strips, each with the default, half and a quarter
-  // of the rows per CTA, and with every FP64 register budget
-  const Plan p0 = h->plan;
-  std::vector<Plan> cands;
-  const int wide = 256, half_rows = std::max(8, p0.rows_per_cta / 2);
-  const int quarter_rows = std::max(8, p0.rows_per_cta / 4);
+  // candidates: the current plan and the widest one, each with the current, half and a quarter of
+  // the rows per CTA (down to 8), and with every FP64 register budget
+  const StageShape p0 = h->plan;
+  std::vector<StageShape> cands;
+  const int half_rows = p0.rows <= 8 ? p0.rows : std::max(8, p0.rows / 2);
+  const int quarter_rows = p0.rows <= 8 ? p0.rows : std::max(8, p0.rows / 4);
   const int nvar = h->cfg.precision == CATO_FP64 ? 3 : 1;
   for (int v = 0; v < nvar; ++v) {
-    Plan a = p0, b = p0, c = p0, d = p0, e = p0, f = p0;
-    a.variant = b.variant = c.variant = d.variant = e.variant = f.variant = v;
-    b.threads = e.threads = f.threads = wide;
-    c.rows_per_cta = e.rows_per_cta = half_rows;
-    d.rows_per_cta = f.rows_per_cta = quarter_rows;
-    for (const Plan& q : {a, b, c, d, e, f}) {
-      bool dup = false;
-      for (const Plan& x : cands)
-        dup |= x.threads == q.threads && x.rows_per_cta == q.rows_per_cta && x.variant == q.variant;
-      if (!dup && q.threads - 2 * h->ng <= h->ni + 2 * h->ng) cands.push_back(q);
+    for (int width : {p0.width, 256}) {
+      for (int rows : {p0.rows, half_rows, quarter_rows}) {
+        StageShape q = p0;
+        q.variant = v;
+        if (width != p0.width || rows != p0.rows) q = plan_of(h, width, rows, v);
+        bool dup = false;
+        for (const StageShape& x : cands)
+          dup |= x.width == q.width && x.rows == q.rows && x.variant == q.variant;
+        if (!dup && q.width - 2 * h->ng <= h->ni + 2 * h->ng) cands.push_back(q);
+      }
     }
   }
-  Plan best = p0;
+  StageShape best = p0;
   float best_t = INFINITY;
   int taken = 0;
-  for (const Plan& q : cands) {
+  for (const StageShape& q : cands) {
     h->plan = q;
     float ms = 0.0f;
     const int rc = cato_gpu_run_timed(h, steps, &ms, nullptr, 0);
@@ -1287,8 +1279,8 @@ int cato_gpu_tune(cato_handle* h, int32_t steps, int32_t* steps_taken, float* be
 
 int cato_gpu_get_plan(const cato_handle* h, int32_t* threads, int32_t* rows_per_cta) {
   if (!h) return CATO_ERR_ARG;
-  if (threads) *threads = h->plan.threads;
-  if (rows_per_cta) *rows_per_cta = h->plan.rows_per_cta;
+  if (threads) *threads = h->plan.width;
+  if (rows_per_cta) *rows_per_cta = h->plan.rows;
   return CATO_OK;
 }
 

@@ -1,8 +1,9 @@
-// cato_launch.cuh -- host-side launchers of the stage kernel, instantiated per (precision, flux)
+// cato_launch.cuh -- host-side launchers of the stage kernels, instantiated per (precision, flux)
 // in separate translation units (stage_inst.cu compiled once per pair) so that the FP64 ones can
 // be built with --fmad=false and the build parallelises.
 #pragma once
 
+#include <algorithm>
 #include <atomic>
 
 #include "cato_batch.cuh"
@@ -24,98 +25,159 @@ inline int launch_device() {
   return dev;
 }
 
-template <typename R, int NG, int FLUX, int RECON, bool EXT, int MB = min_blocks<R>()>
-cudaError_t launch_stage_ext(dim3 grid, int threads, cudaStream_t stream, const StageArgs& A,
-                             const FluxConsts<R>& K) {
+// The shape of a single-grid launch: CTA columns incl. the x-halo, rows marched per CTA, and for
+// the edge-parallel kernels (FP64, double-float) the rows of a block and the register budget.
+struct StageShape {
+  int width = 128;  // the plan's CTA width, as the caller knows it
+  int threads = 128;
+  int rows = 64;
+  int block = 4;
+  int variant = 0;
+};
+
+// Raises kernel's dynamic shared-memory limit once per device.
+template <typename F>
+inline cudaError_t allow_smem(PerDevice& attr, int dev, F* kernel, size_t bytes) {
+  if (attr.done[dev].load(std::memory_order_acquire)) return cudaSuccess;
+  const cudaError_t e =
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e != cudaSuccess) return e;
+  int n = 0;
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  attr.sms[dev].store(n > 0 ? n : 1);
+  attr.done[dev].store(true, std::memory_order_release);
+  return cudaSuccess;
+}
+// the largest shared memory an edge-parallel kernel may be launched with
+template <typename R> inline size_t edge_smem_limit(int ng) {
+  const size_t a = edge_smem_bytes<R>({64, 4}, ng), b = edge_smem_bytes<R>({128, 3}, ng);
+  return a > b ? a : b;
+}
+inline bool edge_shape_ok(EdgeShape s) {
+  return s.columns >= 32 && s.columns <= 128 && s.columns % 32 == 0 && s.block >= 1 &&
+         s.block <= 4 && s.columns * (2 * s.block + 1) <= kEdgeThreads;
+}
+
+template <int NG, int FLUX, int RECON, bool EXT>
+cudaError_t launch_strip(const StageShape& s, bool warm, cudaStream_t stream, const StageArgs& A,
+                         const FluxConsts<float>& K) {
   static PerDevice attr;
-  const size_t smem = stage_smem_bytes<R>(threads, NG);
+  constexpr bool TVD = tvd_tile_of(FLUX, RECON);
   const int dev = launch_device();
   if (dev < 0) return cudaErrorInvalidDevice;
-  if (!attr.done[dev].load(std::memory_order_acquire)) {
-    cudaError_t e = cudaFuncSetAttribute(stage_kernel<R, NG, FLUX, RECON, EXT, MB>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)stage_smem_bytes<R>(256, 3));
-    if (e != cudaSuccess) return e;
-    attr.done[dev].store(true, std::memory_order_release);
-  }
-  if (grid.x == 0 || grid.y == 0) return cudaSuccess;  // attribute warm-up only
-  stage_kernel<R, NG, FLUX, RECON, EXT, MB><<<grid, threads, smem, stream>>>(A, K);
+  cudaError_t e = allow_smem(attr, dev, stage_kernel<NG, FLUX, RECON, EXT>,
+                             tile_smem_bytes(256, NG, FLUX, TVD));
+  if (e != cudaSuccess || warm) return e;
+  const int W = s.threads - 2 * NG;
+  const dim3 grid((A.ni + W - 1) / W, (A.nj + s.rows - 1) / s.rows);
+  stage_kernel<NG, FLUX, RECON, EXT>
+      <<<grid, s.threads, tile_smem_bytes(s.threads, NG, FLUX, TVD), stream>>>(A, K);
   return cudaGetLastError();
 }
 
-// The FP32 path has a lean variant without the rectilinear, source and pressure-input code
-// (it is issue-bound: those checks cost ~3 %); double-float keeps one kernel.  The FP64 path
-// has one kernel per register budget (variant 0: the compiler's choice, 1: at most 128, 2: at
-// most 85).
+template <typename R, int NG, int FLUX, int RECON, int REGS>
+cudaError_t launch_edge(const StageShape& s, bool warm, cudaStream_t stream, const StageArgs& A,
+                        const FluxConsts<R>& K) {
+  static PerDevice attr;
+  const int dev = launch_device();
+  if (dev < 0) return cudaErrorInvalidDevice;
+  cudaError_t e = allow_smem(attr, dev, edge_kernel<R, NG, FLUX, RECON, REGS>,
+                             edge_smem_limit<R>(NG));
+  if (e != cudaSuccess || warm) return e;
+  EdgeShape es{s.threads, s.block};
+  // the CTA's warps fit the register file: a quarter of them in each of its four 16 Ki parts
+  const int warps = 4 * (16384 / (32 * REGS));
+  es.block = std::min(es.block, (warps * 32 / es.columns - 1) / 2);
+  if (!edge_shape_ok(es)) return cudaErrorInvalidValue;
+  const int W = es.columns - 2 * NG;
+  const dim3 grid((A.ni + W - 1) / W, (A.nj + s.rows - 1) / s.rows);
+  edge_kernel<R, NG, FLUX, RECON, REGS>
+      <<<grid, dim3(es.columns, 2 * es.block + 1), edge_smem_bytes<R>(es, NG), stream>>>(A, K);
+  return cudaGetLastError();
+}
+
+// One stage of one grid; warm: only prepare every kernel of the scheme (outside stream captures).
+// The FP32 path has a lean variant without the rectilinear, source and pressure-input code (it is
+// issue-bound: those checks cost ~3 %).  The FP64 path has one kernel per register budget
+// (edge_regs).
 template <typename R, int NG, int FLUX, int RECON>
-cudaError_t launch_stage_one(dim3 grid, int threads, cudaStream_t stream, const StageArgs& A,
-                             const FluxConsts<R>& K, int variant) {
-  const bool warm = grid.x == 0 || grid.y == 0;  // attribute warm-up of every variant
+cudaError_t launch_stage_one(const StageShape& s, bool warm, cudaStream_t stream,
+                             const StageArgs& A, const FluxConsts<R>& K) {
   if constexpr (Prec<R>::kind == 1) {
     if (warm) {
-      cudaError_t e = launch_stage_ext<R, NG, FLUX, RECON, false>(grid, threads, stream, A, K);
+      cudaError_t e = launch_strip<NG, FLUX, RECON, false>(s, true, stream, A, K);
       if (e != cudaSuccess) return e;
-      return launch_stage_ext<R, NG, FLUX, RECON, true>(grid, threads, stream, A, K);
+    } else if (!stage_needs_ext(A)) {
+      return launch_strip<NG, FLUX, RECON, false>(s, false, stream, A, K);
     }
-    if (!stage_needs_ext(A))
-      return launch_stage_ext<R, NG, FLUX, RECON, false>(grid, threads, stream, A, K);
-  }
-  if constexpr (Prec<R>::kind == 0) {
-    if (warm) {
-      cudaError_t e = launch_stage_ext<R, NG, FLUX, RECON, true, CATO_F64_MIN_BLOCKS_ALT>(
-          grid, threads, stream, A, K);
-      if (e != cudaSuccess) return e;
-      e = launch_stage_ext<R, NG, FLUX, RECON, true, CATO_F64_MIN_BLOCKS_ALT2>(grid, threads,
-                                                                              stream, A, K);
-      if (e != cudaSuccess) return e;
-    } else if (variant == 1) {
-      return launch_stage_ext<R, NG, FLUX, RECON, true, CATO_F64_MIN_BLOCKS_ALT>(grid, threads,
-                                                                                stream, A, K);
-    } else if (variant == 2) {
-      return launch_stage_ext<R, NG, FLUX, RECON, true, CATO_F64_MIN_BLOCKS_ALT2>(grid, threads,
-                                                                                 stream, A, K);
+    return launch_strip<NG, FLUX, RECON, true>(s, warm, stream, A, K);
+  } else {
+    if constexpr (Prec<R>::kind == 0) {
+      if (warm) {
+        cudaError_t e = launch_edge<R, NG, FLUX, RECON, edge_regs(1)>(s, true, stream, A, K);
+        if (e == cudaSuccess)
+          e = launch_edge<R, NG, FLUX, RECON, edge_regs(2)>(s, true, stream, A, K);
+        if (e != cudaSuccess) return e;
+      } else if (s.variant == 1) {
+        return launch_edge<R, NG, FLUX, RECON, edge_regs(1)>(s, false, stream, A, K);
+      } else if (s.variant == 2) {
+        return launch_edge<R, NG, FLUX, RECON, edge_regs(2)>(s, false, stream, A, K);
+      }
     }
+    return launch_edge<R, NG, FLUX, RECON, edge_regs(0)>(s, warm, stream, A, K);
   }
-  return launch_stage_ext<R, NG, FLUX, RECON, true>(grid, threads, stream, A, K);
 }
 
 // recon: 0 = TVD2 (minmod / superbee / van Leer), 3 = MLP3, 5 = MLP5
 template <typename R, int FLUX>
-inline cudaError_t launch_stage_flux(int recon, dim3 grid, int threads, cudaStream_t stream,
-                                     const StageArgs& A, const FluxConsts<R>& K, int variant) {
+inline cudaError_t launch_stage_flux(int recon, const StageShape& s, bool warm,
+                                     cudaStream_t stream, const StageArgs& A,
+                                     const FluxConsts<R>& K) {
   switch (recon) {
-    case 0: return launch_stage_one<R, 2, FLUX, 0>(grid, threads, stream, A, K, variant);
-    case 3: return launch_stage_one<R, 2, FLUX, 3>(grid, threads, stream, A, K, variant);
-    case 5: return launch_stage_one<R, 3, FLUX, 5>(grid, threads, stream, A, K, variant);
+    case 0: return launch_stage_one<R, 2, FLUX, 0>(s, warm, stream, A, K);
+    case 3: return launch_stage_one<R, 2, FLUX, 3>(s, warm, stream, A, K);
+    case 5: return launch_stage_one<R, 3, FLUX, 5>(s, warm, stream, A, K);
     default: return cudaErrorInvalidValue;
   }
+}
+
+// The shape of a batch launch for a plan's CTA width: FP32 strips are as wide as the plan says;
+// the edge-parallel tiles half as wide (32 to 64 columns), in blocks of 4 rows.
+template <typename R> inline EdgeShape batch_shape(int threads) {
+  if (Prec<R>::kind == 1) return {threads, 0};
+  return {threads < 128 ? 32 : 64, 4};
 }
 
 // Persistent batch launch: as many CTAs as can be resident, each looping over work items.
 template <typename R, int NG, int FLUX, int RECON>
 cudaError_t launch_batch_one(int threads, cudaStream_t stream, const BatchStageArgs& B) {
   static PerDevice attr;
-  const size_t smem = stage_smem_bytes<R>(threads, NG);
   const int dev = launch_device();
   if (dev < 0) return cudaErrorInvalidDevice;
-  if (!attr.done[dev].load(std::memory_order_acquire)) {
-    cudaError_t e = cudaFuncSetAttribute(batch_stage_kernel<R, NG, FLUX, RECON>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)stage_smem_bytes<R>(256, 3));
-    if (e != cudaSuccess) return e;
-    int n = 0;
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    attr.sms[dev].store(n > 0 ? n : 1);
-    attr.done[dev].store(true, std::memory_order_release);
+  const EdgeShape shape = batch_shape<R>(threads);
+  void (*kernel)(const BatchStageArgs);
+  size_t smem, most;
+  dim3 block;
+  if constexpr (Prec<R>::kind == 1) {
+    kernel = batch_stage_kernel<NG, FLUX, RECON>;
+    smem = tile_smem_bytes(threads, NG, FLUX, batch_tvd_tile_of(FLUX, RECON));
+    most = tile_smem_bytes(256, NG, FLUX, batch_tvd_tile_of(FLUX, RECON));
+    block = dim3(threads);
+  } else {
+    kernel = batch_edge_kernel<R, NG, FLUX, RECON>;
+    smem = edge_smem_bytes<R>(shape, NG);
+    most = edge_smem_limit<R>(NG);
+    block = dim3(shape.columns, 2 * shape.block + 1);
   }
+  cudaError_t e = allow_smem(attr, dev, kernel, most);
+  if (e != cudaSuccess) return e;
   if (B.n_items <= 0) return cudaSuccess;
   int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &per_sm, batch_stage_kernel<R, NG, FLUX, RECON>, threads, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (int)(block.x * block.y), smem);
   if (e != cudaSuccess) return e;
   long long grid = (long long)(per_sm > 0 ? per_sm : 1) * attr.sms[dev].load();
   if (grid > B.n_items) grid = B.n_items;
-  batch_stage_kernel<R, NG, FLUX, RECON><<<(unsigned)grid, threads, smem, stream>>>(B);
+  kernel<<<(unsigned)grid, block, smem, stream>>>(B);
   return cudaGetLastError();
 }
 
@@ -134,9 +196,9 @@ inline cudaError_t launch_batch_flux(int recon, int threads, cudaStream_t stream
 // unit (stage_inst.cu, compiled once per precision and flux, and for the slow double-float units
 // once per reconstruction and kernel kind); everywhere else these are extern.
 #define CATO_DECLARE_ONE(R, F, NG, RC)                                                         \
-  extern template cudaError_t launch_stage_one<R, NG, F, RC>(dim3, int, cudaStream_t,          \
-                                                             const StageArgs&,                 \
-                                                             const FluxConsts<R>&, int);       \
+  extern template cudaError_t launch_stage_one<R, NG, F, RC>(const StageShape&, bool,          \
+                                                             cudaStream_t, const StageArgs&,   \
+                                                             const FluxConsts<R>&);            \
   extern template cudaError_t launch_batch_one<R, NG, F, RC>(int, cudaStream_t,               \
                                                              const BatchStageArgs&);
 #define CATO_DECLARE_STAGE(R, F) \
@@ -152,20 +214,19 @@ CATO_DECLARE_PREC(df)
 #undef CATO_DECLARE_STAGE
 #undef CATO_DECLARE_ONE
 
-// variant: the FP64 kernel's register budget (0, 1 or 2, see launch_stage_one); ignored otherwise
 template <typename R>
-inline cudaError_t launch_stage(int flux, int recon, dim3 grid, int threads, cudaStream_t s,
-                                const StageArgs& A, const FluxConsts<R>& K, int variant = 0) {
+inline cudaError_t launch_stage(int flux, int recon, const StageShape& h, bool warm, cudaStream_t s,
+                                const StageArgs& A, const FluxConsts<R>& K) {
   switch (flux) {
-    case 0: return launch_stage_flux<R, 0>(recon, grid, threads, s, A, K, variant);
-    case 1: return launch_stage_flux<R, 1>(recon, grid, threads, s, A, K, variant);
-    case 2: return launch_stage_flux<R, 2>(recon, grid, threads, s, A, K, variant);
-    case 3: return launch_stage_flux<R, 3>(recon, grid, threads, s, A, K, variant);
-    case 4: return launch_stage_flux<R, 4>(recon, grid, threads, s, A, K, variant);
-    case 5: return launch_stage_flux<R, 5>(recon, grid, threads, s, A, K, variant);
-    case 6: return launch_stage_flux<R, 6>(recon, grid, threads, s, A, K, variant);
-    case 7: return launch_stage_flux<R, 7>(recon, grid, threads, s, A, K, variant);
-    case 8: return launch_stage_flux<R, 8>(recon, grid, threads, s, A, K, variant);
+    case 0: return launch_stage_flux<R, 0>(recon, h, warm, s, A, K);
+    case 1: return launch_stage_flux<R, 1>(recon, h, warm, s, A, K);
+    case 2: return launch_stage_flux<R, 2>(recon, h, warm, s, A, K);
+    case 3: return launch_stage_flux<R, 3>(recon, h, warm, s, A, K);
+    case 4: return launch_stage_flux<R, 4>(recon, h, warm, s, A, K);
+    case 5: return launch_stage_flux<R, 5>(recon, h, warm, s, A, K);
+    case 6: return launch_stage_flux<R, 6>(recon, h, warm, s, A, K);
+    case 7: return launch_stage_flux<R, 7>(recon, h, warm, s, A, K);
+    case 8: return launch_stage_flux<R, 8>(recon, h, warm, s, A, K);
     default: return cudaErrorInvalidValue;
   }
 }

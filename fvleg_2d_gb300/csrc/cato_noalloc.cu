@@ -118,7 +118,7 @@ extern "C" int cato_gpu_solve_noalloc(const cato_config* cfg, double* rho, doubl
   // flux constants, uniform geometry and launch shape: those a handle derives from cfg
   const FluxConsts<double> K = flux_consts_of(*cfg);
   const Geom G = uniform_geom(cfg->dx, cfg->dy);
-  const LaunchShape shape = default_shape(ni, nj, ng);
+  const StageShape shape = default_shape(ni, nj, ng, cfg->precision);
 
   StageArgs A;
   std::memset(&A, 0, sizeof(A));
@@ -127,8 +127,7 @@ extern "C" int cato_gpu_solve_noalloc(const cato_config* cfg, double* rho, doubl
   A.pitch = pitch;
   for (int k = 0; k < 4; ++k) A.bc[k] = cfg->bc[k];
   A.limiter = cfg->limiter;
-  const int threads = shape.threads;
-  A.rows_per_cta = shape.rows_per_cta;
+  A.rows_per_cta = shape.rows;
   A.kind = 2;
   A.dt = ctl;
   A.dt_min = reinterpret_cast<unsigned long long*>(ctl + 1);
@@ -142,11 +141,8 @@ extern "C" int cato_gpu_solve_noalloc(const cato_config* cfg, double* rho, doubl
     A.Uk[k] = prim[k];
     A.Uo[k] = res[k];
   }
-  const int W = threads - 2 * ng;
   const int recon = recon_of_limiter(cfg->limiter);
-  NA_CK(launch_stage<double>(cfg->flux, recon, dim3((ni + W - 1) / W, (nj + A.rows_per_cta - 1) /
-                                                                          A.rows_per_cta),
-                             threads, s, A, K));
+  NA_CK(launch_stage<double>(cfg->flux, recon, shape, false, s, A, K));
   const int4 bc = make_int4(cfg->bc[0], cfg->bc[1], cfg->bc[2], cfg->bc[3]);
   const long long nh = hld * (nj + 2 * ng);
   int blocks = (int)((nh + 255) / 256);

@@ -42,20 +42,6 @@ static __device__ __noinline__ double sqrt_rn(double a) {
   const uint64_t r = intdiv::sqrt_bits(intdiv::bits_of(a), ok);
   return ok ? intdiv::double_of(r) : sqrt_hw(a);
 }
-// IEEE binary64 a * b on the integer pipe (intdiv::mul_bits), bit-identical to the FP64
-// instruction: a zero operand times a finite one is the zero with the product's sign; operands
-// or products outside the normal range take the hardware instruction.  Out of line, as div_rn.
-static __device__ __noinline__ double mul_hw(double a, double b) { return a * b; }
-static __device__ __noinline__ double mul_rn(double a, double b) {
-  const uint64_t ua = intdiv::bits_of(a), ub = intdiv::bits_of(b);
-  const uint64_t za = ua << 1, zb = ub << 1;
-  if ((za == 0ULL || zb == 0ULL) && za < 0xffe0000000000000ULL && zb < 0xffe0000000000000ULL)
-    return intdiv::double_of((ua ^ ub) & 0x8000000000000000ULL);
-  bool ok;
-  const uint64_t r = intdiv::mul_bits(ua, ub, ok);
-  return ok ? intdiv::double_of(r) : mul_hw(a, b);
-}
-
 // RN(a / b) with the part that depends on b alone given (intdiv::recip62 of b's bits)
 static __device__ __noinline__ double quot_rn(double a, double b, uint64_t y62) {
   bool ok;
@@ -96,11 +82,6 @@ template <> struct Num<double> {
     if ((intdiv::bits_of(a) << 1) == 0ULL) return a;
     return sqrt_rn(a);
   }
-#ifdef CATO_F64_MUL_INT
-  static __device__ __forceinline__ double mul(double a, double b) { return mul_rn(a, b); }
-#else
-  static __device__ __forceinline__ double mul(double a, double b) { return a * b; }
-#endif
 };
 
 // A divisor of several quotients: div_by(a, Rcp(b)) is Num<R>::div(a, b).  FP64 shares the
@@ -130,7 +111,6 @@ template <> struct Num<float> {
   static constexpr float tiny = FLT_MIN;
   static __device__ __forceinline__ float div(float a, float b) { return __fdividef(a, b); }
   static __device__ __forceinline__ float sqrt(float a) { return ::sqrtf(a); }
-  static __device__ __forceinline__ float mul(float a, float b) { return a * b; }
 };
 
 template <> struct Num<df> {
@@ -138,7 +118,6 @@ template <> struct Num<df> {
   static constexpr df tiny = df(FLT_MIN, 0.0f);
   static __device__ __forceinline__ df div(df a, df b) { return df_div(a, b); }
   static __device__ __forceinline__ df sqrt(df a) { return df_sqrt(a); }
-  static __device__ __forceinline__ df mul(df a, df b) { return a * b; }
 };
 
 template <> __device__ __forceinline__ float div_by<float>(float a, const Rcp<float>& c) {
@@ -520,17 +499,10 @@ __device__ __forceinline__ void recon_tvd2(int lim, R qm1, R q0, R qp1, R qp2, R
   Rr = slope_step(qp1, tvd_phi_edge(lim, d0, dp), dp, true);
 }
 
-// FP64 TVD2 edge values out of line: one copy per kernel instead of one per variable and
-// direction keeps the stage kernel inside the instruction cache
+// a pair of edge values
 struct EdgePair {
   double L, R;
 };
-static __device__ __noinline__ EdgePair recon_tvd2_f64(int lim, double qm1, double q0, double qp1,
-                                                      double qp2) {
-  EdgePair e;
-  recon_tvd2<double>(lim, qm1, q0, qp1, qp2, e.L, e.R);
-  return e;
-}
 
 // FP32 (mixed path): the limited slope phi(r) * dq without the ratio.  For r = d0/dq > 0,
 // minmod gives min(r, 1) dq = (|d0| < |dq| ? d0 : dq), superbee picks one of 2 d0, dq, d0, 2 dq,
@@ -636,13 +608,200 @@ __device__ __forceinline__ void recon_mlp(R qm2, R qm1, R q0, R qp1, R qp2, R qp
   Rr = slope_step(qp1, phiR, dp, true);
 }
 
-// FP64 MLP edge values out of line (one copy per kernel, as recon_tvd2_f64)
+// the general edge values, out of line: extreme differences and signed zeros
 template <int ORDER>
-static __device__ __noinline__ EdgePair recon_mlp_f64(double qm2, double qm1, double q0, double qp1,
+static __device__ __noinline__ EdgePair recon_mlp_any(double qm2, double qm1, double q0, double qp1,
                                                      double qp2, double qp3, double t0p,
                                                      double t0m, double t1p, double t1m) {
   EdgePair e;
   recon_mlp<double, ORDER>(qm2, qm1, q0, qp1, qp2, qp3, t0p, t0m, t1p, t1m, e.L, e.R);
+  return e;
+}
+
+// x + 1e-30 (the limiter's SMALL_NUM): x itself from 2^-45 up, where 1e-30 is below half a unit in
+// the last place (and below half a unit of the next lower binade); infinities and NaN pass.
+__device__ __forceinline__ double add_small(double x) {
+  return (uint32_t)(mag_bits(x) >> 32) >= ((1023u - 45u) << 20) ? x : x + 1e-30;
+}
+// RN(a / b) for normal operands and a normal quotient
+static __device__ __noinline__ double div_normal(double a, double b) {
+  bool ok;
+  return intdiv::double_of(intdiv::div_bits(intdiv::bits_of(a), intdiv::bits_of(b), ok));
+}
+// q + t or q - t: q itself for a zero t and a non-zero q, on the integer pipe
+__device__ __forceinline__ double add_slope(double q, double t, bool minus) {
+  if (mag_bits(t) == 0ULL && mag_bits(q) != 0ULL) return q;
+  return minus ? q - t : q + t;
+}
+// half(x) for |x| >= 2^-1021
+__device__ __forceinline__ double half_normal(double x) {
+  return intdiv::double_of(intdiv::bits_of(x) - (1ULL << 52));
+}
+
+// FP64 MLP edge values (out of line: one copy per kernel, as recon_tvd2_f64), the values of
+// recon_mlp<double, ORDER> bit for bit.  The limiter is phi = max(0, min(alpha r, alpha, beta)):
+// FP32 estimates of alpha and beta from the differences tell which of them decides, so that the
+// quotients of the other are left out (16 divisions per edge with all of them, each ~120
+// instructions; typically 3 to 6 remain: 1700 -> 900 instructions per edge).  Only what decides is
+// formed, in the reference's order; where the estimates are within 1e-3 of each other (100 times
+// their error) both are.  r >= 1 is |d0| >= |dq + S|, and alpha is clamped to [1, 2], where
+// alpha r and alpha / 2 are exact.
+template <int ORDER>
+static __device__ __noinline__ EdgePair recon_mlp_f64(double qm2, double qm1, double q0, double qp1,
+                                                     double qp2, double qp3, double t0p,
+                                                     double t0m, double t1p, double t1m) {
+  const double EPS = Num<double>::eps;
+  double d0 = qp1 - q0, D[2] = {q0 - qm1, qp2 - qp1}, X[2] = {0.0, 0.0};
+  const double n[2] = {t0p - t0m, t1p - t1m};
+  if (abs_lt(d0, EPS)) d0 = 0.0;
+  if (ORDER == 5) {
+    X[0] = qm1 - qm2;
+    X[1] = qp3 - qp2;
+  }
+  uint32_t most = (uint32_t)(mag_bits(d0) >> 32);
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    if (abs_lt(D[s], EPS)) D[s] = 0.0;
+    if (abs_lt(X[s], EPS)) X[s] = 0.0;
+    most = max(most, max((uint32_t)(mag_bits(D[s]) >> 32),
+                         max((uint32_t)(mag_bits(X[s]) >> 32), (uint32_t)(mag_bits(n[s]) >> 32))));
+  }
+  // differences of 2^60 and above (NaN and infinities among them): the general form
+  if (most >= (1023u + 60u) << 20)
+    return recon_mlp_any<ORDER>(qm2, qm1, q0, qp1, qp2, qp3, t0p, t0m, t1p, t1m);
+  const float f0 = d2f_fast(d0), fD[2] = {d2f_fast(D[0]), d2f_fast(D[1])};
+  const float fX[2] = {d2f_fast(X[0]), d2f_fast(X[1])};
+  const float fn[2] = {fabsf(d2f_fast(n[0])), fabsf(d2f_fast(n[1]))};
+  // central differences along the edge normal; estimates of alpha count where these keep two
+  // digits of their terms and stand well above the epsilon flush
+  const float fe[2] = {fabsf(fD[0] + f0), fabsf(fD[1] + f0)};
+  const float amp = fabsf(f0) + fmaxf(fabsf(fD[0]), fabsf(fD[1]));
+  const bool sure = fminf(fe[0], fe[1]) > 0.01f * amp && fminf(fe[0], fe[1]) > 1e-11f;
+  const float if0 = __fdividef(1.0f, f0);
+  double t[2];
+#pragma unroll 1
+  for (int s = 0; s < 2; ++s) {
+    const double dq = s ? D[1] : D[0], dx = s ? D[0] : D[1];
+    const uint64_t sd = (intdiv::bits_of(d0) ^ intdiv::bits_of(dq)) & kSignBit;
+    if (mag_bits(d0) == 0ULL || mag_bits(dq) == 0ULL || sd != 0ULL) {  // r <= 0, or a zero slope
+      t[s] = intdiv::double_of(intdiv::bits_of(dq) & kSignBit);
+      continue;
+    }
+    const float fq = s ? fD[1] : fD[0], fx = s ? fD[0] : fD[1], fy = s ? fX[1] : fX[0];
+    const float ifq = __fdividef(1.0f, fq), rf = f0 * ifq, mf = fminf(rf, 1.0f);
+    float b, bm;  // beta and the sum of its terms' magnitudes
+    if (ORDER == 5) {
+      b = (11.0f * fq + 24.0f * f0 - (2.0f * fy + 3.0f * fx)) * ifq * (1.0f / 30.0f);
+      bm = (11.0f * fabsf(fq) + 24.0f * fabsf(f0) + (2.0f * fabsf(fy) + 3.0f * fabsf(fx))) *
+           fabsf(ifq) * (1.0f / 30.0f);
+    } else {
+      b = bm = (1.0f + 2.0f * rf) * (1.0f / 3.0f);
+    }
+    // alpha between lo and hi
+    const float town = __fdividef(s ? fn[1] : fn[0], s ? fe[1] : fe[0]);
+    const float toth = __fdividef(s ? fn[0] : fn[1], s ? fe[0] : fe[1]);
+    const float at = __fdividef(2.0f * fmaxf(1.0f, rf) * (1.0f + fmaxf(0.0f, toth * fx * if0)),
+                                1.0f + town);
+    const bool known = sure && at >= 0.0f;
+    const float lo = known ? fmaxf(1.0f, fminf(2.0f, at * 0.999f)) : 1.0f;
+    const float hi = known ? fmaxf(1.0f, fminf(2.0f, at * 1.001f)) : 2.0f;
+    const float db = 1e-3f * bm;
+    if (b + db < 0.0f) {  // beta < 0: phi = 0
+      t[s] = intdiv::double_of(intdiv::bits_of(dq) & kSignBit);
+      continue;
+    }
+    const bool beta_only = b + db < lo * mf * 0.999f, alpha_only = b - db > hi * mf * 1.001f;
+    const bool need_b = !alpha_only, need_a = !beta_only && lo != hi;
+    const double Dq = add_small(dq);
+    const bool r_ge1 = mag_bits(d0) >= mag_bits(Dq);
+    double r = 0.0, bt = 0.0, al = lo == 1.0f ? 1.0 : 2.0;
+    if (need_b || need_a || !r_ge1) r = div_normal(d0, Dq);
+    if (need_b) {
+      if (ORDER == 5) {
+        const double r1 = Num<double>::div(dq, add_small(s ? X[1] : X[0]));
+        const double r2 = Num<double>::div(dx, add_small(d0));
+        bt = (((Num<double>::div(-2.0, add_small(r1))) + 11.0) + 24.0 * r) - 3.0 * r * r2;
+        bt = div_by(bt, Rcp<double>(30.0, 2459565876494606882ULL));
+      } else {
+        bt = div_by(1.0 + twice(r), Rcp<double>(3.0, 3074457345618258602ULL));
+      }
+    }
+    if (need_a) {
+      const double e0 = rabs(qp1 - qm1), e1 = rabs(qp2 - q0);
+      const double to = Num<double>::div(rabs(s ? n[1] : n[0]), add_small(s ? e1 : e0));
+      const double tx = Num<double>::div(rabs(s ? n[0] : n[1]), add_small(s ? e0 : e1));
+      const double ro = Num<double>::div(d0, add_small(dx));
+      const double a = Num<double>::div(
+          (r_ge1 ? twice(r) : 2.0) * (1.0 + rmax(0.0, Num<double>::div(tx, add_small(ro)))), 1.0 + to);
+      al = rmax(1.0, rmin(2.0, a));
+    }
+    double phi;
+    if (beta_only) {
+      phi = rmax(0.0, bt);
+    } else {
+      // min(alpha r, alpha) is alpha for r >= 1
+      phi = r_ge1 ? al : al * r;
+      if (need_b) phi = rmax(0.0, rmin(phi, bt));
+    }
+    t[s] = half(phi) * dq;
+  }
+  EdgePair e;
+  e.L = add_slope(q0, t[0], false);
+  e.R = add_slope(qp1, t[1], true);
+  return e;
+}
+
+// One side of an edge: half(phi(d0 / (dq + 1e-16))) dq for non-zero d0 and dq of one sign and of
+// moderate size.  Minmod and superbee divide only where phi is the ratio itself (a ratio of at
+// least 1, or between 1/2 and 1, or of at least 2, gives phi by comparing the operands: a rounded
+// quotient is below 1 exactly when its operands are so ordered).
+__device__ __forceinline__ double tvd_side_f64(int lim, double d0, double dq) {
+  const double D = dq + 1e-16;
+  if (lim == LIM_VANLEER) {
+    const double r = div_normal(d0, D);
+    return half_normal(div_normal(twice(r), 1.0 + r)) * dq;
+  }
+  const uint64_t m = mag_bits(d0), d = mag_bits(D), one = 1ULL << 52;
+  int k = -1;  // half(phi) = r 2^k where the ratio itself is needed
+  if (lim == LIM_MINMOD) {
+    if (m >= d) return half_normal(dq);
+  } else {
+    if (m >= d + one) return dq;
+    if (m < d) {
+      if (m + one >= d) return half_normal(dq);
+      k = 0;
+    }
+  }
+  return intdiv::double_of(intdiv::bits_of(div_normal(d0, D)) + ((uint64_t)(int64_t)k << 52)) * dq;
+}
+// FP64 TVD2 values of one edge, the values of recon_tvd2<double> bit for bit.  Out of line: one
+// copy per kernel instead of one per variable and direction keeps it inside the instruction cache.
+static __device__ __noinline__ EdgePair recon_tvd2_f64(int lim, double qm1, double q0, double qp1,
+                                                      double qp2) {
+  const double EPS = Num<double>::eps;
+  double dm = q0 - qm1, d0 = qp1 - q0, dp = qp2 - qp1;
+  if (abs_lt(dm, EPS)) dm = 0.0;
+  if (abs_lt(d0, EPS)) d0 = 0.0;
+  if (abs_lt(dp, EPS)) dp = 0.0;
+  const uint32_t most = max((uint32_t)(mag_bits(d0) >> 32), max((uint32_t)(mag_bits(dm) >> 32),
+                                                                (uint32_t)(mag_bits(dp) >> 32)));
+  EdgePair e;
+  if (most >= (1023u + 60u) << 20) {  // extreme differences, NaN and infinities: the general form
+    e.L = slope_step(q0, tvd_phi_edge(lim, d0, dm), dm, false);
+    e.R = slope_step(qp1, tvd_phi_edge(lim, d0, dp), dp, true);
+    return e;
+  }
+#pragma unroll 1
+  for (int s = 0; s < 2; ++s) {
+    const double dq = s ? dp : dm;
+    const bool flat = mag_bits(d0) == 0ULL || mag_bits(dq) == 0ULL ||
+                      ((intdiv::bits_of(d0) ^ intdiv::bits_of(dq)) & kSignBit) != 0ULL;
+    const double t = flat ? intdiv::double_of(intdiv::bits_of(dq) & kSignBit)
+                          : tvd_side_f64(lim, d0, dq);
+    const double v = add_slope(s ? qp1 : q0, t, s != 0);
+    if (s) e.R = v;
+    else e.L = v;
+  }
   return e;
 }
 
@@ -832,6 +991,9 @@ __device__ __forceinline__ void recon_mlp<df, 5>(df qm2, df qm1, df q0, df qp1, 
 // Edge fluxes.  DIR = 0: i-edge (normal x, n = (1,0)); DIR = 1: j-edge (normal y, n = (0,1)).
 // The Cartesian normals are exact (quad_cell.f90:193-229 on axis-aligned cells), so the
 // reference's products with n_x / n_y are folded: x*1 = x and x*0 + y = y exactly.
+// The FP64 and double-float kernels run one copy of each flux for both directions: DIR = 0 in the
+// edge's own frame (u normal, v tangential) with y = true for a j-edge, which only the two places
+// that are not symmetric under the exchange of u and v read.
 // Cell-pressure stencils for the shock sensors are given in edge-local coordinates:
 // pc(n, t) = cell at normal offset n (0 = left cell, 1 = right cell) and tangential offset t.
 // ---------------------------------------------------------------------------------------------
@@ -935,20 +1097,23 @@ __device__ __forceinline__ void flux_ausmpw(const FluxConsts<R>& K, const Prim<R
   const R U_L = DIR == 0 ? u_LHS : v_LHS, U_R = DIR == 0 ? u_RHS : v_RHS;
   const R V_L = DIR == 0 ? v_LHS : u_LHS, V_R = DIR == 0 ? v_RHS : u_RHS;
   const Rcp<R> rc_L(rho_L), rc_R(rho_R);
-  if (K.low_mach_fix && !(above_low_mach(u_LHS, v_LHS, g, p_L, rho_L) &&
-                          above_low_mach(u_RHS, v_RHS, g, p_R, rho_R))) {
+  R M_LHS, M_RHS;
+  bool low = false;
+  if (kFP32<R> || (K.low_mach_fix && !(above_low_mach(u_LHS, v_LHS, g, p_L, rho_L) &&
+                                       above_low_mach(u_RHS, v_RHS, g, p_R, rho_R)))) {
     R cs_L = Num<R>::sqrt(div_by(g * p_L, rc_L));
     R cs_R = Num<R>::sqrt(div_by(g * p_R, rc_R));
-    R M_LHS = Num<R>::div(Num<R>::sqrt(u_LHS * u_LHS + v_LHS * v_LHS), cs_L);
-    R M_RHS = Num<R>::div(Num<R>::sqrt(u_RHS * u_RHS + v_RHS * v_RHS), cs_R);
-    if (abs_lt(M_LHS, R(0.1)) || abs_lt(M_RHS, R(0.1))) {  // LOW_MACH
-      R f_M = rmin(R(1), rmax(M_LHS, M_RHS));
-      R uLf = half(u_LHS + u_RHS) + half(f_M) * (u_LHS - u_RHS);
-      R uRf = half(u_LHS + u_RHS) - half(f_M) * (u_LHS - u_RHS);
-      R vLf = half(v_LHS + v_RHS) + half(f_M) * (v_LHS - v_RHS);
-      R vRf = half(v_LHS + v_RHS) - half(f_M) * (v_LHS - v_RHS);
-      u_LHS = uLf; u_RHS = uRf; v_LHS = vLf; v_RHS = vRf;
-    }
+    M_LHS = Num<R>::div(Num<R>::sqrt(u_LHS * u_LHS + v_LHS * v_LHS), cs_L);
+    M_RHS = Num<R>::div(Num<R>::sqrt(u_RHS * u_RHS + v_RHS * v_RHS), cs_R);
+    low = K.low_mach_fix && (abs_lt(M_LHS, R(0.1)) || abs_lt(M_RHS, R(0.1)));
+  }
+  if (low) {  // LOW_MACH
+    R f_M = rmin(R(1), rmax(M_LHS, M_RHS));
+    R uLf = half(u_LHS + u_RHS) + half(f_M) * (u_LHS - u_RHS);
+    R uRf = half(u_LHS + u_RHS) - half(f_M) * (u_LHS - u_RHS);
+    R vLf = half(v_LHS + v_RHS) + half(f_M) * (v_LHS - v_RHS);
+    R vRf = half(v_LHS + v_RHS) - half(f_M) * (v_LHS - v_RHS);
+    u_LHS = uLf; u_RHS = uRf; v_LHS = vLf; v_RHS = vRf;
   }
   const R gg = R(K.g_over_gm1);
   R H_L = gg * div_by(p_L, rc_L) + half(u_LHS * u_LHS + v_LHS * v_LHS);
@@ -1042,20 +1207,23 @@ __device__ __forceinline__ void flux_mausmpw(const FluxConsts<R>& K, const Prim<
   const R U_L = DIR == 0 ? u_LHS : v_LHS, U_R = DIR == 0 ? u_RHS : v_RHS;
   const R V_L = DIR == 0 ? v_LHS : u_LHS, V_R = DIR == 0 ? v_RHS : u_RHS;
   const Rcp<R> rc_L(rho_L), rc_R(rho_R);
-  if (K.low_mach_fix && !(above_low_mach(u_LHS, v_LHS, g, p_L, rho_L) &&
-                          above_low_mach(u_RHS, v_RHS, g, p_R, rho_R))) {
+  R M_LHS, M_RHS;
+  bool low = false;
+  if (kFP32<R> || (K.low_mach_fix && !(above_low_mach(u_LHS, v_LHS, g, p_L, rho_L) &&
+                                       above_low_mach(u_RHS, v_RHS, g, p_R, rho_R)))) {
     R cs_L = Num<R>::sqrt(div_by(g * p_L, rc_L));
     R cs_R = Num<R>::sqrt(div_by(g * p_R, rc_R));
-    R M_LHS = Num<R>::div(Num<R>::sqrt(u_LHS * u_LHS + v_LHS * v_LHS), cs_L);
-    R M_RHS = Num<R>::div(Num<R>::sqrt(u_RHS * u_RHS + v_RHS * v_RHS), cs_R);
-    if (abs_lt(M_LHS, R(0.1)) || abs_lt(M_RHS, R(0.1))) {  // LOW_MACH
-      R f_M = rmin(R(1), rmax(M_LHS, M_RHS));
-      R uLf = half(u_LHS + u_RHS) + half(f_M) * (u_LHS - u_RHS);
-      R uRf = half(u_LHS + u_RHS) - half(f_M) * (u_LHS - u_RHS);
-      R vLf = half(v_LHS + v_RHS) + half(f_M) * (v_LHS - v_RHS);
-      R vRf = half(v_LHS + v_RHS) - half(f_M) * (v_LHS - v_RHS);
-      u_LHS = uLf; u_RHS = uRf; v_LHS = vLf; v_RHS = vRf;
-    }
+    M_LHS = Num<R>::div(Num<R>::sqrt(u_LHS * u_LHS + v_LHS * v_LHS), cs_L);
+    M_RHS = Num<R>::div(Num<R>::sqrt(u_RHS * u_RHS + v_RHS * v_RHS), cs_R);
+    low = K.low_mach_fix && (abs_lt(M_LHS, R(0.1)) || abs_lt(M_RHS, R(0.1)));
+  }
+  if (low) {  // LOW_MACH
+    R f_M = rmin(R(1), rmax(M_LHS, M_RHS));
+    R uLf = half(u_LHS + u_RHS) + half(f_M) * (u_LHS - u_RHS);
+    R uRf = half(u_LHS + u_RHS) - half(f_M) * (u_LHS - u_RHS);
+    R vLf = half(v_LHS + v_RHS) + half(f_M) * (v_LHS - v_RHS);
+    R vRf = half(v_LHS + v_RHS) - half(f_M) * (v_LHS - v_RHS);
+    u_LHS = uLf; u_RHS = uRf; v_LHS = vLf; v_RHS = vRf;
   }
   const R gg = R(K.g_over_gm1);
   R H_L = gg * div_by(p_L, rc_L) + half(u_LHS * u_LHS + v_LHS * v_LHS);
@@ -1125,7 +1293,7 @@ __device__ __forceinline__ void flux_mausmpw(const FluxConsts<R>& K, const Prim<
 // SLAU / SLAU2 / SD-SLAU / SD-SLAU2, slau_solver.fypp:332-490.  dpair[6][2]: delta_p1..6 cells.
 template <typename R, int DIR, int VARIANT>
 __device__ __forceinline__ void flux_slau(const FluxConsts<R>& K, const Prim<R>& A, const Prim<R>& B,
-                                          const R dpa[6], const R dpb[6], R F[4]) {
+                                          const R dpa[6], const R dpb[6], R F[4], bool y = false) {
   const R g = R(K.gamma);
   const R EPS = Num<R>::eps;
   const R THRESHOLD = R(5e-3), C_SD1 = R(0.01);
@@ -1140,7 +1308,13 @@ __device__ __forceinline__ void flux_slau(const FluxConsts<R>& K, const Prim<R>&
   R c_bar = half(c_plus + c_minus);
   const Rcp<R> rc_c(c_bar);
   R V_n_bar = Num<R>::div(rho_L * rabs(Vp) + rho_R * rabs(Vm), rho_L + rho_R);
-  R vel2 = half(u_L * u_L + v_L * v_L + u_R * u_R + v_R * v_R);
+  R vel2;
+  if constexpr (kFP32<R>) {
+    vel2 = half(u_L * u_L + v_L * v_L + u_R * u_R + v_R * v_R);
+  } else {  // left to right in x, y order
+    const R uu = u_R * u_R, vv = v_R * v_R;
+    vel2 = half(u_L * u_L + v_L * v_L + (y ? vv : uu) + (y ? uu : vv));
+  }
   R M_hat = rmin(R(1), div_by(Num<R>::sqrt(vel2), rc_c));
   R M_plus = div_by(Vp, rc_c);
   R M_minus = div_by(Vm, rc_c);
@@ -1231,6 +1405,11 @@ template <> __device__ __forceinline__ bool roe_sensor<df>(df a, df b) {
   if (lo > 1e-25f && hi < 1.99f * lo) return false;
   return roe_sensor_slow<df>(a, b);
 }
+// half(s) - x; FP32 as one FMA of the halved sum
+template <typename R> __device__ __forceinline__ R half_less(R s, R x) { return half(s) - x; }
+template <> __device__ __forceinline__ float half_less<float>(float s, float x) {
+  return __fmaf_rn(0.5f, s, -__fmul_rn(x, 1.0f));
+}
 // whether the correction of a quiet sensor, 0 rav cav (...), is a zero that leaves F1 and F2 alone
 __device__ __forceinline__ bool roe_quiet(double F1, double F2, double rav, double cav, double du,
                                           double dut, double cl, double cr) {
@@ -1253,10 +1432,8 @@ __device__ __forceinline__ bool roe_quiet(df F1, df F2, df rav, df cav, df du, d
 // roe_solver.fypp:420-512; optional Harten fix (:529-536).  fh: the five f_h pairs (:495-508).
 template <typename R, int DIR>
 __device__ __forceinline__ void flux_roe(const FluxConsts<R>& K, const Prim<R>& A, const Prim<R>& B,
-                                         const R fa[5], const R fb[5], R F[4]) {
-  // products through Num<R>::mul (the integer pipe on the FP64 path), in the same left-to-right
-  // order as the expressions they spell out
-  auto m = [](R x, R y) { return Num<R>::mul(x, y); };
+                                         const R fa[5], const R fb[5], R F[4], bool y = false) {
+  auto m = [](R x, R y) { return x * y; };
   const R g = R(K.gamma);
   R rl = rabs(A.r), ul = A.u, vl = A.v, pl = rabs(A.p);
   R rr = rabs(B.r), ur = B.u, vr = B.v, pr = rabs(B.p);
@@ -1279,7 +1456,9 @@ __device__ __forceinline__ void flux_roe(const FluxConsts<R>& K, const Prim<R>& 
   auto dotn = [](R x, R y) { return DIR == 0 ? add_mul0(x, y) : add_mul0(y, x); };
   R uv = dotn(uav, vav);
   R du = dotn(ur - ul, vr - vl);
-  R du_trans = DIR == 0 ? add_mul0(vr - vl, rneg(ur - ul)) : add_mul0(rneg(ur - ul), vr - vl);
+  // du_trans = -(du n_y) + dv n_x, of the Cartesian components
+  R du_trans = y ? add_mul0(rneg(vr - vl), ur - ul)
+               : DIR == 0 ? add_mul0(vr - vl, rneg(ur - ul)) : add_mul0(rneg(ur - ul), vr - vl);
   R cs_R = Num<R>::sqrt(div_by(m(g, pr), rc_r));
   R cs_L = Num<R>::sqrt(q_gpl);
   R h1 = rabs(rmin(uv - cav, dotn(ul, vl) - cs_L));
@@ -1312,8 +1491,9 @@ __device__ __forceinline__ void flux_roe(const FluxConsts<R>& K, const Prim<R>& 
   R m3 = (m(h2, hav - m(cav, uv)) + m(h3, q2a) +
           m(h4, m(uav, ur - ul) + m(vav, vr - vl) - m(uv, du)) + m(h5, hav + m(cav, uv)));
   F[0] = half(FR0 + FL0 - m0);
-  F[1] = half(FR1 + FL1 - m1);
-  F[2] = half(FR2 + FL2 - m2);
+  const R S1 = FR1 + FL1 - m1, S2 = FR2 + FL2 - m2;
+  F[1] = half(S1);
+  F[2] = half(S2);
   F[3] = half(FR3 + FL3 - m3);
   // the shear correction: nothing where the pressure sensor is quiet (a zero product leaves the
   // flux as it is; roe_quiet: unless a zero's sign or a NaN would come of it)
@@ -1324,10 +1504,11 @@ __device__ __forceinline__ void flux_roe(const FluxConsts<R>& K, const Prim<R>& 
   const R fmax = fires ? R(1) : R(0);
   R psi = Num<R>::div(rabs(cs_R - cs_L), rmax(cs_R, cs_L));
   // -(du_trans n_y) + psi du n_x and du_trans n_x + psi du n_y
-  const R c1 = DIR == 0 ? add_mul0(m(psi, du), rneg(du_trans)) : add_mul0(rneg(du_trans), m(psi, du));
-  const R c2 = DIR == 0 ? add_mul0(du_trans, m(psi, du)) : add_mul0(m(psi, du), du_trans);
-  F[1] = F[1] - m(m(m(half(fmax), rav), cav), c1);
-  F[2] = F[2] - m(m(m(half(fmax), rav), cav), c2);
+  const R pd = m(psi, du);
+  const R c1 = DIR == 0 ? add_mul0(pd, y ? du_trans : rneg(du_trans)) : add_mul0(rneg(du_trans), pd);
+  const R c2 = DIR == 0 ? add_mul0(y ? rneg(du_trans) : du_trans, pd) : add_mul0(pd, du_trans);
+  F[1] = half_less(S1, m(m(m(half(fmax), rav), cav), c1));
+  F[2] = half_less(S2, m(m(m(half(fmax), rav), cav), c2));
 }
 
 // AUSM+-up (basic), ausm_plus_solver.f90:499-643 + upwinding of the commented driver :313-325.
@@ -1392,9 +1573,9 @@ __device__ __forceinline__ void flux_ausm_up(const FluxConsts<R>& K, const Prim<
 template <typename R, int DIR>
 __device__ __forceinline__ void flux_hllc(const FluxConsts<R>& K, const Prim<R>& A, const Prim<R>& B,
                                           R F[4]) {
-  // products through Num<R>::mul: on the FP64 path they run on the integer pipe (mul_rn), in the
-  // same left-to-right order as the expressions they spell out
-  auto m = [](R x, R y) { return Num<R>::mul(x, y); };
+  // (the products on the integer pipe, which relieved an FP64 pipe 76 % busy in an earlier form of
+  // this kernel, are 6 % slower now: 31.3 against 29.4 ms a step at 4096^2)
+  auto m = [](R x, R y) { return x * y; };
   const R g = R(K.gamma);
   R qnL = DIR == 0 ? A.u : A.v, qtL = DIR == 0 ? A.v : A.u;
   R qnR = DIR == 0 ? B.u : B.v, qtR = DIR == 0 ? B.v : B.u;
@@ -1405,10 +1586,17 @@ __device__ __forceinline__ void flux_hllc(const FluxConsts<R>& K, const Prim<R>&
   const R gf = R(K.hllc_gf);
   // SL = qnL - cL qL, SR = qnR + cR qR with q = 1 (then c q is c) unless p_star exceeds p
   R SL, SR;
-  if (le(p_star, A.p)) SL = qnL - cL;
-  else SL = qnL - m(cL, Num<R>::sqrt(R(1) + m(gf, Num<R>::div(p_star, A.p) - R(1))));
-  if (le(p_star, B.p)) SR = qnR + cR;
-  else SR = qnR + m(cR, Num<R>::sqrt(R(1) + m(gf, Num<R>::div(p_star, B.p) - R(1))));
+  if constexpr (kFP32<R>) {  // selects: no branches in the FP32 chain
+    const R sL = qnL - m(cL, Num<R>::sqrt(R(1) + m(gf, Num<R>::div(p_star, A.p) - R(1))));
+    const R sR = qnR + m(cR, Num<R>::sqrt(R(1) + m(gf, Num<R>::div(p_star, B.p) - R(1))));
+    SL = le(p_star, A.p) ? qnL - cL : sL;
+    SR = le(p_star, B.p) ? qnR + cR : sR;
+  } else {
+    if (le(p_star, A.p)) SL = qnL - cL;
+    else SL = qnL - m(cL, Num<R>::sqrt(R(1) + m(gf, Num<R>::div(p_star, A.p) - R(1))));
+    if (le(p_star, B.p)) SR = qnR + cR;
+    else SR = qnR + m(cR, Num<R>::sqrt(R(1) + m(gf, Num<R>::div(p_star, B.p) - R(1))));
+  }
   // the total energy of the side the flux is taken from (only that one is needed)
   auto energy = [&](const Prim<R>& S) {
     return div_by(S.p, gm1_of(K)) + m(half(S.r), m(S.u, S.u) + m(S.v, S.v));

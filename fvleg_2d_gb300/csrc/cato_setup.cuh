@@ -4,6 +4,7 @@
 #pragma once
 
 #include "../../include/cato_gpu.h"
+#include "cato_launch.cuh"
 #include "cato_physics.cuh"
 
 namespace cato {
@@ -30,21 +31,48 @@ inline FluxConsts<double> flux_consts_of(const cato_config& c) {
   return K;
 }
 
-// Default single-grid launch shape: wide strips for large grids; narrow strips and short marches
-// for small grids so that the launch fills the 152 SMs; narrow strips when a wide one would be
-// wider than the grid with its halo.
-struct LaunchShape {
-  int threads;
-  int rows_per_cta;
-};
-inline LaunchShape default_shape(int ni, int nj, int ng) {
-  const long long cells = (long long)ni * nj;
-  LaunchShape p;
-  if (cells < 200000) { p.threads = 64; p.rows_per_cta = 8; }
-  else if (cells < 4000000) { p.threads = 128; p.rows_per_cta = 32; }
-  else { p.threads = 128; p.rows_per_cta = 64; }
-  if (p.threads - 2 * ng > ni + 2 * ng) p.threads = 64;
-  return p;
+// Default single-grid launch shape.
+//
+// FP32 strips: as many rows per CTA (64 .. 1) as leave the GPU about full; a strip of r rows pays
+// for r + 1.5 of them.  Measured at 64 columns, best of 1 .. 64 rows: 64 x 48 and 256^2: 1 - 2
+// rows, 512^2: 4, 1024^2: 16, 4096^2: 64 (1487 us a step at 128 x 64 against 2200 at 64 x 4; at
+// 1024^2 128 us at 64 x 16 against 178 at 128 x 32).
+//
+// Edge-parallel tiles (FP64, double-float): 32 columns and a single block of 4, 2 or 1 rows while
+// that leaves SMs idle otherwise (the chain of a block is the time of the launch: 64 x 48 HLLC
+// 75 us a step at 1 row, 85 at 4), else 64 columns, blocks of 4 rows and as many blocks per CTA
+// as leave about four waves of the two resident CTAs (1024^2: 2094 us at 8 rows, 2144 at 32;
+// 4096^2: 29.3 ms at 32 rows, 30.6 at 8).
+constexpr int kSMs = 152;
+inline StageShape default_shape(int ni, int nj, int ng, int precision) {
+  auto tiles = [&](int columns, int rows) {
+    const int W = columns - 2 * ng;
+    return (long long)((ni + W - 1) / W) * ((nj + rows - 1) / rows);
+  };
+  StageShape s;
+  if (precision == CATO_MIXED) {
+    s.threads = 64;
+    s.rows = 64;
+    while (s.rows > 1 && tiles(64, s.rows) < 7LL * kSMs) s.rows /= 2;
+    if (s.rows >= 32) s.threads = 128;
+    if (s.threads - 2 * ng > ni + 2 * ng) s.threads = 64;
+    s.width = s.threads;
+    return s;
+  }
+  if (tiles(64, 4) < 2LL * kSMs) {
+    s.width = 64;
+    s.threads = 32;
+    s.block = 4;
+    while (s.block > 1 && tiles(32, s.block) < kSMs * 7 / 8) s.block /= 2;
+    s.rows = s.block;
+    return s;
+  }
+  s.width = 128;
+  s.threads = 64;
+  s.block = 4;
+  s.rows = 32;
+  while (s.rows > 4 && tiles(64, s.rows) < 7LL * kSMs) s.rows /= 2;
+  return s;
 }
 
 // reconstruction kind of a limiter id: 0 = TVD2, 3 = MLP3, 5 = MLP5

@@ -2,12 +2,10 @@
 // recovery, MUSCL/MLP reconstruction, edge fluxes, flux divergence and the RK stage combine in
 // one pass over HBM, with the CFL dt min-reduction and the state checks fused into the last stage.
 //
-// Work decomposition ("marching strip"): a CTA of T threads owns a strip of W = T - 2*NG output
-// columns and marches over rows_per_cta rows.  Thread t always handles column x0 - NG + t, so a
-// row of primitives (T cells incl. the x-halo) is produced by one coalesced row load.  Shared
-// memory keeps a ring of the last 2*NG primitive rows, the i-edge fluxes of the current row and
-// the j-edge fluxes below/above it; each row costs two __syncthreads.  Every primitive is
-// computed once per stage (x-halo overhead 2*NG/T, y-halo 2*NG/rows_per_cta).
+// Work decomposition.  FP32: a CTA of T threads owns a strip of W = T - 2*NG output columns and
+// marches over rows_per_cta rows; thread t always handles column x0 - NG + t (stage_tile_tvd for
+// the TVD2 limiters, stage_tile for the others).  FP64 and double-float, whose chains are ten times
+// longer: several warps per column segment, one row of edges each (edge_tile).
 //
 // Ghost cells are never stored: a ghost row/column index maps to its source interior cell
 // (zero-gradient copy, symmetry mirror with the normal velocity negated, periodic wrap).  This
@@ -110,66 +108,23 @@ template <int RING> __device__ __forceinline__ int slot_of(int row) {
 }
 
 // Row bases of the shared-memory ring for rows center-2 .. center+3 (each row: [var][col]).
-template <typename R, int RING>
-__device__ __forceinline__ void ring_rows(R* ring, int T, int center, const R* rp[6]) {
+template <int RING>
+__device__ __forceinline__ void ring_rows(const float* ring, int T, int center,
+                                          const float* rp[6]) {
 #pragma unroll
   for (int k = 0; k < 6; ++k) rp[k] = ring + slot_of<RING>(center + k - 2) * 4 * T;
 }
 
-// ---------------------------------------------------------------------------------------------
-// one edge: reconstruct the four primitives from the ring and evaluate the flux
-// ---------------------------------------------------------------------------------------------
-template <typename R, int NG, int FLUX, int RECON, int DIR>
-__device__ __forceinline__ void edge_flux(const R* const rp[6], int T, int lim, int col,
-                                          const FluxConsts<R>& K, R F[4]) {
-  // stencil sample at normal offset n and tangential offset t from the edge's left cell;
-  // rp[k] is the ring row (edge row) + k - 2
-  auto Q = [&](int var, int n, int t) -> R {
-    return DIR == 0 ? rp[t + 2][var * T + col + n] : rp[n + 2][var * T + col + t];
-  };
-  R Lv[4], Rv[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (RECON == 0) {
-      if constexpr (Prec<R>::kind == 0) {
-        const EdgePair e = recon_tvd2_f64(lim, Q(k, -1, 0), Q(k, 0, 0), Q(k, 1, 0), Q(k, 2, 0));
-        Lv[k] = e.L;
-        Rv[k] = e.R;
-      } else {
-        recon_tvd2<R>(lim, Q(k, -1, 0), Q(k, 0, 0), Q(k, 1, 0), Q(k, 2, 0), Lv[k], Rv[k]);
-      }
-    } else {
-      R qm2 = RECON == 5 ? Q(k, -2, 0) : R(0), qp3 = RECON == 5 ? Q(k, 3, 0) : R(0);
-      if constexpr (Prec<R>::kind == 0) {
-        const EdgePair e = recon_mlp_f64<RECON>(qm2, Q(k, -1, 0), Q(k, 0, 0), Q(k, 1, 0),
-                                                Q(k, 2, 0), qp3, Q(k, 0, 1), Q(k, 0, -1),
-                                                Q(k, 1, 1), Q(k, 1, -1));
-        Lv[k] = e.L;
-        Rv[k] = e.R;
-      } else {
-        recon_mlp<R, RECON>(qm2, Q(k, -1, 0), Q(k, 0, 0), Q(k, 1, 0), Q(k, 2, 0), qp3,
-                            Q(k, 0, 1), Q(k, 0, -1), Q(k, 1, 1), Q(k, 1, -1), Lv[k], Rv[k]);
-      }
-    }
-  }
-  Prim<R> A = {Lv[0], Lv[1], Lv[2], Lv[3]}, B = {Rv[0], Rv[1], Rv[2], Rv[3]};
-  // cell pressures in reference (i, j) terms: P(di, dj) = p(i+di, j+dj), (i, j) = left cell
-  auto P = [&](int di, int dj) -> R { return DIR == 0 ? Q(3, di, dj) : Q(3, dj, di); };
-  if (FLUX == FLUX_AUSMPW || FLUX == FLUX_M_AUSMPW) {
+// the flux of one edge from its left and right states; P(di, dj): the pressure of cell (i+di, j+dj)
+// in reference terms, (i, j) the edge's left cell
+template <typename R, int FLUX, int DIR, typename PF>
+__device__ __forceinline__ void flux_of(const FluxConsts<R>& K, const Prim<R>& A, const Prim<R>& B,
+                                        PF P, R F[4]) {
+  if (FLUX == FLUX_AUSMPW) {
     R pc[4];
     if (DIR == 0) { pc[0] = P(0, -1); pc[1] = P(1, -1); pc[2] = P(0, 1); pc[3] = P(1, 1); }
     else { pc[0] = P(1, 0); pc[1] = P(1, 1); pc[2] = P(-1, 0); pc[3] = P(-1, 1); }
-    if constexpr (FLUX == FLUX_M_AUSMPW) {
-      // the superbee edge states of the second interpolator (m_ausmpw_plus_solver.fypp:163-167)
-      R Ls[4], Rs[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        recon_tvd2<R>(LIM_SUPERBEE, Q(k, -1, 0), Q(k, 0, 0), Q(k, 1, 0), Q(k, 2, 0), Ls[k], Rs[k]);
-      Prim<R> As = {Ls[0], Ls[1], Ls[2], Ls[3]}, Bs = {Rs[0], Rs[1], Rs[2], Rs[3]};
-      flux_mausmpw<R, DIR>(K, A, B, As, Bs, pc, F);
-    } else {
-      flux_ausmpw<R, DIR>(K, A, B, pc, F);
-    }
+    flux_ausmpw<R, DIR>(K, A, B, pc, F);
   } else if (FLUX == FLUX_SLAU || FLUX == FLUX_SLAU2 || FLUX == FLUX_SD_SLAU ||
              FLUX == FLUX_SD_SLAU2) {
     R pa[6], pb[6];
@@ -212,6 +167,144 @@ __device__ __forceinline__ void edge_flux(const R* const rp[6], int T, int lim, 
   } else {
     flux_hllc<R, DIR>(K, A, B, F);
   }
+}
+
+// ---------------------------------------------------------------------------------------------
+// one edge: reconstruct the four primitives from the ring and evaluate the flux
+// ---------------------------------------------------------------------------------------------
+// FP32, one copy per direction
+template <int NG, int FLUX, int RECON, int DIR>
+__device__ __forceinline__ void edge_flux(const float* const rp[6], int T, int lim, int col,
+                                          const FluxConsts<float>& K, float F[4]) {
+  // stencil sample at normal offset n and tangential offset t from the edge's left cell;
+  // rp[k] is the ring row (edge row) + k - 2
+  auto Q = [&](int var, int n, int t) -> float {
+    return DIR == 0 ? rp[t + 2][var * T + col + n] : rp[n + 2][var * T + col + t];
+  };
+  float Lv[4], Rv[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (RECON == 0) {
+      recon_tvd2<float>(lim, Q(k, -1, 0), Q(k, 0, 0), Q(k, 1, 0), Q(k, 2, 0), Lv[k], Rv[k]);
+    } else {
+      float qm2 = RECON == 5 ? Q(k, -2, 0) : 0.0f, qp3 = RECON == 5 ? Q(k, 3, 0) : 0.0f;
+      recon_mlp<float, RECON>(qm2, Q(k, -1, 0), Q(k, 0, 0), Q(k, 1, 0), Q(k, 2, 0), qp3,
+                              Q(k, 0, 1), Q(k, 0, -1), Q(k, 1, 1), Q(k, 1, -1), Lv[k], Rv[k]);
+    }
+  }
+  Prim<float> A = {Lv[0], Lv[1], Lv[2], Lv[3]}, B = {Rv[0], Rv[1], Rv[2], Rv[3]};
+  // cell pressures in reference (i, j) terms: P(di, dj) = p(i+di, j+dj), (i, j) = left cell
+  auto P = [&](int di, int dj) -> float { return DIR == 0 ? Q(3, di, dj) : Q(3, dj, di); };
+  if constexpr (FLUX == FLUX_M_AUSMPW) {
+    float pc[4];
+    if (DIR == 0) { pc[0] = P(0, -1); pc[1] = P(1, -1); pc[2] = P(0, 1); pc[3] = P(1, 1); }
+    else { pc[0] = P(1, 0); pc[1] = P(1, 1); pc[2] = P(-1, 0); pc[3] = P(-1, 1); }
+    // the superbee edge states of the second interpolator (m_ausmpw_plus_solver.fypp:163-167)
+    float Ls[4], Rs[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      recon_tvd2<float>(LIM_SUPERBEE, Q(k, -1, 0), Q(k, 0, 0), Q(k, 1, 0), Q(k, 2, 0), Ls[k], Rs[k]);
+    Prim<float> As = {Ls[0], Ls[1], Ls[2], Ls[3]}, Bs = {Rs[0], Rs[1], Rs[2], Rs[3]};
+    flux_mausmpw<float, DIR>(K, A, B, As, Bs, pc, F);
+  } else {
+    flux_of<float, FLUX, DIR>(K, A, B, P, F);
+  }
+}
+
+// FP64 and double-float: one copy for both directions, which halves the code (these kernels are
+// sensitive to the instruction cache).  y: an edge along j; prim: shared memory, ro[k]: offset of
+// this column in row (edge row) + k - 2; a variable is T apart.  The fluxes run in the edge's
+// frame: the states' u and v are exchanged before, and the momentum fluxes after.
+template <int RECON>
+__device__ __forceinline__ EdgePair recon_edge(int lim, const double q[10]) {
+  if constexpr (RECON == 0) return recon_tvd2_f64(lim, q[1], q[2], q[3], q[4]);
+  else
+    return recon_mlp_f64<RECON>(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7], q[8], q[9]);
+}
+template <int RECON> __device__ __forceinline__ DfPair recon_edge(int lim, const df q[10]) {
+  if constexpr (RECON == 0) return recon_tvd2_df(lim, q[1], q[2], q[3], q[4]);
+  else
+    return recon_mlp_df_ool<RECON>(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7], q[8], q[9]);
+}
+template <typename R, int FLUX, int RECON>
+__device__ __forceinline__ void edge_flux_any(const R* prim, const int ro[6], int T, int lim, bool y,
+                                              const FluxConsts<R>& K, R F[4]) {
+  // offset of the sample n cells along and t cells across the edge normal
+  auto at = [&](int n, int t) { return y ? ro[n + 2] + t : ro[t + 2] + n; };
+  int o[10];
+  o[0] = RECON == 5 ? at(-2, 0) : 0;
+  o[1] = at(-1, 0);
+  o[2] = at(0, 0);
+  o[3] = at(1, 0);
+  o[4] = at(2, 0);
+  o[5] = RECON == 5 ? at(3, 0) : 0;
+  o[6] = at(0, 1);
+  o[7] = at(0, -1);
+  o[8] = at(1, 1);
+  o[9] = at(1, -1);
+  R Lv[4], Rv[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    R q[10];
+#pragma unroll
+    for (int m = 0; m < 10; ++m)
+      q[m] = (RECON == 0 && (m == 0 || m > 4)) || (RECON == 3 && (m == 0 || m == 5))
+                 ? R(0)
+                 : prim[o[m] + k * T];
+    const auto e = recon_edge<RECON>(lim, q);
+    Lv[k] = e.L;
+    Rv[k] = e.R;
+  }
+  const Prim<R> A = {Lv[0], y ? Lv[2] : Lv[1], y ? Lv[1] : Lv[2], Lv[3]};
+  const Prim<R> B = {Rv[0], y ? Rv[2] : Rv[1], y ? Rv[1] : Rv[2], Rv[3]};
+  // cell pressures n along and t across the normal, with t counted so that the reference's lists
+  // (ausmpw_plus_solver.fypp:430-442, slau_solver.fypp:410-428) come out in their order
+  [[maybe_unused]] auto P = [&](int n, int t) -> R {
+    return prim[(y ? ro[n + 2] - t : ro[t + 2] + n) + 3 * T];
+  };
+  R G[4];
+  if constexpr (FLUX == FLUX_AUSMPW) {
+    const R pc[4] = {P(0, -1), P(1, -1), P(0, 1), P(1, 1)};
+    flux_ausmpw<R, 0>(K, A, B, pc, G);
+  } else if constexpr (FLUX == FLUX_M_AUSMPW) {
+    const R pc[4] = {P(0, -1), P(1, -1), P(0, 1), P(1, 1)};
+    // the superbee edge states of the second interpolator (m_ausmpw_plus_solver.fypp:163-167)
+    R Ls[4], Rs[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      R q[10] = {};
+#pragma unroll
+      for (int m = 1; m < 5; ++m) q[m] = prim[o[m] + k * T];
+      const auto e = recon_edge<0>(LIM_SUPERBEE, q);
+      Ls[k] = e.L;
+      Rs[k] = e.R;
+    }
+    const Prim<R> As = {Ls[0], y ? Ls[2] : Ls[1], y ? Ls[1] : Ls[2], Ls[3]};
+    const Prim<R> Bs = {Rs[0], y ? Rs[2] : Rs[1], y ? Rs[1] : Rs[2], Rs[3]};
+    flux_mausmpw<R, 0>(K, A, B, As, Bs, pc, G);
+  } else if constexpr (FLUX == FLUX_SD_SLAU || FLUX == FLUX_SD_SLAU2) {
+    const R l = P(0, 0), r = P(1, 0);
+    const R pa[6] = {P(0, 1), P(-1, 0), P(0, -1), P(1, -1), P(2, 0), P(1, 1)};
+    const R pb[6] = {l, l, l, r, r, r};
+    flux_slau<R, 0, FLUX>(K, A, B, pa, pb, G, y);
+  } else if constexpr (FLUX == FLUX_SLAU || FLUX == FLUX_SLAU2) {
+    const R none[6] = {};
+    flux_slau<R, 0, FLUX>(K, A, B, none, none, G, y);
+  } else if constexpr (FLUX == FLUX_ROE) {
+    // roe_solver.fypp:496-506; the last two pairs differ between the directions
+    const R l = P(0, 0), r = P(1, 0), lp = P(0, 1), lm = P(0, -1), rp = P(1, 1), rm = P(1, -1);
+    const R fa[5] = {l, l, l, y ? r : lp, y ? r : lm};
+    const R fb[5] = {r, lp, lm, rp, rm};
+    flux_roe<R, 0>(K, A, B, fa, fb, G, y);
+  } else if constexpr (FLUX == FLUX_AUSM_UP) {
+    flux_ausm_up<R, 0>(K, A, B, G);
+  } else {
+    flux_hllc<R, 0>(K, A, B, G);
+  }
+  F[0] = G[0];
+  F[1] = y ? G[2] : G[1];
+  F[2] = y ? G[1] : G[2];
+  F[3] = G[3];
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -296,12 +389,210 @@ __device__ __forceinline__ void src_to_prim(const StageArgs& A, const RowSrc<R>&
 // ---------------------------------------------------------------------------------------------
 // the kernel
 // ---------------------------------------------------------------------------------------------
-// One tile: columns [bx*W, bx*W + W) x rows [by*rows_per_cta, ...) of one instance.
+// What a thread keeps for its column during a tile.
+template <typename R> struct ColumnConsts {
+  double cc;  // coef * dt
+  float ccf, cfl_f;        // mixed: the stage increment c L in FP32
+  float idx_col, idy_uni;  // FP32 reciprocal cell width of the column / row height (uniform grid)
+  df dx_inv, dy_inv, cfl_df, cc_df;  // mixed_df constants of the update
+  double dt_loc;           // smallest CFL dt and status bits of the column's new states
+  int st_loc;
+
+  template <bool EXT> __device__ __forceinline__ void init(const StageArgs& A, int gx) {
+    cc = A.coef * *A.dt;
+    ccf = (float)cc;
+    cfl_f = (float)A.cfl;
+    if constexpr (Prec<R>::kind == 2) {
+      dx_inv = to_df(A.G.rdxc ? A.G.rdxc[min(max(gx, 0), A.ni - 1)] : 1.0 / A.G.dx);
+      dy_inv = to_df(1.0 / A.G.dy);
+      cfl_df = to_df(A.cfl);
+      cc_df = to_df(cc);
+    }
+    if constexpr (Prec<R>::kind == 1) {
+      idx_col = (EXT && A.G.rdxf) ? A.G.rdxf[min(max(gx, 0), A.ni - 1)] : (float)(1.0 / A.G.dx);
+      idy_uni = (float)(1.0 / A.G.dy);  // one FP64 division per thread, not per row
+    }
+    dt_loc = INFINITY;
+    st_loc = 0;
+  }
+  // mixed_df on a rectilinear grid: the reciprocal height of row j
+  __device__ __forceinline__ void set_row(const StageArgs& A, int j) {
+    if (A.G.rdyc) dy_inv = to_df(A.G.rdyc[j]);
+  }
+};
+
+// The operands of a cell's stage combine.
+__device__ __forceinline__ void load_operands(const StageArgs& A, size_t cidx, double ua[4],
+                                              double uk[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    ua[k] = A.Ua[k] ? A.Ua[k][cidx] : 0.0;  // may alias Uo: plain load, read before write
+    uk[k] = (A.kind == 1) ? __ldg(A.Uk[k] + cidx) : 0.0;
+  }
+}
+
+// FP64 and double-float: the divergence of variable k of a cell and its stage combine, from the
+// fluxes of the cell's right, left, upper and lower edge.
+template <typename R>
+__device__ __forceinline__ double combine_var(const StageArgs& A, const ColumnConsts<R>& C,
+                                              [[maybe_unused]] const Geom& cg,
+                                              [[maybe_unused]] const Rcp<double>& vol, int k,
+                                              size_t cidx, double ua, double uk, R Fi, R Fim, R Fj,
+                                              R Fjm) {
+  double r;
+  if constexpr (Prec<R>::kind == 0) {
+    double L = divergence_fp64(Fi, Fim, Fj, Fjm, cg, vol);
+    if (k == 3 && A.src_q) L = L + A.src_q[cidx];
+    if (A.kind == 2) {
+      r = L;
+    } else if (A.kind == 0) {
+      r = ua + __dmul_rn(L, C.cc);
+      if (abs_lt(r, Num<double>::eps)) r = 0.0;
+    } else {
+      double s = __dmul_rn(ua, A.a) + __dmul_rn(uk, A.b);
+      if (abs_lt(s, Num<double>::eps)) s = 0.0;
+      r = s + __dmul_rn(L, C.cc);
+      if (abs_lt(r, Num<double>::eps)) r = 0.0;
+    }
+  } else {
+    // double-float divergence (pairs on the FP32 pipe) carried to FP64 once; the RK
+    // accumulation in FP64: U^n + c L, or a U^n + b U^k + c L as two FP64 FMAs with the
+    // increment c L formed in double-float: three FP64 operations per variable instead
+    // of six (stages 2 and 3 of SSP-RK3 on the 4096^2 quadrant: 6 % faster)
+    const df Ld = -((Fi - Fim) * C.dx_inv + (Fj - Fjm) * C.dy_inv);
+    const bool src = k == 3 && A.src_q;
+    if (A.kind == 2) {
+      r = from_df(Ld);
+      if (src) r = r + A.src_q[cidx];
+    } else if (A.kind == 0) {
+      double L = from_df(Ld);
+      if (src) L = L + A.src_q[cidx];
+      r = ua + __dmul_rn(L, C.cc);
+      if (abs_lt(r, Num<double>::eps)) r = 0.0;
+    } else {
+      const double d = src ? __dmul_rn(from_df(Ld) + A.src_q[cidx], C.cc)
+                           : from_df(Ld * C.cc_df);
+      r = fma(uk, A.b, fma(ua, A.a, d));
+      if (abs_lt(r, Num<double>::eps)) r = 0.0;
+    }
+  }
+  return r;
+}
+
+// The CFL dt and the checks of a cell's new state (the last stage).
+template <typename R, bool EXT>
+__device__ __forceinline__ void check_state(const StageArgs& A, ColumnConsts<R>& C,
+                                            [[maybe_unused]] const Geom& cg,
+                                            [[maybe_unused]] int j, const double un[4]) {
+  [[maybe_unused]] const R g = R(A.gamma), g1 = R(A.gamma - 1.0);
+  // CFL dt of the new state (get_timestep, mod_fluid.f90:554-558) and the sanity checks
+  if constexpr (Prec<R>::kind == 0) {
+    double u, v, p, cs;
+    prim_from_cons(A.gamma, A.gamma - 1.0, un[0], un[1], un[2], un[3], u, v, p, cs);
+    double d = div_rn(A.cfl, div_rn(rabs(u) + cs, cg.dx) + div_rn(rabs(v) + cs, cg.dy));
+    if (d_less(d, C.dt_loc)) C.dt_loc = d;
+    if (d_isnan(un[0]) || d_isnan(u) || d_isnan(v) || d_isnan(p)) C.st_loc |= ST_NAN;
+    if (lt0(un[0])) C.st_loc |= ST_NEG_DENSITY;
+    if (lt0(p)) C.st_loc |= ST_NEG_PRESSURE;
+  } else if constexpr (Prec<R>::kind == 2) {
+    df u, v, p, cs;
+    const df rE = to_df(un[3]);
+    prim_from_cons(g, g1, to_df(un[0]), to_df(un[1]), to_df(un[2]), rE, u, v, p, cs, true);
+    if (near_vacuum(p.hi, rE.hi, 1e-4f)) {  // the FP64 recovery decides p and its sign
+      double u64, v64, p64;
+      prim_from_cons_f64(A.gamma, un[0], un[1], un[2], un[3], u64, v64, p64);
+      u = to_df(u64); v = to_df(v64); p = to_df(p64);
+      cs = df_sqrt(g * df_div(p, to_df(un[0])));
+    }
+    const df d = df_div(C.cfl_df, (df_abs(u) + cs) * C.dx_inv + (df_abs(v) + cs) * C.dy_inv);
+    const double dd = from_df(d);
+    if (dd > 0.0 && dd < C.dt_loc) C.dt_loc = dd;
+    if (isnan(un[0]) || isnan(u.hi) || isnan(v.hi) || isnan(p.hi)) C.st_loc |= ST_NAN;
+    if (un[0] < 0.0) C.st_loc |= ST_NEG_DENSITY;
+    if (p.hi < 0.0f) C.st_loc |= ST_NEG_PRESSURE;
+  } else {
+    const float4 uf = make_float4(d2f_fast(un[0]), d2f_fast(un[1]), d2f_fast(un[2]),
+                                  d2f_fast(un[3]));
+    float u, v, p, cs;
+    prim_from_cons(g, g1, uf.x, uf.y, uf.z, uf.w, u, v, p, cs);
+    float d = C.cfl_f / ((fabsf(u) + cs) * C.idx_col +
+                       (fabsf(v) + cs) * ((EXT && A.G.rdyf) ? A.G.rdyf[j] : C.idy_uni));
+    double dd = f2d_int(d);
+    if (__double_as_longlong(dd) < __double_as_longlong(C.dt_loc) && d > 0.0f) C.dt_loc = dd;
+    // NaN and sign tests on the FP64 state itself (the fast conversion keeps neither)
+    if (d_isnan(un[0]) || d_isnan(un[1]) || d_isnan(un[2]) || d_isnan(un[3]) ||
+        isnan(u) || isnan(v) || isnan(p))
+      C.st_loc |= ST_NAN;
+    if (lt0(un[0])) C.st_loc |= ST_NEG_DENSITY;
+    if (p < 0.0f) C.st_loc |= ST_NEG_PRESSURE;
+  }
+}
+
+// FP32: one cell's divergence, stage combine and (in the last stage) CFL dt and state checks.
+template <bool EXT>
+__device__ __forceinline__ void update_cell(const StageArgs& A, ColumnConsts<float>& C, int gx, int j,
+                                            size_t cidx, const double ua[4], const double uk[4],
+                                            const float Fi_[4], const float Fim_[4], const float Fj_[4],
+                                            const float Fjm_[4]) {
+  double un[4];
+  // the cell's metrics (constants on a uniform grid)
+  const Geom cg = cell_geom(A.G, gx, j);
+  // FP32 divergence and stage increment c L; the stage combine (the RK accumulation)
+  // in FP64
+  const float idx_f = C.idx_col;
+  const float idy_f = (EXT && A.G.rdyf) ? A.G.rdyf[j] : C.idy_uni;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    float Fi = Fi_[k], Fim = Fim_[k], Fj = Fj_[k], Fjm = Fjm_[k];
+    float Lf = -((Fi - Fim) * idx_f + (Fj - Fjm) * idy_f);
+    if (EXT && k == 3 && A.src_q) Lf = Lf + d2f_int(A.src_q[cidx]);
+    double r;
+    if (A.kind == 2) r = f2d_int(Lf);
+    else if (A.kind == 0) r = ua[k] + f2d_int(Lf * C.ccf);
+    else r = fma(uk[k], A.b, fma(ua[k], A.a, f2d_int(Lf * C.ccf)));
+    un[k] = r;
+    A.Uo[k][cidx] = r;
+  }
+  if (A.last) check_state<float, EXT>(A, C, cg, j, un);
+}
+
+// The column's CFL dt and status into the step control.
+template <typename R>
+__device__ __forceinline__ void reduce_column(const StageArgs& A, const ColumnConsts<R>& C) {
+  double dt_loc = C.dt_loc;
+  int st_loc = C.st_loc;
+  const int t = threadIdx.x;
+  if (!A.last) return;
+  // block min of dt (bits of positive doubles order as unsigned integers) and status OR
+  unsigned long long bits =
+      (dt_loc > 0.0) ? (unsigned long long)__double_as_longlong(dt_loc) : ~0ULL;
+  for (int o = 16; o > 0; o >>= 1) {
+    unsigned long long ob = __shfl_xor_sync(0xffffffffu, bits, o);
+    bits = ob < bits ? ob : bits;
+    st_loc |= __shfl_xor_sync(0xffffffffu, st_loc, o);
+  }
+  if ((t & 31) == 0) {
+    if (bits != ~0ULL) atomicMin(A.dt_min, bits);
+    if (st_loc) atomicOr(A.status, st_loc);
+  }
+}
+
+// How a column's samples are made: 0 interior / mapped ghost, 1 +x outlet ghost column, 2 +x
+// pressure-input ghost column (the lowest-priority BCs).
+template <bool EXT> __device__ __forceinline__ int column_mode(const StageArgs& A, int gx) {
+  return gx < A.ni ? 0
+         : A.bc[SIDE_PX] == BC_OUTLET
+             ? 1
+             : (EXT && A.bc[SIDE_PX] == BC_PRESSURE_INPUT ? 2 : 0);
+}
+
+// FP32: one tile: columns [bx*W, bx*W + W) x rows [by*rows_per_cta, ...) of one instance.
 // EXT = false compiles out the rectilinear metrics, the energy source and the pressure-input
 // ghost columns (a uniform grid without them); the issue-bound FP32 path uses it whenever it can.
-template <typename R, int NG, int FLUX, int RECON, bool EXT = true>
-__device__ __forceinline__ void stage_tile(const StageArgs& A, const FluxConsts<R>& K, int bx,
+template <int NG, int FLUX, int RECON, bool EXT>
+__device__ __forceinline__ void stage_tile(const StageArgs& A, const FluxConsts<float>& K, int bx,
                                            int by, unsigned char* smem_raw) {
+  using R = float;
   constexpr int RING = 2 * NG;
   const int T = blockDim.x, W = T - 2 * NG, t = threadIdx.x;
   const int x0 = bx * W;
@@ -315,31 +606,12 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, const FluxConsts<
   const R g = R(A.gamma), g1 = R(A.gamma - 1.0);
   bool flipx;
   const int sx = map_index(min(gx, A.ni + NG - 1), A.ni, A.bc[SIDE_MX], A.bc[SIDE_PX], flipx);
-  // +x outlet / pressure-input ghost columns get the boundary state (lowest-priority BCs)
-  const int xmode = gx < A.ni ? 0
-                    : (A.bc[SIDE_PX] == BC_OUTLET
-                           ? 1
-                           : (EXT && A.bc[SIDE_PX] == BC_PRESSURE_INPUT ? 2 : 0));
+  const int xmode = column_mode<EXT>(A, gx);
   const bool in_i_edge = (t >= NG - 1) && (t <= NG + W - 1) && (gx <= A.ni - 1);
   const bool in_cell = (t >= NG) && (t <= NG + W - 1) && (gx < A.ni);
-  const double dt = *A.dt;
-  const double cc = A.coef * dt;
-  [[maybe_unused]] const float ccf = (float)cc;  // mixed: the stage increment c L in FP32
-  [[maybe_unused]] const float cfl_f = (float)A.cfl;
+  ColumnConsts<R> C;
+  C.template init<EXT>(A, gx);
   const R* rp[6];
-  // mixed_df constants of the update (unused by the other paths)
-  [[maybe_unused]] df dx_inv, dy_inv, cfl_df, cc_df;
-  if constexpr (Prec<R>::kind == 2) {
-    dx_inv = to_df(A.G.rdxc ? A.G.rdxc[min(max(gx, 0), A.ni - 1)] : 1.0 / A.G.dx);
-    dy_inv = to_df(1.0 / A.G.dy);
-    cfl_df = to_df(A.cfl);
-    cc_df = to_df(cc);
-  }
-  // FP32 reciprocal cell width of this thread's column (mixed path)
-  [[maybe_unused]] const float idx_col =
-      (EXT && A.G.rdxf) ? A.G.rdxf[min(max(gx, 0), A.ni - 1)] : (float)(1.0 / A.G.dx);
-  // FP32 reciprocal row height of a uniform grid (one FP64 division per thread, not per row)
-  [[maybe_unused]] const float idy_uni = (float)(1.0 / A.G.dy);
 
   // prologue: rows y0-NG .. y0+NG-1
   for (int r = y0 - NG; r < y0 + NG; ++r) {
@@ -354,8 +626,8 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, const FluxConsts<
   __syncthreads();
   if (in_cell && y0 < y1) {
     R F[4];
-    ring_rows<R, RING>(ring, T, y0 - 1, rp);
-    edge_flux<R, NG, FLUX, RECON, 1>(rp, T, A.limiter, t, K, F);
+    ring_rows<RING>(ring, T, y0 - 1, rp);
+    edge_flux<NG, FLUX, RECON, 1>(rp, T, A.limiter, t, K, F);
 #pragma unroll
     for (int k = 0; k < 4; ++k) sfj[(((y0 - 1) & 1) * 4 + k) * T + t] = F[k];
   }
@@ -364,20 +636,11 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, const FluxConsts<
   RowSrc<R> pre;
   if (y0 < y1) load_src<R>(A, sx, y0 + NG, pre);
 
-  double dt_loc = INFINITY;
-  int st_loc = 0;
-
   for (int j = y0; j < y1; ++j) {
     // operands of this row's cell update, issued early
     const size_t cidx = (size_t)j * A.pitch + (size_t)min(max(gx, 0), A.ni - 1);
     double ua[4], uk[4];
-    if (in_cell) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        ua[k] = A.Ua[k] ? A.Ua[k][cidx] : 0.0;  // may alias Uo: plain load, read before write
-        uk[k] = (A.kind == 1) ? __ldg(A.Uk[k] + cidx) : 0.0;
-      }
-    }
+    if (in_cell) load_operands(A, cidx, ua, uk);
     RowSrc<R> nxt;
     if (j + 1 < y1) load_src<R>(A, sx, j + 1 + NG, nxt);
     {
@@ -389,228 +652,377 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, const FluxConsts<
     }
     pre = nxt;
     __syncthreads();
-    ring_rows<R, RING>(ring, T, j, rp);
+    ring_rows<RING>(ring, T, j, rp);
     if (in_i_edge) {
       R F[4];
-      edge_flux<R, NG, FLUX, RECON, 0>(rp, T, A.limiter, t, K, F);
+      edge_flux<NG, FLUX, RECON, 0>(rp, T, A.limiter, t, K, F);
 #pragma unroll
       for (int k = 0; k < 4; ++k) sfi[k * T + t] = F[k];
     }
     if (in_cell) {
       R F[4];
-      edge_flux<R, NG, FLUX, RECON, 1>(rp, T, A.limiter, t, K, F);
+      edge_flux<NG, FLUX, RECON, 1>(rp, T, A.limiter, t, K, F);
 #pragma unroll
       for (int k = 0; k < 4; ++k) sfj[((j & 1) * 4 + k) * T + t] = F[k];
     }
     __syncthreads();
     if (in_cell) {
-      double un[4];
-      // the cell's metrics (constants on a uniform grid)
-      const Geom cg = cell_geom(A.G, gx, j);
-      if constexpr (Prec<R>::kind == 2) {
-        if (A.G.rdyc) dy_inv = to_df(A.G.rdyc[j]);
-      }
-      if constexpr (Prec<R>::kind != 1) {
-        [[maybe_unused]] const Rcp<double> vol(cg.vol, cg.vol_y62);
+      R Fi[4], Fim[4], Fj[4], Fjm[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const R Fi = sfi[k * T + t], Fim = sfi[k * T + t - 1];
-          const R Fj = sfj[((j & 1) * 4 + k) * T + t];
-          const R Fjm = sfj[(((j - 1) & 1) * 4 + k) * T + t];
-          double r;
-          if constexpr (Prec<R>::kind == 0) {
-            double L = divergence_fp64(Fi, Fim, Fj, Fjm, cg, vol);
-            if (k == 3 && A.src_q) L = L + A.src_q[cidx];
-            if (A.kind == 2) {
-              r = L;
-            } else if (A.kind == 0) {
-              r = ua[k] + __dmul_rn(L, cc);
-              if (abs_lt(r, Num<double>::eps)) r = 0.0;
-            } else {
-              double s = __dmul_rn(ua[k], A.a) + __dmul_rn(uk[k], A.b);
-              if (abs_lt(s, Num<double>::eps)) s = 0.0;
-              r = s + __dmul_rn(L, cc);
-              if (abs_lt(r, Num<double>::eps)) r = 0.0;
-            }
-          } else {
-            // double-float divergence (pairs on the FP32 pipe) carried to FP64 once; the RK
-            // accumulation in FP64: U^n + c L, or a U^n + b U^k + c L as two FP64 FMAs with the
-            // increment c L formed in double-float: three FP64 operations per variable instead
-            // of six (stages 2 and 3 of SSP-RK3 on the 4096^2 quadrant: 6 % faster)
-            const df Ld = -((Fi - Fim) * dx_inv + (Fj - Fjm) * dy_inv);
-            const bool src = k == 3 && A.src_q;
-            if (A.kind == 2) {
-              r = from_df(Ld);
-              if (src) r = r + A.src_q[cidx];
-            } else if (A.kind == 0) {
-              double L = from_df(Ld);
-              if (src) L = L + A.src_q[cidx];
-              r = ua[k] + __dmul_rn(L, cc);
-              if (abs_lt(r, Num<double>::eps)) r = 0.0;
-            } else {
-              const double d = src ? __dmul_rn(from_df(Ld) + A.src_q[cidx], cc)
-                                   : from_df(Ld * cc_df);
-              r = fma(uk[k], A.b, fma(ua[k], A.a, d));
-              if (abs_lt(r, Num<double>::eps)) r = 0.0;
-            }
-          }
-          un[k] = r;
-          A.Uo[k][cidx] = r;
-        }
-      } else {
-        // FP32 divergence and stage increment c L; the stage combine (the RK accumulation)
-        // in FP64
-        const float idx_f = idx_col;
-        const float idy_f = (EXT && A.G.rdyf) ? A.G.rdyf[j] : idy_uni;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          float Fi = sfi[k * T + t], Fim = sfi[k * T + t - 1];
-          float Fj = sfj[((j & 1) * 4 + k) * T + t];
-          float Fjm = sfj[(((j - 1) & 1) * 4 + k) * T + t];
-          float Lf = -((Fi - Fim) * idx_f + (Fj - Fjm) * idy_f);
-          if (EXT && k == 3 && A.src_q) Lf = Lf + d2f_int(A.src_q[cidx]);
-          double r;
-          if (A.kind == 2) r = f2d_int(Lf);
-          else if (A.kind == 0) r = ua[k] + f2d_int(Lf * ccf);
-          else r = fma(uk[k], A.b, fma(ua[k], A.a, f2d_int(Lf * ccf)));
-          un[k] = r;
-          A.Uo[k][cidx] = r;
-        }
+      for (int k = 0; k < 4; ++k) {
+        Fi[k] = sfi[k * T + t];
+        Fim[k] = sfi[k * T + t - 1];
+        Fj[k] = sfj[((j & 1) * 4 + k) * T + t];
+        Fjm[k] = sfj[(((j - 1) & 1) * 4 + k) * T + t];
       }
-      if (A.last) {
-        // CFL dt of the new state (get_timestep, mod_fluid.f90:554-558) and the sanity checks
-        if constexpr (Prec<R>::kind == 0) {
-          double u, v, p, cs;
-          prim_from_cons(A.gamma, A.gamma - 1.0, un[0], un[1], un[2], un[3], u, v, p, cs);
-          double d = div_rn(A.cfl, div_rn(rabs(u) + cs, cg.dx) + div_rn(rabs(v) + cs, cg.dy));
-          if (d_less(d, dt_loc)) dt_loc = d;
-          if (d_isnan(un[0]) || d_isnan(u) || d_isnan(v) || d_isnan(p)) st_loc |= ST_NAN;
-          if (lt0(un[0])) st_loc |= ST_NEG_DENSITY;
-          if (lt0(p)) st_loc |= ST_NEG_PRESSURE;
-        } else if constexpr (Prec<R>::kind == 2) {
-          df u, v, p, cs;
-          const df rE = to_df(un[3]);
-          prim_from_cons(g, g1, to_df(un[0]), to_df(un[1]), to_df(un[2]), rE, u, v, p, cs, true);
-          if (near_vacuum(p.hi, rE.hi, 1e-4f)) {  // the FP64 recovery decides p and its sign
-            double u64, v64, p64;
-            prim_from_cons_f64(A.gamma, un[0], un[1], un[2], un[3], u64, v64, p64);
-            u = to_df(u64); v = to_df(v64); p = to_df(p64);
-            cs = df_sqrt(g * df_div(p, to_df(un[0])));
-          }
-          const df d = df_div(cfl_df, (df_abs(u) + cs) * dx_inv + (df_abs(v) + cs) * dy_inv);
-          const double dd = from_df(d);
-          if (dd > 0.0 && dd < dt_loc) dt_loc = dd;
-          if (isnan(un[0]) || isnan(u.hi) || isnan(v.hi) || isnan(p.hi)) st_loc |= ST_NAN;
-          if (un[0] < 0.0) st_loc |= ST_NEG_DENSITY;
-          if (p.hi < 0.0f) st_loc |= ST_NEG_PRESSURE;
-        } else {
-          const float4 uf = make_float4(d2f_fast(un[0]), d2f_fast(un[1]), d2f_fast(un[2]),
-                                        d2f_fast(un[3]));
-          float u, v, p, cs;
-          prim_from_cons(g, g1, uf.x, uf.y, uf.z, uf.w, u, v, p, cs);
-          float d = cfl_f / ((fabsf(u) + cs) * idx_col +
-                             (fabsf(v) + cs) * ((EXT && A.G.rdyf) ? A.G.rdyf[j] : idy_uni));
-          double dd = f2d_int(d);
-          if (__double_as_longlong(dd) < __double_as_longlong(dt_loc) && d > 0.0f) dt_loc = dd;
-          // NaN and sign tests on the FP64 state itself (the fast conversion keeps neither)
-          if (d_isnan(un[0]) || d_isnan(un[1]) || d_isnan(un[2]) || d_isnan(un[3]) ||
-              isnan(u) || isnan(v) || isnan(p))
-            st_loc |= ST_NAN;
-          if (lt0(un[0])) st_loc |= ST_NEG_DENSITY;
-          if (p < 0.0f) st_loc |= ST_NEG_PRESSURE;
-        }
-      }
+      update_cell<EXT>(A, C, gx, j, cidx, ua, uk, Fi, Fim, Fj, Fjm);
     }
   }
-
-  if (A.last) {
-    // block min of dt (bits of positive doubles order as unsigned integers) and status OR
-    unsigned long long bits =
-        (dt_loc > 0.0) ? (unsigned long long)__double_as_longlong(dt_loc) : ~0ULL;
-    for (int o = 16; o > 0; o >>= 1) {
-      unsigned long long ob = __shfl_xor_sync(0xffffffffu, bits, o);
-      bits = ob < bits ? ob : bits;
-      st_loc |= __shfl_xor_sync(0xffffffffu, st_loc, o);
-    }
-    if ((t & 31) == 0) {
-      if (bits != ~0ULL) atomicMin(A.dt_min, bits);
-      if (st_loc) atomicOr(A.status, st_loc);
-    }
-  }
+  reduce_column(A, C);
 }
 
-// Minimum resident 256-thread CTAs per SM requested from the register allocator for the
-// double-float kernels (their pair arithmetic is latency-bound; more warps hide it).
-#ifndef CATO_DF_MIN_BLOCKS
-#define CATO_DF_MIN_BLOCKS 2
-#endif
-// the same for the FP32 (mixed) kernels: the single-grid kernels run best unconstrained, the
-// persistent batch kernels at 4 CTAs per SM (64 registers; +4.5 % on the batched workload)
+// ---------------------------------------------------------------------------------------------
+// the TVD2 tile
+// ---------------------------------------------------------------------------------------------
+// Whether a flux reads cell pressures around the edge (shock sensors).
+constexpr bool flux_reads_pressure(int flux) {
+  return flux == FLUX_AUSMPW || flux == FLUX_SD_SLAU || flux == FLUX_SD_SLAU2 || flux == FLUX_ROE;
+}
+// M-AUSMPW+ reconstructs twice per edge (its second interpolator) and keeps the general tile.
+constexpr bool tvd_tile_of(int flux, int recon) { return recon == 0 && flux != FLUX_M_AUSMPW; }
+// rows of primitives it keeps
+constexpr int tvd_ring_rows(int flux) { return flux_reads_pressure(flux) ? 4 : 2; }
+
+// Edge values of N cells from their lower and upper differences: L the left state of the edge
+// above, Rr the right state of the edge below.  phi(b / a) a is symmetric in a and b for every
+// TVD2 limiter, so one limited slope serves both.  One limiter choice for all N cells, so that
+// their slopes stand in one block.
+template <int N>
+__device__ __forceinline__ void tvd_cells(int lim, const float q[N], const float a[N],
+                                          const float b[N], float L[N], float Rr[N]) {
+  auto all = [&](auto lc) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const float s = tvd_slope_f32(decltype(lc)::value, b[k], a[k]);
+      L[k] = q[k] + 0.5f * s;
+      Rr[k] = q[k] - 0.5f * s;
+    }
+  };
+  if (lim == LIM_MINMOD) all(std::integral_constant<int, LIM_MINMOD>{});
+  else if (lim == LIM_SUPERBEE) all(std::integral_constant<int, LIM_SUPERBEE>{});
+  else all(std::integral_constant<int, LIM_VANLEER>{});
+}
+
+// One tile of a TVD2 scheme (FP32).  A cell's two edge values along a direction come from the same
+// two differences and one limited slope, so they are made once per cell (the edge-wise form makes
+// every difference three times and every slope twice), and the march keeps what the next row needs
+// in registers: the lower difference and the upper left state of the column, the right-hand left
+// state of the row, the fluxes of the edge below.  Shared memory only carries what the
+// neighbouring columns read: the row of primitives (a ring of 4 rows where the flux reads
+// pressures around the edge, else 2), the right states and the x fluxes, each double-buffered by
+// row, so that one __syncthreads per row orders them all.
+//
+// Row j of the march: row j + 2 enters; the y values of cell j + 1 complete edge j + 1/2; the x
+// fluxes of row j use the values of the row before; the x values of row j + 1; barrier; update.
+template <int FLUX, bool EXT>
+__device__ __forceinline__ void stage_tile_tvd(const StageArgs& A, const FluxConsts<float>& K,
+                                               int bx, int by, unsigned char* smem_raw) {
+  constexpr int NG = 2, RR = tvd_ring_rows(FLUX);
+  const int T = blockDim.x, W = T - 2 * NG, t = threadIdx.x;
+  const int gx = bx * W - NG + t;
+  const int y0 = by * A.rows_per_cta;
+  const int y1 = min(y0 + A.rows_per_cta, A.nj);
+  float* const ring = reinterpret_cast<float*>(smem_raw);  // [RR][4][T] row r at slot r % RR
+  float* const srm = ring + RR * 4 * T;  // [2][4][T] right state of the cell's left edge
+  float* const sfi = srm + 8 * T;        // [2][4][T] flux of the edge right of the cell
+  auto row_at = [&](int r) { return ring + ((r + RR) & (RR - 1)) * 4 * T; };
+
+  const float g = float(A.gamma), g1 = float(A.gamma - 1.0);
+  bool flipx;
+  const int sx = map_index(min(gx, A.ni + NG - 1), A.ni, A.bc[SIDE_MX], A.bc[SIDE_PX], flipx);
+  const int xmode = column_mode<EXT>(A, gx);
+  const bool in_x = t >= 1 && t <= T - 2 && gx <= A.ni;  // columns whose x values are read
+  const bool in_cell = t >= NG && t <= NG + W - 1 && gx < A.ni;
+  ColumnConsts<float> C;
+  C.template init<EXT>(A, gx);
+
+  auto prims_of = [&](const RowSrc<float>& src, int row, float q[4]) {
+    src_to_prim<float>(A, src, flipx, xmode, row, g, g1, q);
+  };
+  auto store_row = [&](int r, const float q[4]) {
+    float* row = row_at(r);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) row[k * T + t] = q[k];
+  };
+  auto flux_y = [&](int j, const float L[4], const float Rr[4], float F[4]) {
+    auto P = [&](int di, int dj) -> float { return row_at(j + dj)[3 * T + t + di]; };
+    flux_of<float, FLUX, 1>(K, {L[0], L[1], L[2], L[3]}, {Rr[0], Rr[1], Rr[2], Rr[3]}, P, F);
+  };
+  auto flux_x = [&](int j, const float L[4], float F[4]) {
+    auto P = [&](int di, int dj) -> float { return row_at(j + dj)[3 * T + t + di]; };
+    const float* rm = srm + (j & 1) * 4 * T + t + 1;
+    flux_of<float, FLUX, 0>(K, {L[0], L[1], L[2], L[3]}, {rm[0], rm[T], rm[2 * T], rm[3 * T]}, P, F);
+  };
+
+  float q1[4], a[4], Lt[4], Lx[4], Fb[4];  // row j + 1, its lower difference; carried values
+  RowSrc<float> pre;
+  // rows y0-2 .. y0+1, the y values of cells y0-1 and y0, the flux of edge y0-1/2, the x values
+  // of row y0
+  {
+    float q[4][4], d[3][4], Rt[4], Rb[4], L1[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      load_src<float>(A, sx, y0 - 2 + r, pre);
+      prims_of(pre, y0 - 2 + r, q[r]);
+      if (r >= 4 - RR) store_row(y0 - 2 + r, q[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) d[r][k] = q[r + 1][k] - q[r][k];
+    if (in_cell) {
+      tvd_cells<4>(A.limiter, q[1], d[0], d[1], Lt, Rt);
+      tvd_cells<4>(A.limiter, q[2], d[1], d[2], L1, Rb);
+    }
+    __syncthreads();
+    if (in_cell) {
+      flux_y(y0 - 1, Lt, Rb, Fb);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) Lt[k] = L1[k];
+    }
+    if (in_x) {
+      const float* row = row_at(y0);
+      float lo[4], up[4], Rm[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        lo[k] = q[2][k] - row[k * T + t - 1];
+        up[k] = row[k * T + t + 1] - q[2][k];
+      }
+      tvd_cells<4>(A.limiter, q[2], lo, up, Lx, Rm);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) srm[((y0 & 1) * 4 + k) * T + t] = Rm[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      q1[k] = q[3][k];
+      a[k] = d[2][k];
+    }
+  }
+  if (y0 < y1) load_src<float>(A, sx, y0 + 2, pre);
+  __syncthreads();
+
+  for (int j = y0; j < y1; ++j) {
+    const size_t cidx = (size_t)j * A.pitch + (size_t)min(max(gx, 0), A.ni - 1);
+    double ua[4], uk[4];
+    if (in_cell) load_operands(A, cidx, ua, uk);
+    float q2[4], Ft[4];
+    {
+      RowSrc<float> nxt;
+      if (j + 1 < y1) load_src<float>(A, sx, j + 3, nxt);
+      prims_of(pre, j + 2, q2);
+      pre = nxt;
+    }
+    store_row(j + 2, q2);
+    // one block for both directions (columns without a cell compute values nobody reads), so that
+    // the two chains overlap
+    if (in_x) {
+      const float* row = row_at(j + 1);
+      float q[8], lo[8], up[8], Lv[8], Rv[8], F[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        q[k] = q[4 + k] = q1[k];
+        lo[k] = a[k];
+        up[k] = q2[k] - q1[k];
+        lo[4 + k] = q1[k] - row[k * T + t - 1];
+        up[4 + k] = row[k * T + t + 1] - q1[k];
+      }
+      tvd_cells<8>(A.limiter, q, lo, up, Lv, Rv);
+      flux_y(j, Lt, Rv, Ft);
+      flux_x(j, Lx, F);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        sfi[((j & 1) * 4 + k) * T + t] = F[k];
+        srm[(((j + 1) & 1) * 4 + k) * T + t] = Rv[4 + k];
+        a[k] = up[k];
+        Lt[k] = Lv[k];
+        Lx[k] = Lv[4 + k];
+        q1[k] = q2[k];
+      }
+    }
+    __syncthreads();
+    if (in_cell) {
+      float Fi[4], Fim[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        Fi[k] = sfi[((j & 1) * 4 + k) * T + t];
+        Fim[k] = sfi[((j & 1) * 4 + k) * T + t - 1];
+      }
+      update_cell<EXT>(A, C, gx, j, cidx, ua, uk, Fi, Fim, Ft, Fb);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) Fb[k] = Ft[k];
+    }
+  }
+  reduce_column(A, C);
+}
+
+// ---------------------------------------------------------------------------------------------
+// the edge-parallel tile
+// ---------------------------------------------------------------------------------------------
+// One row of edges per warp (or per warp pair), both directions side by side: blockDim =
+// (T, 2 RW + 1), T = 32 or 64 columns incl. the x-halo.  The tile marches in blocks of RW rows.
+// Per block RW new rows of primitives enter a ring of RW + 2 NG rows, then threadIdx.y = 1 .. RW
+// makes the y edges above the block's rows (0 the one below the first block) and the others its x
+// edges, then all of them share the (cell, variable) updates; a barrier lies between the phases.
+// The serial chain of a block is one edge, against a row's two edges and update in the marching
+// strip, and a CTA has 2 RW + 1 times the warps for the same columns, so that small grids finish
+// early and the latency of the long FP64 chains is covered with few registers per thread.
+struct EdgeShape {
+  int columns;  // T
+  int block;    // RW
+};
+template <typename R, int NG, int FLUX, int RECON>
+__device__ __forceinline__ void edge_tile(const StageArgs& A, const FluxConsts<R>& K, int bx,
+                                          int by, unsigned char* smem_raw) {
+  const int T = blockDim.x, nw = blockDim.y, RW = nw >> 1, NR = RW + 2 * NG;
+  const int t = threadIdx.x, w = threadIdx.y;
+  const int gx = bx * (T - 2 * NG) - NG + t;
+  const int y0 = by * A.rows_per_cta, y1 = min(y0 + A.rows_per_cta, A.nj);
+  double* const un = reinterpret_cast<double*>(smem_raw);  // [RW][4][T] new states
+  R* const prim = reinterpret_cast<R*>(un + RW * 4 * T);   // [NR][4][T] row r at slot (r - y0 + NG) % NR
+  R* const sfx = prim + NR * 4 * T;                        // [RW][4][T] edge right of the cell
+  R* const sfy = sfx + RW * 4 * T;                         // [RW + 1][4][T] edge above row e at
+                                                           // slot (e - y0 + 1) % (RW + 1)
+  const R g = R(A.gamma), g1 = R(A.gamma - 1.0);
+  bool flipx;
+  const int sx = map_index(min(gx, A.ni + NG - 1), A.ni, A.bc[SIDE_MX], A.bc[SIDE_PX], flipx);
+  const int xmode = column_mode<true>(A, gx);
+  const bool in_i_edge = t >= NG - 1 && t < T - NG && gx <= A.ni - 1;
+  const bool in_cell = t >= NG && t < T - NG && gx < A.ni;
+  ColumnConsts<R> C;
+  C.template init<true>(A, gx);
+
+  int next = -NG;  // first row (relative to y0) not yet in the ring
+  for (int yb = y0; yb < y1; yb += RW) {
+    const int rows = min(RW, y1 - yb);
+    const int upto = yb - y0 + rows + NG;  // rows below this one are needed
+    for (int r = next + w; r < upto; r += nw) {
+      RowSrc<R> s;
+      load_src<R>(A, sx, y0 + r, s);
+      R q[4];
+      src_to_prim<R>(A, s, flipx, xmode, y0 + r, g, g1, q);
+      R* row = prim + (r + NG) % NR * 4 * T;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) row[k * T + t] = q[k];
+    }
+    next = upto;
+    __syncthreads();
+    const bool along_y = w <= RW;
+    const int e = along_y ? yb - 1 + w : yb + w - RW - 1;  // the edges' (lower) row
+    if (e < y1 && (w > 0 || yb == y0)) {
+      const bool act = along_y ? in_cell : in_i_edge;
+      if (act) {
+        // rows e - 2 .. e + 3; NG = 2 reads e - 1 .. e + 2
+        int ro[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) ro[k] = (e - y0 + NG + k - 2 + NR) % NR * 4 * T + t;
+        R F[4];
+        edge_flux_any<R, FLUX, RECON>(prim, ro, T, A.limiter, along_y, K, F);
+        R* out = along_y ? sfy + (e - y0 + 1) % (RW + 1) * 4 * T : sfx + (e - yb) * 4 * T;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) out[k * T + t] = F[k];
+      }
+    }
+    __syncthreads();
+    for (int n = w; n < rows * 4; n += nw) {
+      if (!in_cell) continue;
+      const int r = n >> 2, k = n & 3, j = yb + r;
+      const size_t cidx = (size_t)j * A.pitch + gx;
+      const Geom cg = cell_geom(A.G, gx, j);
+      if constexpr (Prec<R>::kind == 2) C.set_row(A, j);
+      const double ua = A.Ua[k] ? A.Ua[k][cidx] : 0.0;
+      const double uk = A.kind == 1 ? __ldg(A.Uk[k] + cidx) : 0.0;
+      const R* fj = sfy + ((j - y0 + 1) % (RW + 1) * 4 + k) * T + t;
+      const R* fjm = sfy + ((j - y0) % (RW + 1) * 4 + k) * T + t;
+      const double u = combine_var<R>(A, C, cg, Rcp<double>(cg.vol, cg.vol_y62), k, cidx, ua, uk,
+                                      sfx[n * T + t], sfx[n * T + t - 1], *fj, *fjm);
+      A.Uo[k][cidx] = u;
+      if (A.last) un[n * T + t] = u;
+    }
+    if (!A.last) continue;
+    __syncthreads();
+    if (w < rows && in_cell) {
+      const int j = yb + w;
+      const double* v = un + w * 4 * T + t;
+      const double u4[4] = {v[0], v[T], v[2 * T], v[3 * T]};
+      if constexpr (Prec<R>::kind == 2) C.set_row(A, j);
+      check_state<R, true>(A, C, cell_geom(A.G, gx, j), j, u4);
+    }
+  }
+  if (w < RW) reduce_column(A, C);
+}
+template <typename R> constexpr size_t edge_smem_bytes(EdgeShape s, int ng) {
+  return (size_t)s.columns * 4 *
+         (sizeof(double) * s.block + sizeof(R) * (size_t)(3 * s.block + 2 * ng + 1));
+}
+constexpr int kEdgeThreads = 128 * 7;  // most threads of a CTA: 128 columns, blocks of 3 rows
+
+// ---------------------------------------------------------------------------------------------
+// kernels
+// ---------------------------------------------------------------------------------------------
+// FP32: the marching strips.  The tile of a scheme, and its dynamic shared memory.
+template <int NG, int FLUX, int RECON, bool EXT, bool TVD = tvd_tile_of(FLUX, RECON)>
+__device__ __forceinline__ void tile_of(const StageArgs& A, const FluxConsts<float>& K, int bx,
+                                        int by, unsigned char* smem_raw) {
+  if constexpr (TVD) stage_tile_tvd<FLUX, EXT>(A, K, bx, by, smem_raw);
+  else stage_tile<NG, FLUX, RECON, EXT>(A, K, bx, by, smem_raw);
+}
+constexpr size_t tile_smem_bytes(int T, int ng, int flux, bool tvd) {
+  const int per_column = tvd ? tvd_ring_rows(flux) * 4 + 16 : 2 * ng * 4 + 4 + 8;
+  return sizeof(float) * (size_t)T * per_column;
+}
+// In the persistent batch kernels AUSMPW+ keeps the general tile: there the contraction the
+// assembler picks for its TVD2 tile rounds the products the other way (5e-10 of the density in 6
+// steps), and a request's result would change.
+constexpr bool batch_tvd_tile_of(int flux, int recon) {
+  return tvd_tile_of(flux, recon) && flux != FLUX_AUSMPW;
+}
+
+// Minimum resident 256-thread CTAs per SM requested from the register allocator: the single-grid
+// kernels run best unconstrained, the persistent batch kernels of the general tile at 4 (64
+// registers; +4.5 % on the batched workload), those of the TVD2 tile, whose carried rows need
+// more, at 2
 #ifndef CATO_F32_MIN_BLOCKS
 #define CATO_F32_MIN_BLOCKS 1
 #endif
 #ifndef CATO_F32_BATCH_MIN_BLOCKS
 #define CATO_F32_BATCH_MIN_BLOCKS 4
 #endif
-// and for the FP64 kernels, which come in three register budgets (kernel variants 0, 1, 2): the
-// compiler's choice, at most 128 registers (two 256-thread CTAs per SM) and at most 85 (three).
-// Which is faster depends on the flux, the reconstruction, the plan and the flow
-// (cato_gpu_tune measures it; the 4096^2 quadrant and Kelvin-Helmholtz grids run best with 85
-// registers in 256-thread strips of 16 rows: +3 % and +4 % over the best 128-register plan);
-// all give bit-identical results.
-#ifndef CATO_F64_MIN_BLOCKS
-#define CATO_F64_MIN_BLOCKS 1
+#ifndef CATO_F32_BATCH_TVD_MIN_BLOCKS
+#define CATO_F32_BATCH_TVD_MIN_BLOCKS 2
 #endif
-#ifndef CATO_F64_MIN_BLOCKS_ALT
-#define CATO_F64_MIN_BLOCKS_ALT 2
-#endif
-#ifndef CATO_F64_MIN_BLOCKS_ALT2
-#define CATO_F64_MIN_BLOCKS_ALT2 3
-#endif
-template <typename R> constexpr int min_blocks() {
-  return Prec<R>::kind == 2 ? CATO_DF_MIN_BLOCKS
-                            : (Prec<R>::kind == 1 ? CATO_F32_MIN_BLOCKS : CATO_F64_MIN_BLOCKS);
-}
-// the persistent batch kernels (256-thread CTAs) run best with more resident warps than the
-// single-grid kernels: FP64 and double-float at most 85 registers (3 CTAs per SM), measured on
-// the batched random-circle workload (SLAU + MLP5) at +28 % (FP64, over the compiler's 229
-// registers) and +21 % (double-float, over 122); both spill a little to the stack.  FP64 at 128
-// registers gave +20 %, double-float at 64 less than at 85.
-#ifndef CATO_F64_BATCH_MIN_BLOCKS
-#define CATO_F64_BATCH_MIN_BLOCKS 3
-#endif
-#ifndef CATO_DF_BATCH_MIN_BLOCKS
-#define CATO_DF_BATCH_MIN_BLOCKS 3
-#endif
-// FP64 M-AUSMPW+ (two interpolators' edge states live at once) spills too much at 85: at most
-// 128 registers (205 against 168 M cell-updates/s); Roe and the other fluxes measured best at 85
-#ifndef CATO_F64_BATCH_MIN_BLOCKS_MAUSMPW
-#define CATO_F64_BATCH_MIN_BLOCKS_MAUSMPW 2
-#endif
-template <typename R, int FLUX> constexpr int batch_min_blocks() {
-  return Prec<R>::kind == 2
-             ? CATO_DF_BATCH_MIN_BLOCKS
-             : (Prec<R>::kind == 1 ? CATO_F32_BATCH_MIN_BLOCKS
-                                   : (FLUX == FLUX_M_AUSMPW ? CATO_F64_BATCH_MIN_BLOCKS_MAUSMPW
-                                                            : CATO_F64_BATCH_MIN_BLOCKS));
-}
 
-template <typename R, int NG, int FLUX, int RECON, bool EXT, int MB>
-__global__ void __launch_bounds__(256, MB)
-    stage_kernel(const StageArgs A, const FluxConsts<R> K) {
+template <int NG, int FLUX, int RECON, bool EXT>
+__global__ void __launch_bounds__(256, CATO_F32_MIN_BLOCKS)
+    stage_kernel(const StageArgs A, const FluxConsts<float> K) {
   if (A.active && *A.active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  stage_tile<R, NG, FLUX, RECON, EXT>(A, K, blockIdx.x, blockIdx.y, smem_raw);
+  tile_of<NG, FLUX, RECON, EXT>(A, K, blockIdx.x, blockIdx.y, smem_raw);
+}
+
+// FP64 and double-float: the edge-parallel tile, with a register budget per kernel variant.
+// 56 registers (36 warps per SM) run best or within 3 % of it nearly everywhere measured; the
+// FP64 path offers two more to the tuner.
+constexpr int edge_regs(int variant) { return variant == 0 ? 56 : (variant == 1 ? 72 : 96); }
+template <typename R, int NG, int FLUX, int RECON, int REGS>
+__global__ void __maxnreg__(REGS) edge_kernel(const StageArgs A, const FluxConsts<R> K) {
+  if (A.active && *A.active == 0) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  edge_tile<R, NG, FLUX, RECON>(A, K, blockIdx.x, blockIdx.y, smem_raw);
 }
 
 // whether a stage needs the EXT kernel (rectilinear grid, energy source, pressure input)
 inline bool stage_needs_ext(const StageArgs& A) {
   return A.G.dxc != nullptr || A.src_q != nullptr || A.bc[SIDE_PX] == BC_PRESSURE_INPUT;
-}
-
-// dynamic shared memory of one CTA
-template <typename R> inline size_t stage_smem_bytes(int T, int ng) {
-  return sizeof(R) * (size_t)T * (2 * ng * 4 + 4 + 8);
 }
 
 }  // namespace cato

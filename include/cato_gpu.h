@@ -288,19 +288,21 @@ int cato_gpu_run_timed(cato_handle* h, int64_t n_steps, float* total_ms, float* 
                        int32_t capacity);
 
 /* Work decomposition of the stage kernel (the autotuner's knobs): CTA width `threads` (a
- * multiple of 32 in [64, 256], including 2*n_ghost halo columns) and rows marched per CTA. */
+ * multiple of 32 in [64, 256], including 2*n_ghost halo columns; the FP64 and double-float
+ * kernels, which put several warps on a column, take half of it in columns) and rows marched per
+ * CTA. */
 int cato_gpu_set_plan(cato_handle* h, int32_t threads, int32_t rows_per_cta);
 int cato_gpu_get_plan(const cato_handle* h, int32_t* threads, int32_t* rows_per_cta);
 
-/* Register budget of the FP64 stage kernel (the third knob): 0 = the compiler's choice (fewer
- * resident warps, more registers each), 1 = at most 128 registers per thread, 2 = at most 85.
- * Which is faster depends on the flux, the reconstruction, the plan and the flow; the results
- * are bit-identical.  Accepted and ignored by the mixed precisions. */
+/* Register budget of the FP64 stage kernel (the third knob): 0 = at most 56 registers per thread,
+ * 1 = at most 72, 2 = at most 96 (fewer resident warps, fewer spills).  Which is fastest depends
+ * on the flux, the reconstruction, the plan and the flow; the results are bit-identical.
+ * Accepted and ignored by the mixed precisions. */
 int cato_gpu_set_kernel_variant(cato_handle* h, int32_t variant);
 int cato_gpu_get_kernel_variant(const cato_handle* h, int32_t* variant);
 
-/* Autotune the stage kernel on the live state: a few candidate plans (the current strip width
- * and 256-wide strips, each with the current, half and a quarter of the rows per CTA), each
+/* Autotune the stage kernel on the live state: a few candidate plans (the current width and the
+ * widest, each with the current, half and a quarter of the rows per CTA), each
  * with every FP64 register budget, run `steps` CFL steps each (timed with CUDA events), and the
  * fastest stays set.  These are real steps of the run
  * (the solution advances by *steps_taken steps, bit-identical whichever candidate runs them);
