@@ -181,8 +181,11 @@ static int rebuild(cato_batch* b) {
     BK(cudaGetDevice(&dev));
     BK(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev));
   }
-  // Rows per tile: the plan's, halved (down to 4) while the batch would give fewer than two
-  // tiles per SM, so that a batch of small grids still fills the GPU.
+  // Rows per tile, at most the plan's.  FP32 strips hide their latency with neighbours: the most
+  // rows that leave five tiles per SM (served stream, 1.1 M cells: 1.93 ms per 16 steps at 8 rows,
+  // 3.06 at 32).  The edge-parallel tiles fill an SM with two: what counts is the share of the
+  // busiest SM, its tiles times the rows they hold and the edges they repeat (FP64 sweep of
+  // 0.29 M cells: 19.9 ms at 4 rows with 9 tiles on an SM, 24.4 at 16 rows with 3).
   auto n_tiles = [&](int r) {
     long long n = 0;
     for (int i : order) {
@@ -193,7 +196,14 @@ static int rebuild(cato_batch* b) {
     return n;
   };
   int tile_rows = b->rows;
-  while (tile_rows > 4 && n_tiles(tile_rows) < 2LL * b->sms) tile_rows = std::max(4, tile_rows / 2);
+  if (b->prec == CATO_MIXED) {
+    while (tile_rows > 4 && n_tiles(tile_rows) < 5LL * b->sms)
+      tile_rows = std::max(4, tile_rows / 2);
+  } else {
+    auto share = [&](int r) { return (double)((n_tiles(r) + b->sms - 1) / b->sms) * (r + 1.2); };
+    for (int r = tile_rows / 2; r >= 4; r /= 2)
+      if (share(r) < share(tile_rows)) tile_rows = r;
+  }
   b->tile_rows = tile_rows;
   for (int i : order) {
     const InstDesc& d = b->h_descs[i];
