@@ -14,6 +14,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/cato_gpu.h"
@@ -417,20 +418,52 @@ static int d2h_interior(cato_handle* h, double* dst, const double* src, int64_t 
   return CATO_OK;
 }
 
-// zero the ghost ring of a halo-padded host field (the interior is overwritten by the copy that
-// follows): the first and last ng columns in full, ng cells at both ends of every other column
-static void zero_host_field(cato_handle* h, double* a, int64_t ld) {
+// zero the ghost ring of columns [c0, c1) of a halo-padded host field (the interior is overwritten
+// by the copy that follows): the first and last ng columns in full, ng cells at both ends of every
+// other column.  touch: also write one value per page of the interior.
+static void zero_host_columns(const cato_handle* h, double* a, int64_t ld, size_t c0, size_t c1,
+                              bool touch) {
   const size_t ng = (size_t)h->ng, ni = (size_t)h->ni, nj = (size_t)h->nj;
   const size_t len = ni + 2 * ng;
-  for (size_t j = 0; j < nj + 2 * ng; ++j) {
+  for (size_t j = c0; j < c1; ++j) {
     double* col = a + j * ld;
     if (j < ng || j >= nj + ng) {
       std::memset(col, 0, sizeof(double) * len);
     } else {
       std::memset(col, 0, sizeof(double) * ng);
       std::memset(col + ng + ni, 0, sizeof(double) * ng);
+      if (touch)
+        for (size_t i = ng; i < ng + ni; i += 4096 / sizeof(double)) col[i] = 0.0;
     }
   }
+}
+static void zero_host_field(const cato_handle* h, double* a, int64_t ld) {
+  zero_host_columns(h, a, ld, 0, (size_t)h->nj + 2 * h->ng, false);
+}
+
+// The ghost rings of the fields of a download.  A caller's fresh arrays have no pages yet, and the
+// copy's page faults come one after the other (4096^2, four fields of 134 MB: 20.7 ms, against
+// 3.0 ms into touched memory): large fields are touched by several threads first (together 8.4 ms).
+static void zero_host_fields(const cato_handle* h, double* const* fields, int n, int64_t ld) {
+  const size_t cols = (size_t)h->nj + 2 * h->ng;
+  const size_t bytes = cols * (size_t)ld * sizeof(double) * (size_t)n;
+  const unsigned hw = std::thread::hardware_concurrency();
+  const size_t threads = bytes < (size_t(16) << 20) ? 1 : std::min<size_t>(16, hw ? hw : 1);
+  auto part = [&](size_t k) {
+    for (int f = 0; f < n; ++f)
+      zero_host_columns(h, fields[f], ld, cols * k / threads, cols * (k + 1) / threads,
+                        threads > 1);
+  };
+  std::vector<std::thread> pool;
+  size_t started = 1;
+  try {
+    pool.reserve(threads);
+    for (; started < threads; ++started) pool.emplace_back(part, started);
+  } catch (...) {  // no more threads to be had: the rest is done here
+  }
+  part(0);
+  for (size_t k = started; k < threads; ++k) part(k);
+  for (auto& t : pool) t.join();
 }
 
 
@@ -998,11 +1031,15 @@ int cato_gpu_download(cato_handle* h, double* rho, double* rho_u, double* rho_v,
   double* cons_out[4] = {rho, rho_u, rho_v, rho_E};
   double* der_out[4] = {u, v, p, cs};
   int rc;
+  double* outs[8];
+  int n_out = 0;
   for (int k = 0; k < 4; ++k)
-    if (cons_out[k]) {
-      zero_host_field(h, cons_out[k], ld);
-      if ((rc = d2h_interior(h, cons_out[k], Un[k], ld))) return rc;
-    }
+    if (cons_out[k]) outs[n_out++] = cons_out[k];
+  for (int k = 0; k < 4; ++k)
+    if (der_out[k]) outs[n_out++] = der_out[k];
+  zero_host_fields(h, outs, n_out, ld);
+  for (int k = 0; k < 4; ++k)
+    if (cons_out[k] && (rc = d2h_interior(h, cons_out[k], Un[k], ld))) return rc;
   if (u || v || p || cs) {
     if ((rc = ensure_scratch(h))) return rc;
     const int raw = h->raw_pending ? 1 : 0;
@@ -1012,10 +1049,7 @@ int cato_gpu_download(cato_handle* h, double* rho, double* rho_u, double* rho_v,
         h->scratch[1], h->scratch[2], h->scratch[3]);
     CK(cudaGetLastError());
     for (int k = 0; k < 4; ++k)
-      if (der_out[k]) {
-        zero_host_field(h, der_out[k], ld);
-        if ((rc = d2h_interior(h, der_out[k], h->scratch[k], ld))) return rc;
-      }
+      if (der_out[k] && (rc = d2h_interior(h, der_out[k], h->scratch[k], ld))) return rc;
   }
   CK(cudaStreamSynchronize(h->stream));
   return CATO_OK;
