@@ -96,6 +96,7 @@ __device__ __forceinline__ void batch_loop(const BatchStageArgs& B, Tile tile) {
     StageArgs A;
     batch_stage_args<R>(d, B, A);
     A.rows_per_cta = w.w;
+    A.block = 4;  // batch_shape
     tile(A, d, w.y, w.z);
   }
 }
@@ -117,8 +118,8 @@ template <typename R, int NG, int FLUX, int RECON>
 __global__ void __maxnreg__(edge_regs(0)) batch_edge_kernel(const BatchStageArgs B) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   batch_loop<R>(B, [&](const StageArgs& A, const InstDesc* d, int bx, int by) {
-    if constexpr (Prec<R>::kind == 0) edge_tile<R, NG, FLUX, RECON>(A, d->K64, bx, by, smem_raw);
-    else edge_tile<R, NG, FLUX, RECON>(A, d->Kdf, bx, by, smem_raw);
+    if constexpr (Prec<R>::kind == 0) edge_tile<R, NG, FLUX, RECON, false>(A, d->K64, bx, by, smem_raw);
+    else edge_tile<R, NG, FLUX, RECON, false>(A, d->Kdf, bx, by, smem_raw);
   });
 }
 

@@ -1235,7 +1235,8 @@ static StageShape plan_of(const cato_handle* h, int threads, int rows, int varia
   s.width = s.threads = threads;
   if (h->cfg.precision != CATO_MIXED) {
     s.threads = threads / 64 * 32;
-    s.block = std::min(rows, s.threads > 64 ? 3 : 4);
+    s.block = std::min(rows, s.threads > 64 ? 2 : 4);
+    s.warps = 2 * s.block + 1;
   }
   return s;
 }

@@ -32,6 +32,7 @@ struct StageShape {
   int threads = 128;
   int rows = 64;
   int block = 4;
+  int warps = 9;    // blockDim.y of the edge-parallel kernels, at least 2 block + 1
   int variant = 0;
 };
 
@@ -50,12 +51,13 @@ inline cudaError_t allow_smem(PerDevice& attr, int dev, F* kernel, size_t bytes)
 }
 // the largest shared memory an edge-parallel kernel may be launched with
 template <typename R> inline size_t edge_smem_limit(int ng) {
-  const size_t a = edge_smem_bytes<R>({64, 4}, ng), b = edge_smem_bytes<R>({128, 3}, ng);
-  return a > b ? a : b;
+  return std::max({edge_smem_bytes<R>({64, 4, 9}, ng), edge_smem_bytes<R>({128, 2, 5}, ng),
+                   edge_smem_bytes<R>({32, 2, 10}, ng)});
 }
 inline bool edge_shape_ok(EdgeShape s) {
   return s.columns >= 32 && s.columns <= 128 && s.columns % 32 == 0 && s.block >= 1 &&
-         s.block <= 4 && s.columns * (2 * s.block + 1) <= kEdgeThreads;
+         s.block * s.columns <= 256 && s.warps >= 2 * s.block + 1 &&
+         s.columns * s.warps <= kEdgeThreads;
 }
 
 template <int NG, int FLUX, int RECON, bool EXT>
@@ -75,24 +77,27 @@ cudaError_t launch_strip(const StageShape& s, bool warm, cudaStream_t stream, co
   return cudaGetLastError();
 }
 
-template <typename R, int NG, int FLUX, int RECON, int REGS>
+template <typename R, int NG, int FLUX, int RECON, int REGS, bool SPLIT = false>
 cudaError_t launch_edge(const StageShape& s, bool warm, cudaStream_t stream, const StageArgs& A,
                         const FluxConsts<R>& K) {
   static PerDevice attr;
   const int dev = launch_device();
   if (dev < 0) return cudaErrorInvalidDevice;
-  cudaError_t e = allow_smem(attr, dev, edge_kernel<R, NG, FLUX, RECON, REGS>,
+  cudaError_t e = allow_smem(attr, dev, edge_kernel<R, NG, FLUX, RECON, REGS, SPLIT>,
                              edge_smem_limit<R>(NG));
   if (e != cudaSuccess || warm) return e;
-  EdgeShape es{s.threads, s.block};
+  EdgeShape es{s.threads, s.block, s.warps};
   // the CTA's warps fit the register file: a quarter of them in each of its four 16 Ki parts
-  const int warps = 4 * (16384 / (32 * REGS));
-  es.block = std::min(es.block, (warps * 32 / es.columns - 1) / 2);
-  if (!edge_shape_ok(es)) return cudaErrorInvalidValue;
+  es.warps = std::min(es.warps, 4 * (16384 / (32 * REGS)) * 32 / es.columns);
+  es.block = std::min(es.block, (es.warps - 1) / 2);
+  if (!SPLIT) es.warps = 2 * es.block + 1;
+  if (!edge_shape_ok(es) || es.split() != SPLIT) return cudaErrorInvalidValue;
   const int W = es.columns - 2 * NG;
   const dim3 grid((A.ni + W - 1) / W, (A.nj + s.rows - 1) / s.rows);
-  edge_kernel<R, NG, FLUX, RECON, REGS>
-      <<<grid, dim3(es.columns, 2 * es.block + 1), edge_smem_bytes<R>(es, NG), stream>>>(A, K);
+  StageArgs B = A;
+  B.block = es.block;
+  edge_kernel<R, NG, FLUX, RECON, REGS, SPLIT>
+      <<<grid, dim3(es.columns, es.warps), edge_smem_bytes<R>(es, NG), stream>>>(B, K);
   return cudaGetLastError();
 }
 
@@ -112,6 +117,13 @@ cudaError_t launch_stage_one(const StageShape& s, bool warm, cudaStream_t stream
     }
     return launch_strip<NG, FLUX, RECON, true>(s, warm, stream, A, K);
   } else {
+    const bool split = EdgeShape{s.threads, s.block, s.warps}.split();
+    if (warm) {
+      cudaError_t e = launch_edge<R, NG, FLUX, RECON, edge_regs(0), true>(s, true, stream, A, K);
+      if (e != cudaSuccess) return e;
+    } else if (split && s.variant == 0) {
+      return launch_edge<R, NG, FLUX, RECON, edge_regs(0), true>(s, false, stream, A, K);
+    }
     if constexpr (Prec<R>::kind == 0) {
       if (warm) {
         cudaError_t e = launch_edge<R, NG, FLUX, RECON, edge_regs(1)>(s, true, stream, A, K);
@@ -144,8 +156,8 @@ inline cudaError_t launch_stage_flux(int recon, const StageShape& s, bool warm,
 // The shape of a batch launch for a plan's CTA width: FP32 strips are as wide as the plan says;
 // the edge-parallel tiles half as wide (32 to 64 columns), in blocks of 4 rows.
 template <typename R> inline EdgeShape batch_shape(int threads) {
-  if (Prec<R>::kind == 1) return {threads, 0};
-  return {threads < 128 ? 32 : 64, 4};
+  if (Prec<R>::kind == 1) return {threads, 0, 0};
+  return {threads < 128 ? 32 : 64, 4, 9};
 }
 
 // Persistent batch launch: as many CTAs as can be resident, each looping over work items.
@@ -167,7 +179,7 @@ cudaError_t launch_batch_one(int threads, cudaStream_t stream, const BatchStageA
     kernel = batch_edge_kernel<R, NG, FLUX, RECON>;
     smem = edge_smem_bytes<R>(shape, NG);
     most = edge_smem_limit<R>(NG);
-    block = dim3(shape.columns, 2 * shape.block + 1);
+    block = dim3(shape.columns, shape.warps);
   }
   cudaError_t e = allow_smem(attr, dev, kernel, most);
   if (e != cudaSuccess) return e;

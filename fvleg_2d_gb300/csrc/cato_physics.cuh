@@ -1601,14 +1601,15 @@ __device__ __forceinline__ void flux_hllc(const FluxConsts<R>& K, const Prim<R>&
   auto energy = [&](const Prim<R>& S) {
     return div_by(S.p, gm1_of(K)) + m(half(S.r), m(S.u, S.u) + m(S.v, S.v));
   };
-  R S_star = Num<R>::div(B.p - A.p + m(m(A.r, qnL), SL - qnL) - m(m(B.r, qnR), SR - qnR),
-                         m(A.r, SL - qnL) - m(B.r, SR - qnR));
+  const R rqL = m(A.r, qnL), rqR = m(B.r, qnR);
+  const R rkL = m(A.r, SL - qnL), rkR = m(B.r, SR - qnR);
+  R S_star = Num<R>::div(B.p - A.p + m(rqL, SL - qnL) - m(rqR, SR - qnR), rkL - rkR);
   R Fn[4];
   if (ge0(SL) || !(gt0(SR) || ge0(S_star))) {
     const bool useL = ge0(SL);
     const Prim<R>& S = useL ? A : B;
     R qn = useL ? qnL : qnR, qt = useL ? qtL : qtR, E = energy(S);
-    const R rq = m(S.r, qn);
+    const R rq = kFP32<R> ? m(S.r, qn) : (useL ? rqL : rqR);
     Fn[0] = rq;
     Fn[1] = m(rq, qn) + S.p;
     Fn[2] = m(rq, qt);
@@ -1617,11 +1618,12 @@ __device__ __forceinline__ void flux_hllc(const FluxConsts<R>& K, const Prim<R>&
     const bool useL = ge0(S_star);
     const Prim<R>& S = useL ? A : B;
     R qn = useL ? qnL : qnR, qt = useL ? qtL : qtR, E = energy(S), SK = useL ? SL : SR;
-    const R rk = m(S.r, SK - qn);
+    // FP64: the products of S_star's operands again
+    const R rk = kFP32<R> ? m(S.r, SK - qn) : (useL ? rkL : rkR);
     R f = Num<R>::div(rk, SK - S_star);
     R Us0 = f, Us1 = m(f, S_star), Us2 = m(f, qt);
     R Us3 = m(f, Num<R>::div(E, S.r) + m(S_star - qn, S_star + Num<R>::div(S.p, rk)));
-    const R rq = m(S.r, qn);
+    const R rq = kFP32<R> ? m(S.r, qn) : (useL ? rqL : rqR);
     Fn[0] = rq + m(SK, Us0 - S.r);
     Fn[1] = (m(rq, qn) + S.p) + m(SK, Us1 - rq);
     Fn[2] = m(rq, qt) + m(SK, Us2 - m(S.r, qt));
@@ -1641,7 +1643,7 @@ constexpr int kNotPow2 = 1 << 20;
 struct Geom {
   double vol, l1, l2, l3, l4;  // volume, edge lengths (bottom, right, top, left)
   double dx, dy;               // min_dx / min_dy for the CFL step
-  uint64_t vol_y62;            // recip62 of vol (uniform grid)
+  uint64_t vol_y62, dx_y62, dy_y62;  // recip62 of vol, dx, dy
   double inv_vol;              // 1/vol when vol is a power of two (x/vol == x*inv_vol exactly), else 0
   // base-2 exponents of l1..l4 and inv_vol when they are powers of two, else kNotPow2: the
   // products with them are exponent steps
@@ -1675,6 +1677,8 @@ __device__ __forceinline__ Geom cell_geom(const Geom& G, int i, int j) {
   c.dx = dx;
   c.dy = dy;
   c.vol_y62 = intdiv::recip62(intdiv::bits_of(c.vol));
+  c.dx_y62 = intdiv::recip62(intdiv::bits_of(dx));
+  c.dy_y62 = intdiv::recip62(intdiv::bits_of(dy));
   c.inv_vol = 0.0;
   c.k1 = c.k2 = c.k3 = c.k4 = c.kinv = kNotPow2;
   return c;
@@ -1696,6 +1700,8 @@ inline Geom uniform_geom(double dx, double dy) {
   // a division by a power of two is the multiplication by its reciprocal, which is exactly
   // representable: both round the same real number (power-of-two grids, e.g. 4096^2 on [0,1]^2)
   G.vol_y62 = intdiv::recip62(intdiv::bits_of(G.vol));
+  G.dx_y62 = intdiv::recip62(intdiv::bits_of(G.dx));
+  G.dy_y62 = intdiv::recip62(intdiv::bits_of(G.dy));
   int e = 0;
   const double m = std::frexp(G.vol, &e);
   G.inv_vol = (m == 0.5 && e > -1020 && e < 1020) ? 1.0 / G.vol : 0.0;
@@ -1741,8 +1747,12 @@ __device__ __forceinline__ double scaled_difference(double F, double Fm, double 
     return a;
   }
   const double s = intdiv::double_of(m);
-  const Rcp<double> rs(s);
-  a = (mul_pow2(div_by(F, rs), l, k) - mul_pow2(div_by(Fm, rs), lm, km)) * s;
+  if (m >= kInfBits) return (F / s * l - Fm / s * lm) * s;  // infinite or NaN: NaN
+  // the larger flux over the scale, itself, is +-1: one division is left
+  const bool first = mag_bits(F) == m;
+  const double q = Num<double>::div(first ? Fm : F, s);
+  const double one = intdiv::double_of((intdiv::bits_of(first ? F : Fm) & kSignBit) | ONE);
+  a = (mul_pow2(first ? one : q, l, k) - mul_pow2(first ? q : one, lm, km)) * s;
   if (mag_bits(a) < intdiv::bits_of(s * REL_TOL)) a = 0.0;
   return a;
 }

@@ -38,11 +38,13 @@ inline FluxConsts<double> flux_consts_of(const cato_config& c) {
 // rows, 512^2: 4, 1024^2: 16, 4096^2: 64 (1487 us a step at 128 x 64 against 2200 at 64 x 4; at
 // 1024^2 128 us at 64 x 16 against 178 at 128 x 32).
 //
-// Edge-parallel tiles (FP64, double-float): 32 columns and a single block of 4, 2 or 1 rows while
-// that leaves SMs idle otherwise (the chain of a block is the time of the launch: 64 x 48 HLLC
-// 75 us a step at 1 row, 85 at 4), else 64 columns, blocks of 4 rows and as many blocks per CTA
-// as leave about four waves of the two resident CTAs (1024^2: 2094 us at 8 rows, 2144 at 32;
-// 4096^2: 29.3 ms at 32 rows, 30.6 at 8).
+// Edge-parallel tiles (FP64, double-float).  While they leave SMs idle the chain of a block is the
+// time of the launch: 32 columns in the split form with a single block of 1 row (64 x 48 HLLC:
+// 55 us a step, 75 in the unsplit form) or 2 rows (128 x 100: 76 us, 86 unsplit at 4 rows; 200^2:
+// 166, 147 unsplit), then a single unsplit block of 4 (256^2: 225 us, 231 with 64 columns), from
+// two tiles per SM on 64 columns, blocks of 4 rows and as many blocks per CTA as leave about four
+// waves of the two resident CTAs (1024^2: 2094 us at 8 rows, 2144 at 32; 4096^2: 29.3 ms at 32
+// rows, 30.6 at 8).
 constexpr int kSMs = 152;
 inline StageShape default_shape(int ni, int nj, int ng, int precision) {
   auto tiles = [&](int columns, int rows) {
@@ -59,14 +61,21 @@ inline StageShape default_shape(int ni, int nj, int ng, int precision) {
     s.width = s.threads;
     return s;
   }
-  if (tiles(64, 4) < 2LL * kSMs) {
-    s.width = 64;
-    s.threads = 32;
-    s.block = 4;
-    while (s.block > 1 && tiles(32, s.block) < kSMs * 7 / 8) s.block /= 2;
-    s.rows = s.block;
+  s.width = 64;
+  s.threads = 32;
+  if (tiles(32, 1) <= kSMs) {
+    s.rows = s.block = 1;
+    s.warps = 12;
     return s;
   }
+  if (tiles(32, 2) <= 2 * kSMs + 16) {
+    s.rows = s.block = 2;
+    s.warps = 10;
+    return s;
+  }
+  s.warps = 9;
+  s.rows = s.block = 4;
+  if (tiles(64, 4) < 2LL * kSMs) return s;
   s.width = 128;
   s.threads = 64;
   s.block = 4;

@@ -34,6 +34,7 @@ struct StageArgs {
   int bc[4];               // by side: +x, +y, -x, -y
   int limiter;             // TVD2 limiter id (runtime)
   int rows_per_cta;
+  int block;               // edge-parallel tiles: rows of a block
   int kind;                // 0: out = U_a + L*c ; 1: out = (U_a*a + U_k*b) + L*c  (each '+'
                            // flushed) ; 2: out = L (flux_solver_t%solve output, FP64 path)
   int last;                // last stage of the step: emit the CFL dt and the state checks
@@ -213,8 +214,7 @@ __device__ __forceinline__ void edge_flux(const float* const rp[6], int T, int l
 
 // FP64 and double-float: one copy for both directions, which halves the code (these kernels are
 // sensitive to the instruction cache).  y: an edge along j; prim: shared memory, ro[k]: offset of
-// this column in row (edge row) + k - 2; a variable is T apart.  The fluxes run in the edge's
-// frame: the states' u and v are exchanged before, and the momentum fluxes after.
+// this column in row (edge row) + k - 2; a variable is T apart.
 template <int RECON>
 __device__ __forceinline__ EdgePair recon_edge(int lim, const double q[10]) {
   if constexpr (RECON == 0) return recon_tvd2_f64(lim, q[1], q[2], q[3], q[4]);
@@ -226,35 +226,35 @@ template <int RECON> __device__ __forceinline__ DfPair recon_edge(int lim, const
   else
     return recon_mlp_df_ool<RECON>(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7], q[8], q[9]);
 }
-template <typename R, int FLUX, int RECON>
-__device__ __forceinline__ void edge_flux_any(const R* prim, const int ro[6], int T, int lim, bool y,
-                                              const FluxConsts<R>& K, R F[4]) {
-  // offset of the sample n cells along and t cells across the edge normal
-  auto at = [&](int n, int t) { return y ? ro[n + 2] + t : ro[t + 2] + n; };
-  int o[10];
-  o[0] = RECON == 5 ? at(-2, 0) : 0;
-  o[1] = at(-1, 0);
-  o[2] = at(0, 0);
-  o[3] = at(1, 0);
-  o[4] = at(2, 0);
-  o[5] = RECON == 5 ? at(3, 0) : 0;
-  o[6] = at(0, 1);
-  o[7] = at(0, -1);
-  o[8] = at(1, 1);
-  o[9] = at(1, -1);
-  R Lv[4], Rv[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    R q[10];
-#pragma unroll
-    for (int m = 0; m < 10; ++m)
-      q[m] = (RECON == 0 && (m == 0 || m > 4)) || (RECON == 3 && (m == 0 || m == 5))
-                 ? R(0)
-                 : prim[o[m] + k * T];
-    const auto e = recon_edge<RECON>(lim, q);
-    Lv[k] = e.L;
-    Rv[k] = e.R;
+// the left and right state of variable k
+template <typename R, int RECON>
+__device__ __forceinline__ void edge_states(const R* prim, const int ro[6], int T, int lim, bool y,
+                                            int k, R& L, R& Rr) {
+  // the sample n cells along and t cells across the edge normal
+  auto Q = [&](int n, int t) -> R { return prim[(y ? ro[n + 2] + t : ro[t + 2] + n) + k * T]; };
+  R q[10];
+  q[1] = Q(-1, 0);
+  q[2] = Q(0, 0);
+  q[3] = Q(1, 0);
+  q[4] = Q(2, 0);
+  q[0] = RECON == 5 ? Q(-2, 0) : R(0);
+  q[5] = RECON == 5 ? Q(3, 0) : R(0);
+  if constexpr (RECON != 0) {
+    q[6] = Q(0, 1);
+    q[7] = Q(0, -1);
+    q[8] = Q(1, 1);
+    q[9] = Q(1, -1);
   }
+  const auto e = recon_edge<RECON>(lim, q);
+  L = e.L;
+  Rr = e.R;
+}
+// the flux from the states Lv, Rv in the edge's frame: u and v are exchanged before, and the
+// momentum fluxes after
+template <typename R, int FLUX>
+__device__ __forceinline__ void edge_flux_any(const R* prim, const int ro[6], int T, bool y,
+                                              const R Lv[4], const R Rv[4],
+                                              const FluxConsts<R>& K, R F[4]) {
   const Prim<R> A = {Lv[0], y ? Lv[2] : Lv[1], y ? Lv[1] : Lv[2], Lv[3]};
   const Prim<R> B = {Rv[0], y ? Rv[2] : Rv[1], y ? Rv[1] : Rv[2], Rv[3]};
   // cell pressures n along and t across the normal, with t counted so that the reference's lists
@@ -270,15 +270,8 @@ __device__ __forceinline__ void edge_flux_any(const R* prim, const int ro[6], in
     const R pc[4] = {P(0, -1), P(1, -1), P(0, 1), P(1, 1)};
     // the superbee edge states of the second interpolator (m_ausmpw_plus_solver.fypp:163-167)
     R Ls[4], Rs[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      R q[10] = {};
-#pragma unroll
-      for (int m = 1; m < 5; ++m) q[m] = prim[o[m] + k * T];
-      const auto e = recon_edge<0>(LIM_SUPERBEE, q);
-      Ls[k] = e.L;
-      Rs[k] = e.R;
-    }
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) edge_states<R, 0>(prim, ro, T, LIM_SUPERBEE, y, k, Ls[k], Rs[k]);
     const Prim<R> As = {Ls[0], y ? Ls[2] : Ls[1], y ? Ls[1] : Ls[2], Ls[3]};
     const Prim<R> Bs = {Rs[0], y ? Rs[2] : Rs[1], y ? Rs[1] : Rs[2], Rs[3]};
     flux_mausmpw<R, 0>(K, A, B, As, Bs, pc, G);
@@ -489,7 +482,8 @@ __device__ __forceinline__ void check_state(const StageArgs& A, ColumnConsts<R>&
   if constexpr (Prec<R>::kind == 0) {
     double u, v, p, cs;
     prim_from_cons(A.gamma, A.gamma - 1.0, un[0], un[1], un[2], un[3], u, v, p, cs);
-    double d = div_rn(A.cfl, div_rn(rabs(u) + cs, cg.dx) + div_rn(rabs(v) + cs, cg.dy));
+    double d = div_rn(A.cfl, quot_rn(rabs(u) + cs, cg.dx, cg.dx_y62) +
+                                  quot_rn(rabs(v) + cs, cg.dy, cg.dy_y62));
     if (d_less(d, C.dt_loc)) C.dt_loc = d;
     if (d_isnan(un[0]) || d_isnan(u) || d_isnan(v) || d_isnan(p)) C.st_loc |= ST_NAN;
     if (lt0(un[0])) C.st_loc |= ST_NEG_DENSITY;
@@ -868,22 +862,29 @@ __device__ __forceinline__ void stage_tile_tvd(const StageArgs& A, const FluxCon
 // ---------------------------------------------------------------------------------------------
 // the edge-parallel tile
 // ---------------------------------------------------------------------------------------------
-// One row of edges per warp (or per warp pair), both directions side by side: blockDim =
-// (T, 2 RW + 1), T = 32 or 64 columns incl. the x-halo.  The tile marches in blocks of RW rows.
-// Per block RW new rows of primitives enter a ring of RW + 2 NG rows, then threadIdx.y = 1 .. RW
-// makes the y edges above the block's rows (0 the one below the first block) and the others its x
-// edges, then all of them share the (cell, variable) updates; a barrier lies between the phases.
-// The serial chain of a block is one edge, against a row's two edges and update in the marching
-// strip, and a CTA has 2 RW + 1 times the warps for the same columns, so that small grids finish
-// early and the latency of the long FP64 chains is covered with few registers per thread.
+// Several warps (warp pairs with T = 64) on a segment of T columns incl. the x-halo: blockDim =
+// (T, nw), nw >= 2 RW + 1.  The tile marches in blocks of RW rows.  Per block RW new rows of
+// primitives enter a ring of RW + 2 NG rows; then every warp makes one row of edges, RW + 1 rows
+// of y edges (RW after the first block, whose lower row is carried) and RW rows of x edges side by
+// side; then all warps share the (cell, variable) updates, with a barrier after each phase.  The
+// serial chain of a block is one edge, against a row's two edges and update in the marching strip,
+// and a CTA has 2 RW + 1 times the warps for the same columns, so that the latency of the long
+// FP64 chains is covered with few registers per thread.
+//
+// SPLIT, for grids that leave SMs idle: the states of an edge row are made by one warp per
+// variable and handed over in shared memory, and nw may be larger, so that the chain is one
+// variable's states, one flux and one update (FP64 64 x 48: 75 -> 55 us a step; where the GPU is
+// full the hand-over costs 3 % in FP64 and 7 % in double-float).
 struct EdgeShape {
   int columns;  // T
   int block;    // RW
+  int warps;    // nw: 2 RW + 1, or more for the split form
+  constexpr bool split() const { return warps > 2 * block + 1; }
 };
-template <typename R, int NG, int FLUX, int RECON>
+template <typename R, int NG, int FLUX, int RECON, bool SPLIT>
 __device__ __forceinline__ void edge_tile(const StageArgs& A, const FluxConsts<R>& K, int bx,
                                           int by, unsigned char* smem_raw) {
-  const int T = blockDim.x, nw = blockDim.y, RW = nw >> 1, NR = RW + 2 * NG;
+  const int T = blockDim.x, nw = blockDim.y, RW = A.block, NR = RW + 2 * NG, NE = 2 * RW + 1;
   const int t = threadIdx.x, w = threadIdx.y;
   const int gx = bx * (T - 2 * NG) - NG + t;
   const int y0 = by * A.rows_per_cta, y1 = min(y0 + A.rows_per_cta, A.nj);
@@ -892,6 +893,7 @@ __device__ __forceinline__ void edge_tile(const StageArgs& A, const FluxConsts<R
   R* const sfx = prim + NR * 4 * T;                        // [RW][4][T] edge right of the cell
   R* const sfy = sfx + RW * 4 * T;                         // [RW + 1][4][T] edge above row e at
                                                            // slot (e - y0 + 1) % (RW + 1)
+  R* const st = sfy + (RW + 1) * 4 * T;                    // SPLIT: [NE][4][2][T] left and right states
   const R g = R(A.gamma), g1 = R(A.gamma - 1.0);
   bool flipx;
   const int sx = map_index(min(gx, A.ni + NG - 1), A.ni, A.bc[SIDE_MX], A.bc[SIDE_PX], flipx);
@@ -916,17 +918,50 @@ __device__ __forceinline__ void edge_tile(const StageArgs& A, const FluxConsts<R
     }
     next = upto;
     __syncthreads();
-    const bool along_y = w <= RW;
-    const int e = along_y ? yb - 1 + w : yb + w - RW - 1;  // the edges' (lower) row
-    if (e < y1 && (w > 0 || yb == y0)) {
-      const bool act = along_y ? in_cell : in_i_edge;
-      if (act) {
-        // rows e - 2 .. e + 3; NG = 2 reads e - 1 .. e + 2
-        int ro[6];
+    // edge row m: the y edges above row yb - 1 + m for m <= RW, else the x edges of row
+    // yb + m - RW - 1; none beyond the tile, and m = 0 only in the first block
+    auto edge_row = [&](int m) { return m <= RW ? yb - 1 + m : yb + m - RW - 1; };
+    auto edge_on = [&](int m) { return edge_row(m) < y1 && (m > 0 || yb == y0); };
+    // this column in rows e - 2 .. e + 3 (NG = 2 reads e - 1 .. e + 2)
+    auto rows_of = [&](int e, int ro[6]) {
+      int slot = (e - y0 + NG - 2 + NR) % NR;
 #pragma unroll
-        for (int k = 0; k < 6; ++k) ro[k] = (e - y0 + NG + k - 2 + NR) % NR * 4 * T + t;
-        R F[4];
-        edge_flux_any<R, FLUX, RECON>(prim, ro, T, A.limiter, along_y, K, F);
+      for (int k = 0; k < 6; ++k) {
+        ro[k] = slot * 4 * T + t;
+        slot = slot + 1 == NR ? 0 : slot + 1;
+      }
+    };
+    if constexpr (SPLIT) {
+      for (int n = w; n < NE * 4; n += nw) {
+        const int m = n >> 2, k = n & 3;
+        const bool along_y = m <= RW;
+        if (!edge_on(m) || !(along_y ? in_cell : in_i_edge)) continue;
+        int ro[6];
+        rows_of(edge_row(m), ro);
+        R L, Rr;
+        edge_states<R, RECON>(prim, ro, T, A.limiter, along_y, k, L, Rr);
+        st[(2 * n) * T + t] = L;
+        st[(2 * n + 1) * T + t] = Rr;
+      }
+      __syncthreads();
+    }
+    if (w < NE && edge_on(w)) {
+      const bool along_y = w <= RW;
+      if (along_y ? in_cell : in_i_edge) {
+        const int e = edge_row(w);
+        int ro[6];
+        rows_of(e, ro);
+        R L[4], Rr[4], F[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if constexpr (SPLIT) {
+            L[k] = st[(8 * w + 2 * k) * T + t];
+            Rr[k] = st[(8 * w + 2 * k + 1) * T + t];
+          } else {
+            edge_states<R, RECON>(prim, ro, T, A.limiter, along_y, k, L[k], Rr[k]);
+          }
+        }
+        edge_flux_any<R, FLUX>(prim, ro, T, along_y, L, Rr, K, F);
         R* out = along_y ? sfy + (e - y0 + 1) % (RW + 1) * 4 * T : sfx + (e - yb) * 4 * T;
 #pragma unroll
         for (int k = 0; k < 4; ++k) out[k * T + t] = F[k];
@@ -961,10 +996,10 @@ __device__ __forceinline__ void edge_tile(const StageArgs& A, const FluxConsts<R
   if (w < RW) reduce_column(A, C);
 }
 template <typename R> constexpr size_t edge_smem_bytes(EdgeShape s, int ng) {
-  return (size_t)s.columns * 4 *
-         (sizeof(double) * s.block + sizeof(R) * (size_t)(3 * s.block + 2 * ng + 1));
+  const size_t rows = 3 * s.block + 2 * ng + 1 + (s.split() ? 2 * (2 * s.block + 1) : 0);
+  return (size_t)s.columns * 4 * (sizeof(double) * s.block + sizeof(R) * rows);
 }
-constexpr int kEdgeThreads = 128 * 7;  // most threads of a CTA: 128 columns, blocks of 3 rows
+constexpr int kEdgeThreads = 1024;  // most threads of a CTA
 
 // ---------------------------------------------------------------------------------------------
 // kernels
@@ -1013,11 +1048,11 @@ __global__ void __launch_bounds__(256, CATO_F32_MIN_BLOCKS)
 // 56 registers (36 warps per SM) run best or within 3 % of it nearly everywhere measured; the
 // FP64 path offers two more to the tuner.
 constexpr int edge_regs(int variant) { return variant == 0 ? 56 : (variant == 1 ? 72 : 96); }
-template <typename R, int NG, int FLUX, int RECON, int REGS>
+template <typename R, int NG, int FLUX, int RECON, int REGS, bool SPLIT>
 __global__ void __maxnreg__(REGS) edge_kernel(const StageArgs A, const FluxConsts<R> K) {
   if (A.active && *A.active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  edge_tile<R, NG, FLUX, RECON>(A, K, blockIdx.x, blockIdx.y, smem_raw);
+  edge_tile<R, NG, FLUX, RECON, SPLIT>(A, K, blockIdx.x, blockIdx.y, smem_raw);
 }
 
 // whether a stage needs the EXT kernel (rectilinear grid, energy source, pressure input)
