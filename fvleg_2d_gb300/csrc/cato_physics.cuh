@@ -1000,6 +1000,7 @@ __device__ __forceinline__ void recon_mlp<df, 5>(df qm2, df qm1, df q0, df qp1, 
 template <typename R> struct FluxConsts {
   R gamma, g_over_gm1, gm1, two_gm1_over_gp1, gamma_factor, hllc_gf, harten_delta;
   R ausm_beta, ausm_kp, ausm_ku, ausm_sigma;
+  R cfl, rdx, rdy;  // CFL number and 1 / dx, 1 / dy of a uniform grid
   int low_mach_fix, harten;
   uint64_t gm1_y62;  // FP64: recip62 of gm1
 };
@@ -1025,6 +1026,9 @@ template <typename R> inline FluxConsts<R> convert_consts(const FluxConsts<doubl
   C.ausm_kp = R(K.ausm_kp);
   C.ausm_ku = R(K.ausm_ku);
   C.ausm_sigma = R(K.ausm_sigma);
+  C.cfl = R(K.cfl);
+  C.rdx = R(K.rdx);
+  C.rdy = R(K.rdy);
   C.low_mach_fix = K.low_mach_fix;
   C.harten = K.harten;
   return C;

@@ -25,6 +25,9 @@ inline FluxConsts<double> flux_consts_of(const cato_config& c) {
   K.ausm_kp = c.ausm_kp;
   K.ausm_ku = c.ausm_ku;
   K.ausm_sigma = c.ausm_sigma;
+  K.cfl = c.cfl;
+  K.rdx = 1.0 / c.dx;
+  K.rdy = 1.0 / c.dy;
   K.low_mach_fix = c.apply_low_mach_fix ? 1 : 0;
   K.gm1_y62 = intdiv::recip62(intdiv::bits_of(K.gm1));
   K.harten = c.roe_entropy_fix == CATO_ROE_HARTEN ? 1 : 0;

@@ -391,19 +391,22 @@ template <typename R> struct ColumnConsts {
   double dt_loc;           // smallest CFL dt and status bits of the column's new states
   int st_loc;
 
-  template <bool EXT> __device__ __forceinline__ void init(const StageArgs& A, int gx) {
+  // (the constants come converted with the scheme's: their FP64 divisions and conversions, per
+  // thread, were a quarter of the double-float kernel's FP64-pipe work)
+  template <bool EXT>
+  __device__ __forceinline__ void init(const StageArgs& A, const FluxConsts<R>& K, int gx) {
     cc = A.coef * *A.dt;
-    ccf = (float)cc;
-    cfl_f = (float)A.cfl;
     if constexpr (Prec<R>::kind == 2) {
-      dx_inv = to_df(A.G.rdxc ? A.G.rdxc[min(max(gx, 0), A.ni - 1)] : 1.0 / A.G.dx);
-      dy_inv = to_df(1.0 / A.G.dy);
-      cfl_df = to_df(A.cfl);
+      dx_inv = A.G.rdxc ? to_df(A.G.rdxc[min(max(gx, 0), A.ni - 1)]) : K.rdx;
+      dy_inv = K.rdy;
+      cfl_df = K.cfl;
       cc_df = to_df(cc);
     }
     if constexpr (Prec<R>::kind == 1) {
-      idx_col = (EXT && A.G.rdxf) ? A.G.rdxf[min(max(gx, 0), A.ni - 1)] : (float)(1.0 / A.G.dx);
-      idy_uni = (float)(1.0 / A.G.dy);  // one FP64 division per thread, not per row
+      ccf = (float)cc;
+      cfl_f = K.cfl;
+      idx_col = (EXT && A.G.rdxf) ? A.G.rdxf[min(max(gx, 0), A.ni - 1)] : K.rdx;
+      idy_uni = K.rdy;
     }
     dt_loc = INFINITY;
     st_loc = 0;
@@ -474,15 +477,16 @@ __device__ __forceinline__ double combine_var(const StageArgs& A, const ColumnCo
 
 // The CFL dt and the checks of a cell's new state (the last stage).
 template <typename R, bool EXT>
-__device__ __forceinline__ void check_state(const StageArgs& A, ColumnConsts<R>& C,
+__device__ __forceinline__ void check_state(const StageArgs& A, const FluxConsts<R>& K,
+                                            ColumnConsts<R>& C,
                                             [[maybe_unused]] const Geom& cg,
                                             [[maybe_unused]] int j, const double un[4]) {
-  [[maybe_unused]] const R g = R(A.gamma), g1 = R(A.gamma - 1.0);
+  [[maybe_unused]] const R g = K.gamma, g1 = K.gm1;
   // CFL dt of the new state (get_timestep, mod_fluid.f90:554-558) and the sanity checks
   if constexpr (Prec<R>::kind == 0) {
     double u, v, p, cs;
-    prim_from_cons(A.gamma, A.gamma - 1.0, un[0], un[1], un[2], un[3], u, v, p, cs);
-    double d = div_rn(A.cfl, quot_rn(rabs(u) + cs, cg.dx, cg.dx_y62) +
+    prim_from_cons(g, g1, un[0], un[1], un[2], un[3], u, v, p, cs);
+    double d = div_rn(K.cfl, quot_rn(rabs(u) + cs, cg.dx, cg.dx_y62) +
                                   quot_rn(rabs(v) + cs, cg.dy, cg.dy_y62));
     if (d_less(d, C.dt_loc)) C.dt_loc = d;
     if (d_isnan(un[0]) || d_isnan(u) || d_isnan(v) || d_isnan(p)) C.st_loc |= ST_NAN;
@@ -524,7 +528,8 @@ __device__ __forceinline__ void check_state(const StageArgs& A, ColumnConsts<R>&
 
 // FP32: one cell's divergence, stage combine and (in the last stage) CFL dt and state checks.
 template <bool EXT>
-__device__ __forceinline__ void update_cell(const StageArgs& A, ColumnConsts<float>& C, int gx, int j,
+__device__ __forceinline__ void update_cell(const StageArgs& A, const FluxConsts<float>& K,
+                                            ColumnConsts<float>& C, int gx, int j,
                                             size_t cidx, const double ua[4], const double uk[4],
                                             const float Fi_[4], const float Fim_[4], const float Fj_[4],
                                             const float Fjm_[4]) {
@@ -547,7 +552,7 @@ __device__ __forceinline__ void update_cell(const StageArgs& A, ColumnConsts<flo
     un[k] = r;
     A.Uo[k][cidx] = r;
   }
-  if (A.last) check_state<float, EXT>(A, C, cg, j, un);
+  if (A.last) check_state<float, EXT>(A, K, C, cg, j, un);
 }
 
 // The column's CFL dt and status into the step control.
@@ -597,14 +602,14 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, const FluxConsts<
   R* sfi = ring + RING * 4 * T;              // [4][T]   i-edge between cols t and t+1
   R* sfj = sfi + 4 * T;                      // [2][4][T] j-edge between rows j and j+1 at slot j&1
 
-  const R g = R(A.gamma), g1 = R(A.gamma - 1.0);
+  const R g = K.gamma, g1 = K.gm1;
   bool flipx;
   const int sx = map_index(min(gx, A.ni + NG - 1), A.ni, A.bc[SIDE_MX], A.bc[SIDE_PX], flipx);
   const int xmode = column_mode<EXT>(A, gx);
   const bool in_i_edge = (t >= NG - 1) && (t <= NG + W - 1) && (gx <= A.ni - 1);
   const bool in_cell = (t >= NG) && (t <= NG + W - 1) && (gx < A.ni);
   ColumnConsts<R> C;
-  C.template init<EXT>(A, gx);
+  C.template init<EXT>(A, K, gx);
   const R* rp[6];
 
   // prologue: rows y0-NG .. y0+NG-1
@@ -669,7 +674,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, const FluxConsts<
         Fj[k] = sfj[((j & 1) * 4 + k) * T + t];
         Fjm[k] = sfj[(((j - 1) & 1) * 4 + k) * T + t];
       }
-      update_cell<EXT>(A, C, gx, j, cidx, ua, uk, Fi, Fim, Fj, Fjm);
+      update_cell<EXT>(A, K, C, gx, j, cidx, ua, uk, Fi, Fim, Fj, Fjm);
     }
   }
   reduce_column(A, C);
@@ -731,14 +736,14 @@ __device__ __forceinline__ void stage_tile_tvd(const StageArgs& A, const FluxCon
   float* const sfi = srm + 8 * T;        // [2][4][T] flux of the edge right of the cell
   auto row_at = [&](int r) { return ring + ((r + RR) & (RR - 1)) * 4 * T; };
 
-  const float g = float(A.gamma), g1 = float(A.gamma - 1.0);
+  const float g = K.gamma, g1 = K.gm1;
   bool flipx;
   const int sx = map_index(min(gx, A.ni + NG - 1), A.ni, A.bc[SIDE_MX], A.bc[SIDE_PX], flipx);
   const int xmode = column_mode<EXT>(A, gx);
   const bool in_x = t >= 1 && t <= T - 2 && gx <= A.ni;  // columns whose x values are read
   const bool in_cell = t >= NG && t <= NG + W - 1 && gx < A.ni;
   ColumnConsts<float> C;
-  C.template init<EXT>(A, gx);
+  C.template init<EXT>(A, K, gx);
 
   auto prims_of = [&](const RowSrc<float>& src, int row, float q[4]) {
     src_to_prim<float>(A, src, flipx, xmode, row, g, g1, q);
@@ -810,12 +815,8 @@ __device__ __forceinline__ void stage_tile_tvd(const StageArgs& A, const FluxCon
     double ua[4], uk[4];
     if (in_cell) load_operands(A, cidx, ua, uk);
     float q2[4], Ft[4];
-    {
-      RowSrc<float> nxt;
-      if (j + 1 < y1) load_src<float>(A, sx, j + 3, nxt);
-      prims_of(pre, j + 2, q2);
-      pre = nxt;
-    }
+    prims_of(pre, j + 2, q2);
+    if (j + 1 < y1) load_src<float>(A, sx, j + 3, pre);
     store_row(j + 2, q2);
     // one block for both directions (columns without a cell compute values nobody reads), so that
     // the two chains overlap
@@ -851,7 +852,7 @@ __device__ __forceinline__ void stage_tile_tvd(const StageArgs& A, const FluxCon
         Fi[k] = sfi[((j & 1) * 4 + k) * T + t];
         Fim[k] = sfi[((j & 1) * 4 + k) * T + t - 1];
       }
-      update_cell<EXT>(A, C, gx, j, cidx, ua, uk, Fi, Fim, Ft, Fb);
+      update_cell<EXT>(A, K, C, gx, j, cidx, ua, uk, Fi, Fim, Ft, Fb);
 #pragma unroll
       for (int k = 0; k < 4; ++k) Fb[k] = Ft[k];
     }
@@ -894,14 +895,14 @@ __device__ __forceinline__ void edge_tile(const StageArgs& A, const FluxConsts<R
   R* const sfy = sfx + RW * 4 * T;                         // [RW + 1][4][T] edge above row e at
                                                            // slot (e - y0 + 1) % (RW + 1)
   R* const st = sfy + (RW + 1) * 4 * T;                    // SPLIT: [NE][4][2][T] left and right states
-  const R g = R(A.gamma), g1 = R(A.gamma - 1.0);
+  const R g = K.gamma, g1 = K.gm1;
   bool flipx;
   const int sx = map_index(min(gx, A.ni + NG - 1), A.ni, A.bc[SIDE_MX], A.bc[SIDE_PX], flipx);
   const int xmode = column_mode<true>(A, gx);
   const bool in_i_edge = t >= NG - 1 && t < T - NG && gx <= A.ni - 1;
   const bool in_cell = t >= NG && t < T - NG && gx < A.ni;
   ColumnConsts<R> C;
-  C.template init<true>(A, gx);
+  C.template init<true>(A, K, gx);
 
   int next = -NG;  // first row (relative to y0) not yet in the ring
   for (int yb = y0; yb < y1; yb += RW) {
@@ -990,7 +991,7 @@ __device__ __forceinline__ void edge_tile(const StageArgs& A, const FluxConsts<R
       const double* v = un + w * 4 * T + t;
       const double u4[4] = {v[0], v[T], v[2 * T], v[3 * T]};
       if constexpr (Prec<R>::kind == 2) C.set_row(A, j);
-      check_state<R, true>(A, C, cell_geom(A.G, gx, j), j, u4);
+      check_state<R, true>(A, K, C, cell_geom(A.G, gx, j), j, u4);
     }
   }
   if (w < RW) reduce_column(A, C);
