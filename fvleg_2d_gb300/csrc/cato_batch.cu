@@ -27,6 +27,7 @@ using namespace cato;
 namespace {
 
 __global__ void batch_step_begin(InstDesc* descs, int n, int* counters, int n_counters) {
+  wait_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n_counters) counters[i] = 0;
   if (i >= n) return;
@@ -48,6 +49,7 @@ __global__ void batch_step_begin(InstDesc* descs, int n, int* counters, int n_co
 
 // after the last stage: the uploaded primitives have been consumed
 __global__ void batch_step_end(InstDesc* descs, int n) {
+  wait_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   InstDesc& d = descs[i];
@@ -256,9 +258,8 @@ static int rebuild(cato_batch* b) {
 
 static int enqueue_batch_step(cato_batch* b) {
   const int nb = (std::max(b->capacity, b->n_counters_cap) + 127) / 128;
-  batch_step_begin<<<nb, 128, 0, b->stream>>>(b->d_descs, b->capacity, b->d_counters,
-                                              b->n_counters_cap);
-  BK(cudaGetLastError());
+  BK(launch_overlapped(batch_step_begin, dim3(nb), dim3(128), 0, b->stream, b->d_descs, b->capacity,
+                       b->d_counters, b->n_counters_cap));
   const int ns = (int)b->stages.size();
   const int ng = (int)b->groups.size();
   const bool fan = ng > 1;
@@ -286,8 +287,8 @@ static int enqueue_batch_step(cato_batch* b) {
       BK(cudaStreamWaitEvent(b->stream, b->side_done[g], 0));
     }
   }
-  batch_step_end<<<(b->capacity + 127) / 128, 128, 0, b->stream>>>(b->d_descs, b->capacity);
-  BK(cudaGetLastError());
+  BK(launch_overlapped(batch_step_end, dim3((b->capacity + 127) / 128), dim3(128), 0, b->stream,
+                       b->d_descs, b->capacity));
   return CATO_OK;
 }
 

@@ -82,6 +82,7 @@ __device__ __forceinline__ void batch_stage_args(InstDesc* d, const BatchStageAr
 // hands them to tile(A, descriptor, tile x, tile y).
 template <typename R, typename Tile>
 __device__ __forceinline__ void batch_loop(const BatchStageArgs& B, Tile tile) {
+  wait_previous();
   __shared__ int s_item;
   const bool first = threadIdx.x == 0 && threadIdx.y == 0;
   for (;;) {

@@ -288,8 +288,7 @@ static int enqueue_source(cato_handle* h) {
 // Enqueue one full time step (step control + every stage) on the handle's stream.
 // The step-control kernel and the step's energy source field.
 static int enqueue_step_begin(cato_handle* h) {
-  step_begin_kernel<<<1, 1, 0, h->stream>>>(h->ctl);
-  CK(cudaGetLastError());
+  CK(launch_overlapped(step_begin_kernel, dim3(1), dim3(1), 0, h->stream, h->ctl));
   {
     const int rcs = enqueue_source(h);
     if (rcs) return rcs;

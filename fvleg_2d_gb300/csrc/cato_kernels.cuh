@@ -10,6 +10,8 @@ namespace cato {
 
 // one thread: decide whether this step runs and with which dt (master_puppeteer.f90:155-200)
 static __global__ void step_begin_kernel(StepCtl* c) {
+  launch_next();
+  wait_previous();
   int act = (c->status == 0) && (c->time < c->t_end) && (c->iter < c->max_iter);
   c->active = act;
   if (!act) return;

@@ -72,9 +72,8 @@ cudaError_t launch_strip(const StageShape& s, bool warm, cudaStream_t stream, co
   if (e != cudaSuccess || warm) return e;
   const int W = s.threads - 2 * NG;
   const dim3 grid((A.ni + W - 1) / W, (A.nj + s.rows - 1) / s.rows);
-  stage_kernel<NG, FLUX, RECON, EXT>
-      <<<grid, s.threads, tile_smem_bytes(s.threads, NG, FLUX, TVD), stream>>>(A, K);
-  return cudaGetLastError();
+  return launch_overlapped(stage_kernel<NG, FLUX, RECON, EXT>, grid, dim3(s.threads),
+                           tile_smem_bytes(s.threads, NG, FLUX, TVD), stream, A, K);
 }
 
 template <typename R, int NG, int FLUX, int RECON, int REGS, bool SPLIT = false>
@@ -96,9 +95,8 @@ cudaError_t launch_edge(const StageShape& s, bool warm, cudaStream_t stream, con
   const dim3 grid((A.ni + W - 1) / W, (A.nj + s.rows - 1) / s.rows);
   StageArgs B = A;
   B.block = es.block;
-  edge_kernel<R, NG, FLUX, RECON, REGS, SPLIT>
-      <<<grid, dim3(es.columns, es.warps), edge_smem_bytes<R>(es, NG), stream>>>(B, K);
-  return cudaGetLastError();
+  return launch_overlapped(edge_kernel<R, NG, FLUX, RECON, REGS, SPLIT>, grid,
+                           dim3(es.columns, es.warps), edge_smem_bytes<R>(es, NG), stream, B, K);
 }
 
 // One stage of one grid; warm: only prepare every kernel of the scheme (outside stream captures).
@@ -189,8 +187,7 @@ cudaError_t launch_batch_one(int threads, cudaStream_t stream, const BatchStageA
   if (e != cudaSuccess) return e;
   long long grid = (long long)(per_sm > 0 ? per_sm : 1) * attr.sms[dev].load();
   if (grid > B.n_items) grid = B.n_items;
-  kernel<<<(unsigned)grid, block, smem, stream>>>(B);
-  return cudaGetLastError();
+  return launch_overlapped(kernel, dim3((unsigned)grid), block, smem, stream, B);
 }
 
 template <typename R, int FLUX>

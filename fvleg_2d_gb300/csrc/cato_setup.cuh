@@ -37,8 +37,8 @@ inline FluxConsts<double> flux_consts_of(const cato_config& c) {
 // Default single-grid launch shape.
 //
 // FP32 strips: as many rows per CTA (64 .. 1) as leave the GPU about full; a strip of r rows pays
-// for r + 1.5 of them.  Measured at 64 columns, best of 1 .. 64 rows: 64 x 48 and 256^2: 1 - 2
-// rows, 512^2: 4, 1024^2: 16, 4096^2: 64 (1487 us a step at 128 x 64 against 2200 at 64 x 4; at
+// for r + 1.5 of them.  Measured at 64 columns, best of 1 .. 64 rows: 64 x 48 and 200^2: 1
+// row, 300^2: 2 (25.3 us, 36.3 at 1), 512^2: 4, 1024^2: 16, 4096^2: 64 (1487 us a step at 128 x 64 against 2200 at 64 x 4; at
 // 1024^2 128 us at 64 x 16 against 178 at 128 x 32).
 //
 // Edge-parallel tiles (FP64, double-float).  While they leave SMs idle the chain of a block is the
@@ -58,7 +58,8 @@ inline StageShape default_shape(int ni, int nj, int ng, int precision) {
   if (precision == CATO_MIXED) {
     s.threads = 64;
     s.rows = 64;
-    while (s.rows > 1 && tiles(64, s.rows) < 7LL * kSMs) s.rows /= 2;
+    while (s.rows > 2 && tiles(64, s.rows) < 7LL * kSMs) s.rows /= 2;
+    if (tiles(64, 2) < 3LL * kSMs) s.rows = 1;  // 200^2: 20.8 us a step, 23.3 at 2 rows
     if (s.rows >= 32) s.threads = 128;
     if (s.threads - 2 * ng > ni + 2 * ng) s.threads = 64;
     s.width = s.threads;

@@ -14,6 +14,7 @@
 // because for every valid side combination the final ghost value is that composition.
 #pragma once
 
+#include "cato_ctl.cuh"
 #include "cato_physics.cuh"
 
 namespace cato {
@@ -677,6 +678,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, const FluxConsts<
       update_cell<EXT>(A, K, C, gx, j, cidx, ua, uk, Fi, Fim, Fj, Fjm);
     }
   }
+  launch_next();
   reduce_column(A, C);
 }
 
@@ -857,6 +859,7 @@ __device__ __forceinline__ void stage_tile_tvd(const StageArgs& A, const FluxCon
       for (int k = 0; k < 4; ++k) Fb[k] = Ft[k];
     }
   }
+  launch_next();
   reduce_column(A, C);
 }
 
@@ -1040,6 +1043,7 @@ constexpr bool batch_tvd_tile_of(int flux, int recon) {
 template <int NG, int FLUX, int RECON, bool EXT>
 __global__ void __launch_bounds__(256, CATO_F32_MIN_BLOCKS)
     stage_kernel(const StageArgs A, const FluxConsts<float> K) {
+  wait_previous();
   if (A.active && *A.active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   tile_of<NG, FLUX, RECON, EXT>(A, K, blockIdx.x, blockIdx.y, smem_raw);
@@ -1051,6 +1055,7 @@ __global__ void __launch_bounds__(256, CATO_F32_MIN_BLOCKS)
 constexpr int edge_regs(int variant) { return variant == 0 ? 56 : (variant == 1 ? 72 : 96); }
 template <typename R, int NG, int FLUX, int RECON, int REGS, bool SPLIT>
 __global__ void __maxnreg__(REGS) edge_kernel(const StageArgs A, const FluxConsts<R> K) {
+  wait_previous();
   if (A.active && *A.active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   edge_tile<R, NG, FLUX, RECON, SPLIT>(A, K, blockIdx.x, blockIdx.y, smem_raw);
