@@ -104,9 +104,7 @@ __device__ __forceinline__ void batch_loop(const BatchStageArgs& B, Tile tile) {
 
 // FP32; no rectilinear grid, source or pressure input in a batch: the lean tile
 template <int NG, int FLUX, int RECON>
-__global__ void __launch_bounds__(256, batch_tvd_tile_of(FLUX, RECON)
-                                           ? CATO_F32_BATCH_TVD_MIN_BLOCKS
-                                           : CATO_F32_BATCH_MIN_BLOCKS)
+__global__ void __maxnreg__(f32_batch_regs(FLUX, RECON))
     batch_stage_kernel(const BatchStageArgs B) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   batch_loop<float>(B, [&](const StageArgs& A, const InstDesc* d, int bx, int by) {

@@ -36,10 +36,10 @@ inline FluxConsts<double> flux_consts_of(const cato_config& c) {
 
 // Default single-grid launch shape.
 //
-// FP32 strips: as many rows per CTA (64 .. 1) as leave the GPU about full; a strip of r rows pays
-// for r + 1.5 of them.  Measured at 64 columns, best of 1 .. 64 rows: 64 x 48 and 200^2: 1
-// row, 300^2: 2 (25.3 us, 36.3 at 1), 512^2: 4, 1024^2: 16, 4096^2: 64 (1487 us a step at 128 x 64 against 2200 at 64 x 4; at
-// 1024^2 128 us at 64 x 16 against 178 at 128 x 32).
+// FP32 strips of 64 columns: as many rows per CTA (32 .. 1) as leave the GPU about full; a strip
+// of r rows pays for r + 1.5 of them, and more than 32 leave a long last wave (3000 x 2010 Roe:
+// 797 us a step at 32 rows, 1050 at 64 rows of 128 columns; 4096^2 HLLC 1314 and 1328). Best of 1
+// .. 64 rows: 64 x 48 and 200^2: 1 row, 300^2: 2 (25.3 us, 36.3 at 1), 512^2: 4, 1024^2: 16.
 //
 // Edge-parallel tiles (FP64, double-float).  While they leave SMs idle the chain of a block is the
 // time of the launch: 32 columns in the split form with a single block of 1 row (64 x 48 HLLC:
@@ -57,11 +57,9 @@ inline StageShape default_shape(int ni, int nj, int ng, int precision) {
   StageShape s;
   if (precision == CATO_MIXED) {
     s.threads = 64;
-    s.rows = 64;
+    s.rows = 32;
     while (s.rows > 2 && tiles(64, s.rows) < 7LL * kSMs) s.rows /= 2;
     if (tiles(64, 2) < 3LL * kSMs) s.rows = 1;  // 200^2: 20.8 us a step, 23.3 at 2 rows
-    if (s.rows >= 32) s.threads = 128;
-    if (s.threads - 2 * ng > ni + 2 * ng) s.threads = 64;
     s.width = s.threads;
     return s;
   }

@@ -1026,22 +1026,21 @@ constexpr bool batch_tvd_tile_of(int flux, int recon) {
   return tvd_tile_of(flux, recon) && flux != FLUX_AUSMPW;
 }
 
-// Minimum resident 256-thread CTAs per SM requested from the register allocator: the single-grid
-// kernels run best unconstrained, the persistent batch kernels of the general tile at 4 (64
-// registers; +4.5 % on the batched workload), those of the TVD2 tile, whose carried rows need
-// more, at 2
-#ifndef CATO_F32_MIN_BLOCKS
-#define CATO_F32_MIN_BLOCKS 1
-#endif
-#ifndef CATO_F32_BATCH_MIN_BLOCKS
-#define CATO_F32_BATCH_MIN_BLOCKS 4
-#endif
-#ifndef CATO_F32_BATCH_TVD_MIN_BLOCKS
-#define CATO_F32_BATCH_TVD_MIN_BLOCKS 2
-#endif
+// Registers per thread of the FP32 kernels.
+// Single grids: HLLC, Roe and AUSM+-up with the TVD2 tile at 104 (the compiler's 113 to 135 leave
+// four 128-thread CTAs on an SM; 4096^2 HLLC 1469 -> 1307 us a step), the others the compiler's
+// choice, where a cap changes which products the assembler fuses and with it the rounding.
+// Batches: the general tile at 64 (+4.5 % on the batched workload), the TVD2 tile at 128.
+constexpr int f32_regs(int flux, int recon) {
+  const bool capped = flux == FLUX_HLLC || flux == FLUX_ROE || flux == FLUX_AUSM_UP;
+  return recon == 0 && capped ? 104 : 255;
+}
+constexpr int f32_batch_regs(int flux, int recon) {
+  return batch_tvd_tile_of(flux, recon) ? 128 : 64;
+}
 
 template <int NG, int FLUX, int RECON, bool EXT>
-__global__ void __launch_bounds__(256, CATO_F32_MIN_BLOCKS)
+__global__ void __maxnreg__(f32_regs(FLUX, RECON))
     stage_kernel(const StageArgs A, const FluxConsts<float> K) {
   wait_previous();
   if (A.active && *A.active == 0) return;
