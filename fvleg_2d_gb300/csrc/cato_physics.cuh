@@ -316,13 +316,11 @@ __device__ __forceinline__ float d2f_int(double d) {
 }
 // f2d: exact; float denormals flush to zero.
 __device__ __forceinline__ double f2d_int(float f) {
-  unsigned b = __float_as_uint(f);
-  unsigned sign = b & 0x80000000u, e = (b >> 23) & 0xffu, m = b & 0x7fffffu;
-  unsigned hi, lo = m << 29;
-  if (e == 0u) { hi = sign; lo = 0u; }
-  else if (e == 255u) hi = sign | 0x7ff00000u | (m >> 3);
-  else hi = sign | ((e + 896u) << 20) | (m >> 3);
-  return __hiloint2double((int)hi, (int)lo);
+  const unsigned b = __float_as_uint(f), mag = b & 0x7fffffffu;
+  unsigned hi = (mag >> 3) + (896u << 20), lo = b << 29;
+  if (mag < 0x00800000u) hi = lo = 0u;             // zero, denormal
+  if (mag >= 0x7f800000u) hi += 0x38000000u;       // infinity, NaN: the exponent on to 0x7ff
+  return __hiloint2double((int)(hi | (b & 0x80000000u)), (int)lo);
 }
 
 // FP64 -> FP32 for the mixed path's stencil values: the exponent rebiased and the fraction
@@ -339,11 +337,31 @@ __device__ __forceinline__ float d2f_fast(double d) {
   return __uint_as_float((hi << 1) >= (897u << 21) ? (m | sign) : sign);
 }
 
-// FP64 <-> df: hi = the FP64 value rounded to FP32, lo = the (exact) remainder rounded to FP32;
-// one FP64 add, the conversions on the integer pipe.
-__device__ __forceinline__ df to_df(double d) {
+// FP64 -> df: hi = the FP64 value rounded to FP32, lo = the (exact) remainder rounded to FP32.
+static __device__ __noinline__ df to_df_any(double d) {
   const float h = d2f_int(d);
   return df(h, d2f_int(d - f2d_int(h)));
+}
+// The same from the bits, for 2^-60 <= |d| < 2^100: the 29 fraction bits below hi's last place are
+// the remainder as an integer, which one conversion rounds to FP32 and a power of two scales.  16
+// instructions and none on the FP64 pipe, against 61 and one.
+__device__ __forceinline__ df to_df(double d) {
+  const unsigned h = (unsigned)__double2hiint(d), l = (unsigned)__double2loint(d);
+  const unsigned e = h & 0x7ff00000u;  // biased exponent << 20
+  if (e - ((1023u - 60u) << 20) >= (160u << 20)) {
+    if (((h << 1) | l) == 0u) return df(__uint_as_float(h), 0.0f);  // a zero velocity
+    return to_df_any(d);
+  }
+  const unsigned m = __funnelshift_l(l, h, 3) - (384u << 23);  // rebiased exponent, 23 bits; sign lost
+  const int s = (int)h >> 31;
+  int rem = (int)(l & 0x1fffffffu);
+  // to nearest, ties to even
+  const bool up = (unsigned)rem + (m & 1u) > 0x10000000u;
+  if (up) rem -= 0x20000000;
+  const float hi = __uint_as_float((m + (up ? 1u : 0u)) | (h & 0x80000000u));
+  // 2^(E - 52) for the exponent E of d
+  const float scale = __uint_as_float((e << 3) - ((1023u - 127u + 52u) << 23));
+  return df(hi, __fmul_rn(__int2float_rn((rem ^ s) - s), scale));
 }
 __device__ __forceinline__ double from_df(df a) { return f2d_int(a.hi) + f2d_int(a.lo); }
 
