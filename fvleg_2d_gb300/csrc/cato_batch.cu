@@ -186,8 +186,9 @@ static int rebuild(cato_batch* b) {
   // Rows per tile, at most the plan's.  FP32 strips hide their latency with neighbours: the most
   // rows that leave five tiles per SM (served stream, 1.1 M cells: 1.93 ms per 16 steps at 8 rows,
   // 3.06 at 32).  The edge-parallel tiles fill an SM with two: what counts is the share of the
-  // busiest SM, its tiles times the rows they hold and the edges they repeat (FP64 sweep of
-  // 0.29 M cells: 19.9 ms at 4 rows with 9 tiles on an SM, 24.4 at 16 rows with 3).
+  // busiest SM, its tiles times the rows they hold and the edges they repeat (16 steps of an FP64
+  // sweep of 0.29 M cells: 19.9 ms at 4 rows with 9 tiles on an SM, 24.4 at 16 rows with 3; MLP5,
+  // 16 grids up to 512^2: 21.7 ms at 24 rows with 2, 25.0 at 16 with 3), over the multiples of four.
   auto n_tiles = [&](int r) {
     long long n = 0;
     for (int i : order) {
@@ -203,7 +204,7 @@ static int rebuild(cato_batch* b) {
       tile_rows = std::max(4, tile_rows / 2);
   } else {
     auto share = [&](int r) { return (double)((n_tiles(r) + b->sms - 1) / b->sms) * (r + 1.2); };
-    for (int r = tile_rows / 2; r >= 4; r /= 2)
+    for (int r = (tile_rows - 1) / 4 * 4; r >= 4; r -= 4)
       if (share(r) < share(tile_rows)) tile_rows = r;
   }
   b->tile_rows = tile_rows;

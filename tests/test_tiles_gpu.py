@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from conftest import random_prims
+from fvleg_2d_gb300.batch import Batch
 from fvleg_2d_gb300.config import SchemeConfig
 from fvleg_2d_gb300.fluid import Fluid, FluxSolver
 
@@ -97,3 +98,23 @@ def test_limiter_decisions_equal_the_oracle(oracle, limiter, flux):
     got = FluxSolver(cfg).solve(*[p.copy(order="F") for p in prims])
     for k in range(4):
         np.testing.assert_array_equal(got[k], want[k])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed_df"])
+@pytest.mark.parametrize("rows", [5, 12, 24, 28, 32])
+def test_batch_rows_that_are_no_power_of_two(precision, rows):
+    cfgs = [_cfg(ni, nj, "MLP5", "HLLC", precision) for ni, nj in [(59, 25), (200, 127), (16, 57)]]
+    prims = [random_prims(c, np.random.default_rng(c.ni)) for c in cfgs]
+    batch = Batch(len(cfgs), precision=precision, integration_strategy="ssp_rk3")
+    batch.set_plan(128, rows)
+    slots = [batch.add(c, p) for c, p in zip(cfgs, prims)]
+    batch.step(3)
+    for cfg, p, slot in zip(cfgs, prims, slots):
+        f = Fluid(cfg).initialize(*p)
+        f.run_timed(3)
+        want = f.state(FIELDS)
+        f.close()
+        got = batch.state(slot)
+        for k in FIELDS:
+            np.testing.assert_array_equal(got[k], want[k], err_msg=f"{k} {cfg.ni}")
+    batch.close()
