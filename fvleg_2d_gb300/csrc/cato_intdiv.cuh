@@ -13,11 +13,10 @@
 //      and 11.3: Newton-Raphson iterations for the reciprocal and the reciprocal square root);
 //   3. the quotient a y1 (or the root a y1) from three 32 x 32-bit partial products of the
 //      64 x 64-bit product, within 43 units of 2^-61 (29 units of 2^-60 for the root) of the exact
-//      value, far inside the 128 units the next step allows, then the nearest significand M1;
-//   4. the exact rounding decision: the signs of the integer remainders
-//      2^k A - (2 M1 +- 1) B (division) or 2^k A - (2 M1 +- 1)^2 (square root), computed
-//      modulo 2^64 because their magnitudes are below 2^63, decide between M1 - 1, M1 and
-//      M1 + 1, with ties to even.
+//      value, far inside the 128 units the next step allows, and its floor F as a significand;
+//   4. the exact rounding decision: the sign of the integer remainder 2^k A - (2 F + 1) B
+//      (division) or 2^k A - (2 F + 1)^2 (square root), computed modulo 2^64 because its
+//      magnitude is below 2^63, decides between F and F + 1; neither has ties.
 // Exact scalings by 2^-1, 2^-2, 2^-3 and 2 (scale_down, scale_up1) are exponent steps here.
 // Operands that are zero, subnormal, infinite or NaN, negative square-root operands and quotients
 // outside the normal range take the hardware instruction instead (the caller's fallback).
@@ -130,11 +129,9 @@ CATO_HD float rsqrt_seed(float x) {
 constexpr uint64_t kFrac = 0x000fffffffffffffULL;
 constexpr uint64_t kHid = 0x0010000000000000ULL;
 
-// y * 2^30 as an integer for an FP32 seed y near [0.5, 1] (24 significant bits: exact)
-CATO_HD uint32_t fixed30(float y) {
-  const uint32_t yb = fbits_of(y);
-  return ((yb & 0x7fffffu) | 0x800000u) << ((yb >> 23) - 120u);
-}
+// y * 2^30 as an integer for an FP32 seed y in [0.5, 1]: its bits count units of 2^-24 from 0.5
+// (a seed an ulp or two outside becomes another one as near)
+CATO_HD uint32_t fixed30(float y) { return fbits_of(y) * 64u - 0x3e800000u * 64u; }
 
 // y0 (1 + t) * 2^62 for y0 = Y0 / 2^30 and t = T / 2^80 (floor of the correction term)
 CATO_HD uint64_t refine62(uint32_t Y0, int64_t T) {
@@ -155,10 +152,11 @@ CATO_HD uint64_t refine62(uint32_t Y0, int64_t T) {
 //   Y1 = 2^62 y0 (1 + T / 2^80): |Y1 - 2^62 / b'| < 2 (the omitted e^3 term: 2^-57 at most);
 //   H ~ A 2^11 Y1 / 2^64 (mulhi3): |H - 2^61 A / B| < 43;
 //   n = 1 when H < 2^61 (quotient below 1), and with the quotient's significand in [1, 2) as
-//   Hn = 2^n H, An = 2^n A: M1 = round(Hn / 2^9) is within 0.17 + 1/2 of X = 2^53 An / B, so
-//   RN(X) is M1 - 1, M1 or M1 + 1, decided by the signs of Z = 2^53 An - (2 M1 + 1) B and
-//   Z + 2 B (|Z| < 2^55).  Where n is taken wrongly (|H - 2^61| < 43), X lies within 0.17 of
-//   2^52 or 2^53 and either choice rounds to the same value.
+//   Hn = 2^n H, An = 2^n A: Hn / 2^9 is within 0.17 of X = 2^52 An / B, so RN(X) is
+//   F = floor(Hn / 2^9) or F + 1, decided by the sign of Z = 2^53 An - (2 F + 1) B (|Z| < 2^55,
+//   and not 0: the odd 2 F + 1 >= 2^53 would divide A).  Where n is taken wrongly
+//   (|H - 2^61| < 43), X lies within 0.17 of 2^52 or 2^53 and either choice rounds to the same
+//   value.
 // Y1 depends on b alone (recip62): quotients by the same divisor share it (quot_bits).
 CATO_HD uint64_t recip62(uint64_t ub) {
   const uint64_t B = (ub & kFrac) | kHid;
@@ -170,25 +168,19 @@ CATO_HD uint64_t recip62(uint64_t ub) {
   return refine62(Y0, T);
 }
 CATO_HD uint64_t quot_bits(uint64_t ua, uint64_t ub, uint64_t Y1, bool& ok) {
-  const uint32_t ea = (uint32_t)(ua >> 52) & 0x7ffu, eb = (uint32_t)(ub >> 52) & 0x7ffu;
+  const uint32_t ha = (uint32_t)(ua >> 32), hb = (uint32_t)(ub >> 32);
+  const uint32_t ea = ha & 0x7ff00000u, eb = hb & 0x7ff00000u;  // exponents in place
   const uint64_t A = (ua & kFrac) | kHid, B = (ub & kFrac) | kHid;
   const uint64_t H = mulhi3(A << 11, Y1);
   const uint32_t n = (uint32_t)(H >> 61) ^ 1u;
-  const uint64_t Hn = H << n, An = A << n;
-  const uint64_t M1 = (Hn + 256u) >> 9;
-  const int64_t Z = (int64_t)((An << 53) - (2 * M1 + 1) * B);
-  uint64_t M = M1;
-  if (Z > 0 || (Z == 0 && (M1 & 1))) {
-    M = M1 + 1;
-  } else {
-    const int64_t W = Z + (int64_t)(2 * B);  // 2^53 An - (2 M1 - 1) B
-    if (W < 0 || (W == 0 && (M1 & 1))) M = M1 - 1;
-  }
-  const int32_t Ef = (int32_t)ea - (int32_t)eb + 1023 - (int32_t)n;
-  ok = (ea - 1u < 2046u) && (eb - 1u < 2046u) && (Ef >= 1) && (Ef <= 2045);
-  const uint64_t sign = (ua ^ ub) & 0x8000000000000000ULL;
-  // M in [2^52, 2^53]: M = 2^53 carries into the exponent field
-  return sign | (((uint64_t)(uint32_t)Ef << 52) + (M - kHid));
+  const uint64_t F = H >> (9u - n);
+  const int64_t Z = (int64_t)(((uint64_t)((uint32_t)A << (21u + n)) << 32) - (2 * F + 1) * B);
+  const int32_t Ef = (int32_t)ea - (int32_t)eb + ((1022 - (int32_t)n) << 20);
+  ok = (ea - 0x100000u < 2046u << 20) && (eb - 0x100000u < 2046u << 20) && Ef >= 0 &&
+       Ef <= (int32_t)(2044u << 20);
+  const uint32_t sign = (ha ^ hb) & 0x80000000u;
+  // F in [2^52, 2^53): its leading bit and a carry go into the exponent field
+  return ((uint64_t)(sign + (uint32_t)Ef) << 32) + F + (Z > 0 ? 1u : 0u);
 }
 CATO_HD uint64_t div_bits(uint64_t ua, uint64_t ub, bool& ok) {
   return quot_bits(ua, ub, recip62(ub), ok);
@@ -203,8 +195,8 @@ CATO_HD uint64_t div_bits(uint64_t ua, uint64_t ub, bool& ok) {
 //   T = E / 2 + 3 floor(Eh^2 / 2^19) = 2^80 (e/2 + 3e^2/8);  Y1 = 2^62 y0 (1 + T / 2^80), within
 //   6 units (the omitted 5e^3/16 term: 2^-58.7 at most);
 //   H ~ A2 2^10 Y1 / 2^64 (mulhi3): |H - 2^60 sqrt(a'')| < 29, inside the 128 the rounding
-//   allows;
-//   M1 = round(H / 2^8), Z = 2^54 A2 - (2 M1 + 1)^2 (never 0), |Z| < 2^56.
+//   allows, so the root is F = floor(H / 2^8) or F + 1: the sign of
+//   Z = 2^54 A2 - (2 F + 1)^2 (never 0), |Z| < 2^56.
 CATO_HD uint64_t sqrt_bits(uint64_t ua, bool& ok) {
   const uint32_t ea = (uint32_t)(ua >> 52) & 0x7ffu;
   const uint32_t odd = (ea & 1u) ^ 1u;  // the unbiased exponent ea - 1075 is odd
@@ -222,15 +214,11 @@ CATO_HD uint64_t sqrt_bits(uint64_t ua, bool& ok) {
   const int64_t T = (E >> 1) + 3 * (((int64_t)Eh * Eh) >> 19);
   const uint64_t Y1 = refine62(Y0, T);
   const uint64_t H = mulhi3(A2 << 10, Y1);
-  const uint64_t M1 = (H + 128u) >> 8;
-  const uint64_t N = 2 * M1 + 1;
-  const int64_t Z = (int64_t)((A2 << 54) - N * N);
-  uint64_t M = M1;
-  if (Z > 0) M = M1 + 1;
-  else if (Z + (int64_t)(8 * M1) < 0) M = M1 - 1;  // 2^54 A2 - (2 M1 - 1)^2 < 0
+  const uint64_t F = H >> 8, N = 2 * F + 1;
+  const int64_t Z = (int64_t)(((uint64_t)((uint32_t)A2 << 22) << 32) - N * N);
   ok = (ea - 1u < 2046u) && !(ua >> 63);
-  const uint32_t Ef = 512u + ((ea - odd) >> 1);  // 1049 + (ea - 1075 - odd) / 2
-  return (((uint64_t)Ef << 52) + (M - kHid));
+  const uint32_t Ef = 511u + ((ea - odd) >> 1);  // 1048 + (ea - 1075 - odd) / 2
+  return (((uint64_t)Ef << 52) + F) + (Z > 0 ? 1u : 0u);  // F's leading bit adds one to Ef
 }
 
 // RN(a * b) as bits for normal a, b with a normal product; ok = false otherwise (zero, subnormal,
