@@ -167,20 +167,27 @@ CATO_HD uint64_t recip62(uint64_t ub) {
   const int64_t T = E + (((int64_t)Eh * Eh) >> 16);
   return refine62(Y0, T);
 }
-CATO_HD uint64_t quot_bits(uint64_t ua, uint64_t ub, uint64_t Y1, bool& ok) {
+// quot_mag: |a / b|, for operands and a quotient known to be normal.
+CATO_HD uint64_t quot_mag(uint64_t ua, uint64_t ub, uint64_t Y1) {
   const uint32_t ha = (uint32_t)(ua >> 32), hb = (uint32_t)(ub >> 32);
-  const uint32_t ea = ha & 0x7ff00000u, eb = hb & 0x7ff00000u;  // exponents in place
   const uint64_t A = (ua & kFrac) | kHid, B = (ub & kFrac) | kHid;
   const uint64_t H = mulhi3(A << 11, Y1);
   const uint32_t n = (uint32_t)(H >> 61) ^ 1u;
   const uint64_t F = H >> (9u - n);
   const int64_t Z = (int64_t)(((uint64_t)((uint32_t)A << (21u + n)) << 32) - (2 * F + 1) * B);
-  const int32_t Ef = (int32_t)ea - (int32_t)eb + ((1022 - (int32_t)n) << 20);
-  ok = (ea - 0x100000u < 2046u << 20) && (eb - 0x100000u < 2046u << 20) && Ef >= 0 &&
-       Ef <= (int32_t)(2044u << 20);
-  const uint32_t sign = (ha ^ hb) & 0x80000000u;
-  // F in [2^52, 2^53): its leading bit and a carry go into the exponent field
-  return ((uint64_t)(sign + (uint32_t)Ef) << 32) + F + (Z > 0 ? 1u : 0u);
+  // the exponents are subtracted in place; F in [2^52, 2^53): its leading bit and a carry go into
+  // the exponent field
+  const uint32_t Ef = (ha & 0x7ff00000u) - (hb & 0x7ff00000u) + ((1022u - n) << 20);
+  return ((uint64_t)Ef << 32) + F + (Z > 0 ? 1u : 0u);
+}
+CATO_HD uint64_t quot_bits(uint64_t ua, uint64_t ub, uint64_t Y1, bool& ok) {
+  const uint32_t ha = (uint32_t)(ua >> 32), hb = (uint32_t)(ub >> 32);
+  const uint64_t q = quot_mag(ua, ub, Y1);
+  const uint32_t ea = ha & 0x7ff00000u, eb = hb & 0x7ff00000u;
+  // exponents 1..2046, and the quotient's from their difference, which cannot wrap
+  const uint32_t d = ea - eb + (1022u << 20);
+  ok = ea - 0x100000u < 2046u << 20 && eb - 0x100000u < 2046u << 20 && d - 0x100000u < 2044u << 20;
+  return q ^ ((uint64_t)((ha ^ hb) & 0x80000000u) << 32);
 }
 CATO_HD uint64_t div_bits(uint64_t ua, uint64_t ub, bool& ok) {
   return quot_bits(ua, ub, recip62(ub), ok);

@@ -30,7 +30,13 @@ namespace cato {
 // kernel instead of one per call site keeps the stage kernels inside the instruction cache
 // (+18 % FP64 cell-updates/s on the 4096^2 quadrant, +55 % on the serving mix, where five flux
 // kernels run side by side).
-static __device__ __noinline__ double div_hw(double a, double b) { return a / b; }
+// A signed zero over a finite non-zero b (flat data) is the zero with the sign of the product.
+static __device__ __noinline__ double div_hw(double a, double b) {
+  const uint64_t ua = intdiv::bits_of(a), ub = intdiv::bits_of(b);
+  if ((ua << 1) == 0ULL && (ub << 1) != 0ULL && ((ub >> 52) & 0x7ffULL) != 0x7ffULL)
+    return intdiv::double_of((ua ^ ub) & 0x8000000000000000ULL);
+  return a / b;
+}
 static __device__ __noinline__ double sqrt_hw(double a) { return ::sqrt(a); }
 static __device__ __noinline__ double div_rn(double a, double b) {
   bool ok;
@@ -69,14 +75,8 @@ template <> constexpr bool kFP32<float> = true;
 template <> struct Num<double> {
   static constexpr double eps = 2.220446049250313080847263336181640625e-16;  // epsilon(1.0_rk)
   static constexpr double tiny = 2.2250738585072013830902327173324040642e-308; // tiny(1.0_rk)
-  // IEEE a / b on the integer pipe (div_rn).  A signed zero over a finite non-zero b (flat
-  // data) is the zero with the sign of the product, decided before the general routine.
-  static __device__ __forceinline__ double div(double a, double b) {
-    const uint64_t ua = intdiv::bits_of(a), ub = intdiv::bits_of(b);
-    if ((ua << 1) == 0ULL && (ub << 1) != 0ULL && ((ub >> 52) & 0x7ffULL) != 0x7ffULL)
-      return intdiv::double_of((ua ^ ub) & 0x8000000000000000ULL);
-    return div_rn(a, b);
-  }
+  // IEEE a / b on the integer pipe
+  static __device__ __forceinline__ double div(double a, double b) { return div_rn(a, b); }
   // sqrt(+-0) = +-0 (a zero velocity), else sqrt_rn
   static __device__ __forceinline__ double sqrt(double a) {
     if ((intdiv::bits_of(a) << 1) == 0ULL) return a;
@@ -100,9 +100,6 @@ template <> struct Rcp<double> {
 };
 template <typename R> __device__ __forceinline__ R div_by(R a, const Rcp<R>& c);
 template <> __device__ __forceinline__ double div_by<double>(double a, const Rcp<double>& c) {
-  const uint64_t ua = intdiv::bits_of(a), ub = intdiv::bits_of(c.b);
-  if ((ua << 1) == 0ULL && (ub << 1) != 0ULL && ((ub >> 52) & 0x7ffULL) != 0x7ffULL)
-    return intdiv::double_of((ua ^ ub) & 0x8000000000000000ULL);
   return quot_rn(a, c.b, c.y);
 }
 
@@ -641,20 +638,19 @@ static __device__ __noinline__ EdgePair recon_mlp_any(double qm2, double qm1, do
 __device__ __forceinline__ double add_small(double x) {
   return (uint32_t)(mag_bits(x) >> 32) >= ((1023u - 45u) << 20) ? x : x + 1e-30;
 }
-// RN(a / b) for normal operands and a normal quotient
+// RN(|a / b|) for normal operands and a normal quotient
 static __device__ __noinline__ double div_normal(double a, double b) {
-  bool ok;
-  return intdiv::double_of(intdiv::div_bits(intdiv::bits_of(a), intdiv::bits_of(b), ok));
+  const uint64_t ub = intdiv::bits_of(b);
+  return intdiv::double_of(intdiv::quot_mag(intdiv::bits_of(a), ub, intdiv::recip62(ub)));
 }
 // two of them, whose chains overlap
 struct D2 {
   double x, y;
 };
 static __device__ __noinline__ D2 div_normal2(double a0, double b0, double a1, double b1) {
-  bool ok;
-  const uint64_t q0 = intdiv::div_bits(intdiv::bits_of(a0), intdiv::bits_of(b0), ok);
-  const uint64_t q1 = intdiv::div_bits(intdiv::bits_of(a1), intdiv::bits_of(b1), ok);
-  return {intdiv::double_of(q0), intdiv::double_of(q1)};
+  const uint64_t u0 = intdiv::bits_of(b0), u1 = intdiv::bits_of(b1);
+  return {intdiv::double_of(intdiv::quot_mag(intdiv::bits_of(a0), u0, intdiv::recip62(u0))),
+          intdiv::double_of(intdiv::quot_mag(intdiv::bits_of(a1), u1, intdiv::recip62(u1)))};
 }
 // q + t or q - t: q itself for a zero t and a non-zero q, on the integer pipe
 __device__ __forceinline__ double add_slope(double q, double t, bool minus) {
@@ -804,50 +800,50 @@ static __device__ __noinline__ EdgePair recon_tvd2_f64(int lim, double qm1, doub
                                                       double qp2) {
   const double EPS = Num<double>::eps;
   double dm = q0 - qm1, d0 = qp1 - q0, dp = qp2 - qp1;
-  if (abs_lt(dm, EPS)) dm = 0.0;
-  if (abs_lt(d0, EPS)) d0 = 0.0;
-  if (abs_lt(dp, EPS)) dp = 0.0;
-  const uint32_t most = max((uint32_t)(mag_bits(d0) >> 32), max((uint32_t)(mag_bits(dm) >> 32),
-                                                                (uint32_t)(mag_bits(dp) >> 32)));
+  const uint64_t um = intdiv::bits_of(dm), u0 = intdiv::bits_of(d0), up = intdiv::bits_of(dp);
+  const uint32_t hm = (uint32_t)(um >> 32), h0 = (uint32_t)(u0 >> 32), hp = (uint32_t)(up >> 32);
+  const uint32_t am = hm & 0x7fffffffu, a0 = h0 & 0x7fffffffu, ap = hp & 0x7fffffffu;
+  const uint32_t flush = (1023u - 52u) << 20;  // |x| < epsilon by the high word
   EdgePair e;
-  if (most >= (1023u + 60u) << 20) {  // extreme differences, NaN and infinities: the general form
+  if (max(a0, max(am, ap)) >= (1023u + 60u) << 20) {
+    // extreme differences, NaN and infinities: the general form
+    if (abs_lt(dm, EPS)) dm = 0.0;
+    if (abs_lt(d0, EPS)) d0 = 0.0;
+    if (abs_lt(dp, EPS)) dp = 0.0;
     e.L = slope_step(q0, tvd_phi_edge(lim, d0, dm), dm, false);
     e.R = slope_step(qp1, tvd_phi_edge(lim, d0, dp), dp, true);
     return e;
   }
-  if (lim == LIM_VANLEER) {
-    // both sides' quotients in pairs (1024^2 HLLC: 1484 -> 1434 us a step, two at a time; pairing
-    // the fluxes' quotients too costs registers: MLP3 + HLLC 1933 -> 2107); a side without a slope
-    // divides 1 by 1
-    const uint64_t b0 = intdiv::bits_of(d0);
-    const bool fl = mag_bits(d0) == 0ULL || mag_bits(dm) == 0ULL ||
-                    ((b0 ^ intdiv::bits_of(dm)) & kSignBit) != 0ULL;
-    const bool fr = mag_bits(d0) == 0ULL || mag_bits(dp) == 0ULL ||
-                    ((b0 ^ intdiv::bits_of(dp)) & kSignBit) != 0ULL;
-    double tl = intdiv::double_of(intdiv::bits_of(dm) & kSignBit);
-    double tr = intdiv::double_of(intdiv::bits_of(dp) & kSignBit);
-    if (!fl || !fr) {
-      const D2 r = div_normal2(fl ? 1.0 : d0, fl ? 1.0 : dm + 1e-16, fr ? 1.0 : d0,
-                               fr ? 1.0 : dp + 1e-16);
-      const D2 phi = div_normal2(twice(r.x), 1.0 + r.x, twice(r.y), 1.0 + r.y);
-      if (!fl) tl = half_normal(phi.x) * dm;
-      if (!fr) tr = half_normal(phi.y) * dp;
+  // sides without a slope: a difference flushed to zero, or a ratio below zero
+  const bool fl = a0 < flush || am < flush || (int)(h0 ^ hm) < 0;
+  const bool fr = a0 < flush || ap < flush || (int)(h0 ^ hp) < 0;
+  e.L = q0;
+  e.R = qp1;
+  if (!(fl && fr)) {
+    double tl, tr;
+    if (lim == LIM_VANLEER) {
+      // both sides' quotients in pairs (1024^2 HLLC: 1484 -> 1434 us a step, two at a time; pairing
+      // the fluxes' quotients too costs registers: MLP3 + HLLC 1933 -> 2107).  half(phi(r)) is
+      // r / (1 + r).
+      const D2 r = div_normal2(d0, dm + 1e-16, d0, dp + 1e-16);
+      const D2 phi = div_normal2(r.x, 1.0 + r.x, r.y, 1.0 + r.y);
+      tl = phi.x * dm;
+      tr = phi.y * dp;
+    } else {
+      tl = fl ? 0.0 : tvd_side_f64(lim, d0, dm);
+      tr = fr ? 0.0 : tvd_side_f64(lim, d0, dp);
     }
-    e.L = add_slope(q0, tl, false);
-    e.R = add_slope(qp1, tr, true);
-    return e;
+    tl = q0 + tl;
+    tr = qp1 - tr;
+    if (!fl) e.L = tl;
+    if (!fr) e.R = tr;
   }
-#pragma unroll 1
-  for (int s = 0; s < 2; ++s) {
-    const double dq = s ? dp : dm;
-    const bool flat = mag_bits(d0) == 0ULL || mag_bits(dq) == 0ULL ||
-                      ((intdiv::bits_of(d0) ^ intdiv::bits_of(dq)) & kSignBit) != 0ULL;
-    const double t = flat ? intdiv::double_of(intdiv::bits_of(dq) & kSignBit)
-                          : tvd_side_f64(lim, d0, dq);
-    const double v = add_slope(s ? qp1 : q0, t, s != 0);
-    if (s) e.R = v;
-    else e.L = v;
-  }
+  // a flat side adds (on the right subtracts) the zero with the sign of its difference, which only
+  // shows on a zero: -0 stays one where both are negative
+  if (fl && mag_bits(q0) == 0ULL)
+    e.L = intdiv::double_of(am < flush ? 0ULL : intdiv::bits_of(q0) & um);
+  if (fr && mag_bits(qp1) == 0ULL)
+    e.R = intdiv::double_of(intdiv::bits_of(qp1) & (ap < flush ? kSignBit : ~up));
   return e;
 }
 
