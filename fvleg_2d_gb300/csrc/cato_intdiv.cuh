@@ -278,5 +278,37 @@ CATO_HD double scale_up1(double x) {
   return double_of(u + (1ULL << 52));
 }
 
+// x + 1e-16, rounded to nearest even.  1e-16 = C 2^-106 with C = 0x1cd2b297d889bc; against an x of
+// exponent field E >= 992 (2^-31) it is C 2^(969 - E) < 2^30 units of x's last place, never a tie
+// (C's last set bit is its third).  Its rounded value is added to the bit pattern unless x is so
+// near the ends of its binade that the sum could leave it.  ok = false: not computed here.
+CATO_HD uint64_t add_1em16_bits(uint64_t x, bool& ok) {
+  const uint32_t hi = (uint32_t)(x >> 32), s = (hi & 0x7fffffffu) - (992u << 20);
+  ok = s < (1000u << 20) && ((hi + 1) & 0xfffffu) > 1u;
+  const uint32_t sh = (s >> 20) + 1;
+#ifdef __CUDA_ARCH__
+  const uint32_t c = __funnelshift_rc(0xe69594beu, 0u, sh);
+#else
+  const uint32_t c = sh < 32 ? 0xe69594beu >> sh : 0u;
+#endif
+  const int32_t inc = (int32_t)((c + 1) >> 1), sg = (int32_t)hi >> 31;
+  return x + (uint64_t)(int64_t)((inc ^ sg) - sg);
+}
+
+// 1 + x for x in [2^-32, 2), rounded to nearest even: the significand of x shifted to units of
+// 2^-52 (from 1 up: its fraction, to units of 2^-51 above 2) by a multiplication, whose low word
+// decides the rounding.  ok = false: not computed here (adding the 1 in place from 2 up takes more
+// than it saves: 24.9 against 24.7 ms a step at 4096^2).
+CATO_HD uint64_t one_plus_bits(uint64_t x, bool& ok) {
+  const uint32_t hi = (uint32_t)(x >> 32), lo = (uint32_t)x, E = hi >> 20;
+  ok = E - 991u <= 32u;
+  const bool up = E == 1023u;
+  const uint32_t p = 1u << (((up ? 1022u : E) - 991u) & 31u);
+  const uint32_t mh = (hi & 0xfffffu) | (up ? 0u : 1u << 20);
+  const uint64_t a = (uint64_t)lo * p, q = (uint64_t)mh * p + (a >> 32);
+  const uint32_t odd = (uint32_t)q & 1u, round = (uint32_t)a > 0x80000000u - odd;
+  return q + (((uint64_t)(up ? 0x40000000u : 0x3ff00000u) << 32) + round);
+}
+
 }  // namespace intdiv
 }  // namespace cato

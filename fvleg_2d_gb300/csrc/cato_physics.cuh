@@ -245,9 +245,12 @@ __device__ __forceinline__ double div_by_twice<double>(double a, const Rcp<doubl
 // FP64 on the integer pipe: b * 0 is the zero with the sign of b when b is finite (NaN
 // otherwise), and a + (+-0) is a unless a is a zero, where -0 results only from -0 + -0.
 template <typename R> __device__ __forceinline__ R add_mul0(R a, R b) { return a + b * R(0); }
+// (the rare forms of these two are out of line: inline, the compiler executes their FP64 operations
+// under a predicate, which takes the pipe's time all the same)
+static __device__ __noinline__ double add_mul0_any(double a, double b) { return a + b * 0.0; }
 template <> __device__ __forceinline__ double add_mul0<double>(double a, double b) {
   const uint64_t ua = intdiv::bits_of(a), ub = intdiv::bits_of(b);
-  if ((ub << 1) >= 0xffe0000000000000ULL) return a + b * 0.0;  // b infinite or NaN
+  if ((ub << 1) >= 0xffe0000000000000ULL) return add_mul0_any(a, b);  // b infinite or NaN
   if ((ua << 1) != 0ULL) return a;
   return intdiv::double_of(ua & ub & kSignBit);
 }
@@ -258,11 +261,15 @@ template <typename R> __device__ __forceinline__ R add_zeros(R x, R a, R b, R c,
   return x + ((a * R(0) * b) + (c * R(0) * d));
 }
 __device__ __forceinline__ bool d_finite(double x) { return mag_bits(x) < kInfBits; }
+static __device__ __noinline__ double add_zeros_any(double x, double a, double b, double c,
+                                                    double d) {
+  return x + ((a * 0.0 * b) + (c * 0.0 * d));
+}
 template <>
 __device__ __forceinline__ double add_zeros<double>(double x, double a, double b, double c,
                                                     double d) {
   if (mag_bits(x) != 0ULL && d_finite(a) && d_finite(b) && d_finite(c) && d_finite(d)) return x;
-  return x + ((a * 0.0 * b) + (c * 0.0 * d));
+  return add_zeros_any(x, a, b, c, d);
 }
 
 // |x| < c for c > 0 without an FP compare: bit patterns of non-negative IEEE values order like
@@ -652,6 +659,26 @@ static __device__ __noinline__ D2 div_normal2(double a0, double b0, double a1, d
   return {intdiv::double_of(intdiv::quot_mag(intdiv::bits_of(a0), u0, intdiv::recip62(u0))),
           intdiv::double_of(intdiv::quot_mag(intdiv::bits_of(a1), u1, intdiv::recip62(u1)))};
 }
+// x + c and y + c (out of line, so that the compiler branches to it)
+static __device__ __noinline__ D2 add2(double x, double y, double c) { return {x + c, y + c}; }
+// x + 1e-16 and 1 + x of two values (anyx, anyy: any value will do): on the integer pipe where both
+// allow it, which takes 4 of a van Leer edge variable's 11 FP64 operations away (4096^2 HLLC 26.2 ->
+// 24.7 ms a step; with the additions inline the compiler executed them under a predicate, which
+// takes as long: 28.5)
+__device__ __forceinline__ D2 add_1em16(double x, double y, bool anyx, bool anyy) {
+  bool okx, oky;
+  const uint64_t a = intdiv::add_1em16_bits(intdiv::bits_of(x), okx);
+  const uint64_t b = intdiv::add_1em16_bits(intdiv::bits_of(y), oky);
+  if (!((okx || anyx) && (oky || anyy))) return add2(x, y, 1e-16);
+  return {intdiv::double_of(a), intdiv::double_of(b)};
+}
+__device__ __forceinline__ D2 one_plus(double x, double y, bool anyx, bool anyy) {
+  bool okx, oky;
+  const uint64_t a = intdiv::one_plus_bits(intdiv::bits_of(x), okx);
+  const uint64_t b = intdiv::one_plus_bits(intdiv::bits_of(y), oky);
+  if (!((okx || anyx) && (oky || anyy))) return add2(x, y, 1.0);
+  return {intdiv::double_of(a), intdiv::double_of(b)};
+}
 // q + t or q - t: q itself for a zero t and a non-zero q, on the integer pipe
 __device__ __forceinline__ double add_slope(double q, double t, bool minus) {
   if (mag_bits(t) == 0ULL && mag_bits(q) != 0ULL) return q;
@@ -780,7 +807,9 @@ static __device__ __noinline__ EdgePair recon_mlp_f64(double qm2, double qm1, do
 // least 1, or between 1/2 and 1, or of at least 2, gives phi by comparing the operands: a rounded
 // quotient is below 1 exactly when its operands are so ordered).
 __device__ __forceinline__ double tvd_side_f64(int lim, double d0, double dq) {
-  const double D = dq + 1e-16;
+  bool ok;
+  double D = intdiv::double_of(intdiv::add_1em16_bits(intdiv::bits_of(dq), ok));
+  if (!ok) D = add2(dq, 0.0, 1e-16).x;
   const uint64_t m = mag_bits(d0), d = mag_bits(D), one = 1ULL << 52;
   int k = -1;  // half(phi) = r 2^k where the ratio itself is needed
   if (lim == LIM_MINMOD) {
@@ -825,8 +854,10 @@ static __device__ __noinline__ EdgePair recon_tvd2_f64(int lim, double qm1, doub
       // both sides' quotients in pairs (1024^2 HLLC: 1484 -> 1434 us a step, two at a time; pairing
       // the fluxes' quotients too costs registers: MLP3 + HLLC 1933 -> 2107).  half(phi(r)) is
       // r / (1 + r).
-      const D2 r = div_normal2(d0, dm + 1e-16, d0, dp + 1e-16);
-      const D2 phi = div_normal2(r.x, 1.0 + r.x, r.y, 1.0 + r.y);
+      const D2 D = add_1em16(dm, dp, fl, fr);
+      const D2 r = div_normal2(d0, D.x, d0, D.y);
+      const D2 n = one_plus(r.x, r.y, fl, fr);
+      const D2 phi = div_normal2(r.x, n.x, r.y, n.y);
       tl = phi.x * dm;
       tr = phi.y * dp;
     } else {
