@@ -226,6 +226,29 @@ template <> __device__ __forceinline__ double eighth<double>(double x) {
 }
 template <> __device__ __forceinline__ double twice<double>(double x) { return intdiv::scale_up1(x); }
 
+// half(x + |x|) and half(x - |x|): x or +0.  FP64 by the sign, but for values whose double overflows.
+template <typename R> __device__ __forceinline__ R pos_half(R x) { return half(x + rabs(x)); }
+template <typename R> __device__ __forceinline__ R neg_half(R x) { return half(x - rabs(x)); }
+static __device__ __noinline__ double pos_half_any(double x) { return half(x + rabs(x)); }
+static __device__ __noinline__ double neg_half_any(double x) { return half(x - rabs(x)); }
+template <> __device__ __forceinline__ double pos_half<double>(double x) {
+  const uint64_t u = intdiv::bits_of(x);
+  if ((u & ~kSignBit) >= 0x7fe0000000000000ULL) return pos_half_any(x);
+  return (u & kSignBit) ? 0.0 : x;
+}
+template <> __device__ __forceinline__ double neg_half<double>(double x) {
+  const uint64_t u = intdiv::bits_of(x);
+  if ((u & ~kSignBit) >= 0x7fe0000000000000ULL) return neg_half_any(x);
+  return (u & kSignBit) ? x : 0.0;
+}
+// half(1 + fsign1(x)): 1, or 0 for a set sign bit
+template <typename R> __device__ __forceinline__ R half_one_plus_sign(R x) {
+  return half(R(1) + fsign1(x));
+}
+template <> __device__ __forceinline__ double half_one_plus_sign<double>(double x) {
+  return intdiv::bits_of(x) & kSignBit ? 0.0 : 1.0;
+}
+
 // a / twice(b) by the reciprocal of b.  FP64: half the quotient, exactly, unless that leaves the
 // normal range.
 template <typename R> __device__ __forceinline__ R div_by_twice(R a, const Rcp<R>& c) {
@@ -640,10 +663,13 @@ static __device__ __noinline__ EdgePair recon_mlp_any(double qm2, double qm1, do
   return e;
 }
 
+// (out of line, so that the compiler branches to it)
+static __device__ __noinline__ double add_1em30(double x) { return x + 1e-30; }
 // x + 1e-30 (the limiter's SMALL_NUM): x itself from 2^-45 up, where 1e-30 is below half a unit in
 // the last place (and below half a unit of the next lower binade); infinities and NaN pass.
 __device__ __forceinline__ double add_small(double x) {
-  return (uint32_t)(mag_bits(x) >> 32) >= ((1023u - 45u) << 20) ? x : x + 1e-30;
+  if ((uint32_t)(mag_bits(x) >> 32) >= ((1023u - 45u) << 20)) return x;
+  return add_1em30(x);
 }
 // RN(|a / b|) for normal operands and a normal quotient
 static __device__ __noinline__ double div_normal(double a, double b) {
@@ -1111,21 +1137,21 @@ template <typename R> struct Prim { R r, u, v, p; };
 
 // AUSMPW+ split functions, ausmpw_plus_solver.fypp:486-530 (alpha = 1/8)
 template <typename R> __device__ __forceinline__ R aw_p_plus(R M) {
-  if (abs_gt(M, R(1))) return half(R(1) + fsign1(M));
+  if (abs_gt(M, R(1))) return half_one_plus_sign(M);
   return quarter((M + R(1)) * (M + R(1))) * (R(2) - M) +
          eighth(M) * ((M * M - R(1)) * (M * M - R(1)));
 }
 template <typename R> __device__ __forceinline__ R aw_p_minus(R M) {
-  if (abs_gt(M, R(1))) return half(R(1) - fsign1(M));
+  if (abs_gt(M, R(1))) return half_one_plus_sign(rneg(M));
   return quarter((M - R(1)) * (M - R(1))) * (R(2) + M) -
          eighth(M) * ((M * M - R(1)) * (M * M - R(1)));
 }
 template <typename R> __device__ __forceinline__ R aw_m_plus(R M) {
-  if (abs_gt(M, R(1))) return half(M + rabs(M));
+  if (abs_gt(M, R(1))) return pos_half(M);
   return quarter((M + R(1)) * (M + R(1)));
 }
 template <typename R> __device__ __forceinline__ R aw_m_minus(R M) {
-  if (abs_gt(M, R(1))) return half(M - rabs(M));
+  if (abs_gt(M, R(1))) return neg_half(M);
   return -quarter((M - R(1)) * (M - R(1)));
 }
 
@@ -1251,12 +1277,12 @@ __device__ __forceinline__ void flux_ausmpw(const FluxConsts<R>& K, const Prim<R
 // U_L/U_R/V_L/V_R are taken before the low-Mach fix, as in the reference.
 template <typename R>
 __device__ __forceinline__ R mausm_p_plus(R M) {
-  if (abs_gt(M, R(1))) return half(R(1) + fsign1(M));
+  if (abs_gt(M, R(1))) return half_one_plus_sign(M);
   return quarter((M + R(1)) * (M + R(1))) * (R(2) - M);
 }
 template <typename R>
 __device__ __forceinline__ R mausm_p_minus(R M) {
-  if (abs_gt(M, R(1))) return half(R(1) - fsign1(M));
+  if (abs_gt(M, R(1))) return half_one_plus_sign(rneg(M));
   return quarter((M - R(1)) * (M - R(1))) * (R(2) + M);
 }
 template <typename R>
@@ -1367,6 +1393,19 @@ __device__ __forceinline__ void flux_mausmpw(const FluxConsts<R>& K, const Prim<
   if (abs_lt(F[3], EPSF)) F[3] = R(0);
 }
 
+// x (1 - g), g = -max(min(Mp, 0), -1) min(max(Mm, 0), 1).  FP64: g is a zero, and the product x,
+// unless the flow leaves the edge on both sides (or a NaN is among the Mach numbers).
+template <typename R> __device__ __forceinline__ R slau_limited(R x, R Mp, R Mm) {
+  return x * (R(1) - -(rmax(rmin(Mp, R(0)), R(-1)) * rmin(rmax(Mm, R(0)), R(1))));
+}
+static __device__ __noinline__ double slau_limited_any(double x, double Mp, double Mm) {
+  return x * (1.0 - -(rmax(rmin(Mp, 0.0), -1.0) * rmin(rmax(Mm, 0.0), 1.0)));
+}
+template <> __device__ __forceinline__ double slau_limited<double>(double x, double Mp, double Mm) {
+  if ((ge0(Mp) && !d_isnan(Mm)) || (nonpos(Mm) && !d_isnan(Mp))) return x;
+  return slau_limited_any(x, Mp, Mm);
+}
+
 // SLAU / SLAU2 / SD-SLAU / SD-SLAU2, slau_solver.fypp:332-490.  dpair[6][2]: delta_p1..6 cells.
 template <typename R, int DIR, int VARIANT>
 __device__ __forceinline__ void flux_slau(const FluxConsts<R>& K, const Prim<R>& A, const Prim<R>& B,
@@ -1400,10 +1439,10 @@ __device__ __forceinline__ void flux_slau(const FluxConsts<R>& K, const Prim<R>&
   R rho_bar = half(rho_L + rho_R);
   R B_plus, B_minus;
   if (abs_lt(M_plus, R(1))) B_plus = quarter(R(2) - M_plus) * ((M_plus + R(1)) * (M_plus + R(1)));
-  else B_plus = half(R(1) + fsign1(M_plus));
+  else B_plus = half_one_plus_sign(M_plus);
   if (abs_lt(M_minus, R(1)))
     B_minus = quarter(R(2) + M_minus) * ((M_minus - R(1)) * (M_minus - R(1)));
-  else B_minus = half(R(1) + fsign1(rneg(M_minus)));
+  else B_minus = half_one_plus_sign(rneg(M_minus));
   R delta_p = p_R - p_L;
   if (abs_lt(delta_p, EPS) || lt(rabs(delta_p), THRESHOLD * p_bar)) delta_p = R(0);
   R delta_rho = rho_R - rho_L;
@@ -1433,12 +1472,11 @@ __device__ __forceinline__ void flux_slau(const FluxConsts<R>& K, const Prim<R>&
   else
     p_tilde = p_bar + (half(delta_B) * pLmR) +
               Num<R>::sqrt(vel2) * (B_plus + B_minus - R(1)) * rho_bar * c_bar;
-  R gg = -(rmax(rmin(M_plus, R(0)), R(-1)) * rmin(rmax(M_minus, R(0)), R(1)));
   R diss = (VARIANT == FLUX_SLAU || VARIANT == FLUX_SLAU2) ? Chi : theta;
-  R mf = half((rho_L * Vp) + (rho_R * Vm) - rabs(V_n_bar) * delta_rho) * (R(1) - gg) -
-         (div_by_twice(diss, rc_c) * delta_p);
-  R mL = half(mf + rabs(mf));
-  R mR = half(mf - rabs(mf));
+  const R mh = half((rho_L * Vp) + (rho_R * Vm) - rabs(V_n_bar) * delta_rho);
+  R mf = slau_limited(mh, M_plus, M_minus) - (div_by_twice(diss, rc_c) * delta_p);
+  R mL = pos_half(mf);
+  R mR = neg_half(mf);
   const R gq = R(K.g_over_gm1);
   R H_L = gq * div_by(p_L, rc_L) + half(u_L * u_L + v_L * v_L);
   R H_R = gq * div_by(p_R, rc_R) + half(u_R * u_R + v_R * v_R);
@@ -1589,8 +1627,8 @@ __device__ __forceinline__ void flux_roe(const FluxConsts<R>& K, const Prim<R>& 
 }
 
 // AUSM+-up (basic), ausm_plus_solver.f90:499-643 + upwinding of the commented driver :313-325.
-template <typename R> __device__ __forceinline__ R up_m1p(R M) { return half(M + rabs(M)); }
-template <typename R> __device__ __forceinline__ R up_m1m(R M) { return half(M - rabs(M)); }
+template <typename R> __device__ __forceinline__ R up_m1p(R M) { return pos_half(M); }
+template <typename R> __device__ __forceinline__ R up_m1m(R M) { return neg_half(M); }
 template <typename R> __device__ __forceinline__ R up_m2p(R M) { return quarter((M + R(1)) * (M + R(1))); }
 template <typename R> __device__ __forceinline__ R up_m2m(R M) { return -quarter((M - R(1)) * (M - R(1))); }
 
@@ -1795,23 +1833,37 @@ inline Geom uniform_geom(double dx, double dy) {
   return G;
 }
 
-// x * p for p = 2^k (k != kNotPow2): the exponent step when x and the product are normal, a
-// signed zero for a zero x (p > 0); otherwise (and for any p that is not a power of two) the
-// FP64 instruction; bit-identical to x * p
+// x * p for p = 2^k: the exponent step when x and the product are normal, a signed zero for a zero
+// x (p > 0); otherwise the FP64 instruction (out of line, so that the compiler branches to it);
+// bit-identical to x * p
+static __device__ __noinline__ double mul_hw(double x, double p) { return x * p; }
 __device__ __forceinline__ double mul_pow2(double x, double p, int k) {
   const uint64_t u = intdiv::bits_of(x);
   const int e = (int)((u >> 52) & 0x7ffu);
-  if (k != kNotPow2) {
-    if ((u << 1) == 0ULL) return x;
-    if (e >= 1 && e <= 2046 && e + k >= 1 && e + k <= 2046)
-      return intdiv::double_of(u + ((uint64_t)(int64_t)k << 52));
-  }
-  return x * p;
+  if ((u << 1) == 0ULL) return x;
+  if (e >= 1 && e <= 2046 && e + k >= 1 && e + k <= 2046)
+    return intdiv::double_of(u + ((uint64_t)(int64_t)k << 52));
+  return mul_hw(x, p);
+}
+
+// a, or +0 for |a| below s 1e-14 (s >= 1), which it is not from 2^-45 of s's binade up
+static __device__ __noinline__ double flush_below(double a, double s) {
+  return mag_bits(a) < intdiv::bits_of(s * 1e-14) ? 0.0 : a;
+}
+__device__ __forceinline__ double flush_rel(double a, double s) {
+  const uint64_t ma = mag_bits(a);
+  const int ha = (int)(uint32_t)(ma >> 32), hs = (int)(uint32_t)(intdiv::bits_of(s) >> 32);
+  if (ha >= (hs & 0x7ff00000) - (45 << 20)) return a;
+  if (ma == 0ULL) return 0.0;
+  return flush_below(a, s);
 }
 
 // one direction's difference: (F l - Fm lm), the fluxes scaled by the larger of them and 1
+// (flux_solver.f90:448-475).  POW2: the lengths are 2^k and 2^km.
+template <bool POW2>
 __device__ __forceinline__ double scaled_difference(double F, double Fm, double l, int k, double lm,
                                                     int km) {
+  auto mul = [](double x, double p, int e) { return POW2 ? mul_pow2(x, p, e) : x * p; };
   const double REL_TOL = 1e-14;
   const uint64_t ONE = 0x3ff0000000000000ULL;
   // max(|F|, |Fm|, 1) by magnitude bits; with a NaN among them the scale and the result are NaN
@@ -1819,28 +1871,37 @@ __device__ __forceinline__ double scaled_difference(double F, double Fm, double 
   m = m > mm ? m : mm;
   double a;
   if (m <= ONE) {  // the scale is 1: x / 1 and x * 1 are x itself
-    a = mul_pow2(F, l, k) - mul_pow2(Fm, lm, km);
+    a = mul(F, l, k) - mul(Fm, lm, km);
     if (abs_lt(a, REL_TOL)) a = 0.0;
     return a;
   }
   const double s = intdiv::double_of(m);
   if (m >= kInfBits) return (F / s * l - Fm / s * lm) * s;  // infinite or NaN: NaN
-  // the larger flux over the scale, itself, is +-1: one division is left
+  // the larger flux over the scale, itself, is +-1, its product the length with that sign: one
+  // division and one product are left
   const bool first = mag_bits(F) == m;
-  const double q = Num<double>::div(first ? Fm : F, s);
-  const double one = intdiv::double_of((intdiv::bits_of(first ? F : Fm) & kSignBit) | ONE);
-  a = (mul_pow2(first ? one : q, l, k) - mul_pow2(first ? q : one, lm, km)) * s;
-  if (mag_bits(a) < intdiv::bits_of(s * REL_TOL)) a = 0.0;
-  return a;
+  const double q = mul(Num<double>::div(first ? Fm : F, s), first ? lm : l, first ? km : k);
+  const double one = intdiv::double_of((intdiv::bits_of(first ? F : Fm) & kSignBit) ^
+                                       intdiv::bits_of(first ? l : lm));
+  return flush_rel(((first ? one : q) - (first ? q : one)) * s, s);
+}
+// grids whose spacings are no powers of two (out of line: a kernel holds it once for its three
+// uses)
+static __device__ __noinline__ double scaled_difference_any(double F, double Fm, double l,
+                                                            double lm) {
+  return scaled_difference<false>(F, Fm, l, 0, lm, 0);
 }
 
 __device__ __forceinline__ double divergence_fp64(double Fi, double Fim, double Fj, double Fjm,
                                                   const Geom& G, const Rcp<double>& vol) {
   const double NEAR0 = 5.0 * Num<double>::tiny;  // near_zero, flux_solver.f90:461-474
-  double s = scaled_difference(Fi, Fim, G.l2, G.k2, G.l4, G.k4) +
-             scaled_difference(Fj, Fjm, G.l3, G.k3, G.l1, G.k1);
+  const bool pi = G.k2 != kNotPow2 && G.k4 != kNotPow2, pj = G.k3 != kNotPow2 && G.k1 != kNotPow2;
+  double s = (pi ? scaled_difference<true>(Fi, Fim, G.l2, G.k2, G.l4, G.k4)
+                 : scaled_difference_any(Fi, Fim, G.l2, G.l4)) +
+             (pj ? scaled_difference<true>(Fj, Fjm, G.l3, G.k3, G.l1, G.k1)
+                 : scaled_difference_any(Fj, Fjm, G.l3, G.l1));
   if (abs_lt(s, NEAR0)) s = 0.0;
-  return G.inv_vol != 0.0 ? mul_pow2(rneg(s), G.inv_vol, G.kinv) : div_by(rneg(s), vol);
+  return G.kinv != kNotPow2 ? mul_pow2(rneg(s), G.inv_vol, G.kinv) : div_by(rneg(s), vol);
 }
 
 }  // namespace cato

@@ -428,6 +428,9 @@ __device__ __forceinline__ void load_operands(const StageArgs& A, size_t cidx, d
   }
 }
 
+// (out of line, so that the compiler branches to it instead of adding under a predicate)
+static __device__ __noinline__ double add_source(double L, double q) { return L + q; }
+
 // FP64 and double-float: the divergence of variable k of a cell and its stage combine, from the
 // fluxes of the cell's right, left, upper and lower edge.
 template <typename R>
@@ -439,7 +442,7 @@ __device__ __forceinline__ double combine_var(const StageArgs& A, const ColumnCo
   double r;
   if constexpr (Prec<R>::kind == 0) {
     double L = divergence_fp64(Fi, Fim, Fj, Fjm, cg, vol);
-    if (k == 3 && A.src_q) L = L + A.src_q[cidx];
+    if (k == 3 && A.src_q) L = add_source(L, A.src_q[cidx]);
     if (A.kind == 2) {
       r = L;
     } else if (A.kind == 0) {
