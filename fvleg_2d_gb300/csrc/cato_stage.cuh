@@ -430,6 +430,9 @@ __device__ __forceinline__ void load_operands(const StageArgs& A, size_t cidx, d
 
 // (out of line, so that the compiler branches to it instead of adding under a predicate)
 static __device__ __noinline__ double add_source(double L, double q) { return L + q; }
+static __device__ __noinline__ double scaled_source(df L, double q, double c) {
+  return __dmul_rn(from_df(L) + q, c);
+}
 
 // FP64 and double-float: the divergence of variable k of a cell and its stage combine, from the
 // fluxes of the cell's right, left, upper and lower edge.
@@ -463,15 +466,16 @@ __device__ __forceinline__ double combine_var(const StageArgs& A, const ColumnCo
     const bool src = k == 3 && A.src_q;
     if (A.kind == 2) {
       r = from_df(Ld);
-      if (src) r = r + A.src_q[cidx];
+      if (src) r = add_source(r, A.src_q[cidx]);
     } else if (A.kind == 0) {
       double L = from_df(Ld);
-      if (src) L = L + A.src_q[cidx];
+      if (src) L = add_source(L, A.src_q[cidx]);
       r = ua + __dmul_rn(L, C.cc);
       if (abs_lt(r, Num<double>::eps)) r = 0.0;
     } else {
-      const double d = src ? __dmul_rn(from_df(Ld) + A.src_q[cidx], C.cc)
-                           : from_df(Ld * C.cc_df);
+      double d;
+      if (src) d = scaled_source(Ld, A.src_q[cidx], C.cc);
+      else d = from_df(Ld * C.cc_df);
       r = fma(uk, A.b, fma(ua, A.a, d));
       if (abs_lt(r, Num<double>::eps)) r = 0.0;
     }
