@@ -26,7 +26,7 @@ namespace cato {
 // routines of cato_intdiv.cuh, and the hardware instruction for the operands they leave out
 // (zero, subnormal, infinite or NaN operands, quotients outside the normal range).  The hardware
 // forms are kept out of line so that the compiler branches to them instead of evaluating them
-// alongside.  div_rn and sqrt_rn are out of line too: one copy of each (~80 instructions) per
+// alongside.  div_rn and sqrt_rn are out of line too: one copy of each per
 // kernel instead of one per call site keeps the stage kernels inside the instruction cache
 // (+18 % FP64 cell-updates/s on the 4096^2 quadrant, +55 % on the serving mix, where five flux
 // kernels run side by side).
@@ -85,7 +85,7 @@ template <> struct Num<double> {
 };
 
 // A divisor of several quotients: div_by(a, Rcp(b)) is Num<R>::div(a, b).  FP64 shares the
-// divisor's reciprocal (a third of a division's ~120 instructions).
+// divisor's reciprocal (a third of a division).
 template <typename R> struct Rcp {
   R b;
   __device__ __forceinline__ explicit Rcp(R x) : b(x) {}
@@ -718,8 +718,8 @@ __device__ __forceinline__ double half_normal(double x) {
 // FP64 MLP edge values (out of line: one copy per kernel, as recon_tvd2_f64), the values of
 // recon_mlp<double, ORDER> bit for bit.  The limiter is phi = max(0, min(alpha r, alpha, beta)):
 // FP32 estimates of alpha and beta from the differences tell which of them decides, so that the
-// quotients of the other are left out (16 divisions per edge with all of them, each ~120
-// instructions; typically 3 to 6 remain: 1700 -> 900 instructions per edge).  Only what decides is
+// quotients of the other are left out (16 divisions per edge with all of them;
+// typically 3 to 6 remain: 1700 -> 900 instructions per edge when it came in).  Only what decides is
 // formed, in the reference's order; where the estimates are within 1e-3 of each other (100 times
 // their error) both are.  r >= 1 is |d0| >= |dq + S|, and alpha is clamped to [1, 2], where
 // alpha r and alpha / 2 are exact.
