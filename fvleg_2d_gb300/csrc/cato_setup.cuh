@@ -38,16 +38,18 @@ inline FluxConsts<double> flux_consts_of(const cato_config& c) {
 //
 // FP32 strips of 64 columns: as many rows per CTA (32 .. 1) as leave the GPU about full; a strip
 // of r rows pays for r + 1.5 of them, and more than 32 leave a long last wave (3000 x 2010 Roe:
-// 797 us a step at 32 rows, 1050 at 64 rows of 128 columns; 4096^2 HLLC 1314 and 1328). Best of 1
-// .. 64 rows: 64 x 48 and 200^2: 1 row, 300^2: 2 (25.3 us, 36.3 at 1), 512^2: 4, 1024^2: 16.
+// 772 us a step at 32 rows, 1022 at 64 rows of 128 columns; 4096^2 HLLC 1257 and 1279). Best of 1
+// .. 64 rows: 64 x 48 and 200^2: 1 row, 300^2: 1 or 2 (24.6 and 25.9 us, 32.5 at 4), 512^2: 4,
+// 1024^2: 16.
 //
 // Edge-parallel tiles (FP64, double-float).  While they leave SMs idle the chain of a block is the
 // time of the launch: 32 columns in the split form with a single block of 1 row (64 x 48 HLLC:
-// 55 us a step, 75 in the unsplit form) or 2 rows (128 x 100: 76 us, 86 unsplit at 4 rows; 200^2:
-// 166, 147 unsplit), then a single unsplit block of 4 (256^2: 225 us, 231 with 64 columns), from
-// two tiles per SM on 64 columns, blocks of 4 rows and as many blocks per CTA as leave about four
-// waves of the two resident CTAs (1024^2: 2094 us at 8 rows, 2144 at 32; 4096^2: 29.3 ms at 32
-// rows, 30.6 at 8).
+// 40 us a step, 54 in the unsplit form) or 2 rows (128 x 100: 59 us, 62 unsplit at 4 rows), then a
+// single unsplit block of 4 (200^2: 116 us, 149 with 64 columns).  From two tiles per SM on 64
+// columns, blocks of 4 rows and as many blocks per CTA as leave about four waves of the two resident
+// CTAs (1024^2: 1735 us at 8 rows, 1790 at 32; 4096^2: 24.0 ms at 32 rows, 25.3 at 8).  With two ghost
+// columns a side a little later (256^2: 170 us, 191 with 64 columns; Roe 239 and 251, double-float 69
+// and 78); with three, 32 columns lose more to the halo (SLAU + MLP5 357 and 344).
 constexpr int kSMs = 152;
 inline StageShape default_shape(int ni, int nj, int ng, int precision) {
   auto tiles = [&](int columns, int rows) {
@@ -59,7 +61,7 @@ inline StageShape default_shape(int ni, int nj, int ng, int precision) {
     s.threads = 64;
     s.rows = 32;
     while (s.rows > 2 && tiles(64, s.rows) < 7LL * kSMs) s.rows /= 2;
-    if (tiles(64, 2) < 3LL * kSMs) s.rows = 1;  // 200^2: 20.8 us a step, 23.3 at 2 rows
+    if (tiles(64, 2) < 3LL * kSMs) s.rows = 1;  // 200^2: 20.4 us a step, 23.0 at 2 rows
     s.width = s.threads;
     return s;
   }
@@ -77,7 +79,7 @@ inline StageShape default_shape(int ni, int nj, int ng, int precision) {
   }
   s.warps = 9;
   s.rows = s.block = 4;
-  if (tiles(64, 4) < 2LL * kSMs) return s;
+  if (tiles(64, 4) < (ng == 2 ? 7LL * kSMs / 3 : 2LL * kSMs)) return s;
   s.width = 128;
   s.threads = 64;
   s.block = 4;
