@@ -722,7 +722,9 @@ __device__ __forceinline__ double half_normal(double x) {
 // typically 3 to 6 remain: 1700 -> 900 instructions per edge when it came in).  Only what decides is
 // formed, in the reference's order; where the estimates are within 1e-3 of each other (100 times
 // their error) both are.  r >= 1 is |d0| >= |dq + S|, and alpha is clamped to [1, 2], where
-// alpha r and alpha / 2 are exact.
+// alpha r and alpha / 2 are exact.  The estimates leave out SMALL_NUM, which decides a quotient once
+// another is 1e30 times it: alpha = 2 max(1, r) (1 + (toth / (d0 / (dx + S) + S))) / (1 + town) is
+// unknown, and beta = (-2 / (dq / (X + S) + S) + ...) / 30 anywhere, from ratios of 1e24 on.
 template <int ORDER>
 static __device__ __noinline__ EdgePair recon_mlp_f64(double qm2, double qm1, double q0, double qp1,
                                                      double qp2, double qp3, double t0p,
@@ -779,10 +781,10 @@ static __device__ __noinline__ EdgePair recon_mlp_f64(double qm2, double qm1, do
     const float toth = __fdividef(s ? fn[0] : fn[1], s ? fe[0] : fe[1]);
     const float at = __fdividef(2.0f * fmaxf(1.0f, rf) * (1.0f + fmaxf(0.0f, toth * fx * if0)),
                                 1.0f + town);
-    const bool known = sure && at >= 0.0f;
+    const bool known = sure && at >= 0.0f && fabsf(toth * if0) < 1e24f && fabsf(fx * if0) < 1e24f;
     const float lo = known ? fmaxf(1.0f, fminf(2.0f, at * 0.999f)) : 1.0f;
     const float hi = known ? fmaxf(1.0f, fminf(2.0f, at * 1.001f)) : 2.0f;
-    const float db = 1e-3f * bm;
+    const float db = ORDER == 5 && fabsf(fy * ifq) >= 1e24f ? INFINITY : 1e-3f * bm;
     if (b + db < 0.0f) {  // beta < 0: phi = 0
       t[s] = intdiv::double_of(intdiv::bits_of(dq) & kSignBit);
       continue;

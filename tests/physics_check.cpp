@@ -1,0 +1,134 @@
+// Host check of the FP64 stage arithmetic (cato_physics.cuh): the same source as the device code,
+// compiled for the host with the device intrinsics spelled out below.  Each family compares a
+// routine that leaves work out, or does it on the integer pipe, with the general form it stands
+// for, bit for bit (any NaN equals any NaN).
+//
+// usage: physics_check <cases per family and range>
+// Prints one line per family ("<family> tested <n> bad <n>") and exits 1 on any mismatch.
+#include <cfloat>
+#include <cmath>
+#include <cstdint>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <random>
+#include <type_traits>
+
+#include <cuda_runtime.h>
+
+// the runtime header's host spelling of the qualifiers
+#undef __noinline__
+#define __noinline__ __attribute__((__noinline__))
+#undef __forceinline__
+#define __forceinline__ inline
+
+using std::isfinite;
+using std::isnan;
+using std::max;
+using std::min;
+using std::signbit;
+
+template <typename T, typename U> static T bit_cast(U u) {
+  static_assert(sizeof(T) == sizeof(U), "");
+  T t;
+  std::memcpy(&t, &u, sizeof t);
+  return t;
+}
+static inline double __longlong_as_double(long long x) { return bit_cast<double>(x); }
+static inline long long __double_as_longlong(double x) { return bit_cast<long long>(x); }
+static inline float __uint_as_float(unsigned x) { return bit_cast<float>(x); }
+static inline unsigned __float_as_uint(float x) { return bit_cast<unsigned>(x); }
+static inline int __double2hiint(double x) { return (int)(bit_cast<uint64_t>(x) >> 32); }
+static inline int __double2loint(double x) { return (int)(uint32_t)bit_cast<uint64_t>(x); }
+static inline double __hiloint2double(int h, int l) {
+  return bit_cast<double>(((uint64_t)(uint32_t)h << 32) | (uint32_t)l);
+}
+static inline unsigned __funnelshift_l(unsigned lo, unsigned hi, unsigned s) {
+  return (unsigned)(((((uint64_t)hi << 32) | lo) << (s & 31)) >> 32);
+}
+static inline double __dadd_rn(double a, double b) { return a + b; }
+static inline double __dsub_rn(double a, double b) { return a - b; }
+static inline double __dmul_rn(double a, double b) { return a * b; }
+static inline float __fadd_rn(float a, float b) { return a + b; }
+static inline float __fsub_rn(float a, float b) { return a - b; }
+static inline float __fmul_rn(float a, float b) { return a * b; }
+static inline float __fdiv_rn(float a, float b) { return a / b; }
+static inline float __fdividef(float a, float b) { return a / b; }
+static inline float __fmaf_rn(float a, float b, float c) { return fmaf(a, b, c); }
+static inline float __int2float_rn(int a) { return (float)a; }
+static inline float rsqrtf(float a) { return (float)(1.0 / std::sqrt((double)a)); }
+
+#include "../fvleg_2d_gb300/csrc/cato_physics.cuh"
+
+using namespace cato;
+
+static std::mt19937_64 rng(20261205);
+static unsigned long long tested, bad;
+static int fail = 0;
+
+static double unit() { return (double)(rng() >> 11) * 0x1p-53; }
+// +-2^e for e in [lo, hi], one in four a power of two
+static double any_of(double lo, double hi) {
+  double e = lo + unit() * (hi - lo);
+  if (rng() % 4 == 0) e = std::floor(e);
+  const double m = std::exp2(e);
+  return (rng() & 1) ? m : -m;
+}
+static const double kSpecial[] = {0.0,     -0.0,    1.0,     -1.0,     INFINITY, -INFINITY, NAN,
+                                  DBL_MAX, -DBL_MAX, DBL_MIN, 4.9e-324, 1e-16,    -1e-16,    1e-30,
+                                  1e30,    2.220446049250313e-16};
+static double special() { return kSpecial[rng() % (sizeof kSpecial / sizeof *kSpecial)]; }
+
+static bool same(double a, double b) {
+  return (isnan(a) && isnan(b)) || bit_cast<uint64_t>(a) == bit_cast<uint64_t>(b);
+}
+static void report(const char* family) {
+  printf("%s tested %llu bad %llu\n", family, tested, bad);
+  fail |= bad != 0;
+  tested = bad = 0;
+}
+
+// ranges of the reconstruction families: magnitudes 2^lo .. 2^hi; kind 0 values, 1 relative
+// differences around a base value, 2 values and zeros, 3 values and special values
+static const struct {
+  int kind, lo, hi;
+} kRanges[] = {{0, -4, 4},    {1, -50, -1}, {0, -30, 30},  {2, -20, 20},   {2, -52, 30},
+               {0, -52, 58}, {2, -52, 58}, {0, -100, 100}, {3, -52, 58}, {2, -56, 2}};
+template <int N> static void stencil(int kind, int lo, int hi, double (&q)[N]) {
+  const double base = any_of(-3, 3);
+  for (double& x : q) {
+    if (kind == 1) x = base * (1.0 + any_of(lo, hi));
+    else if (kind == 2 && rng() % 3 == 0) x = (rng() & 1) ? 0.0 : -0.0;
+    else if (kind == 3 && rng() % 2 == 0) x = special();
+    else x = any_of(lo, hi);
+  }
+}
+
+// the MLP edge values that leave out what cannot decide, against all of the limiter's terms
+template <int ORDER> static void check_mlp(long n) {
+  for (const auto& r : kRanges)
+    for (long i = 0; i < n; ++i) {
+      double q[10];
+      stencil(r.kind, r.lo, r.hi, q);
+      const EdgePair a = recon_mlp_f64<ORDER>(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7], q[8],
+                                              q[9]);
+      const EdgePair b = recon_mlp_any<ORDER>(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7], q[8],
+                                              q[9]);
+      ++tested;
+      if (same(a.L, b.L) && same(a.R, b.R)) continue;
+      if (bad++ < 3) {
+        printf("mlp%d", ORDER);
+        for (double x : q) printf(" %.17g", x);
+        printf(": %.17g %.17g, general form %.17g %.17g\n", a.L, a.R, b.L, b.R);
+      }
+    }
+}
+
+int main(int argc, char** argv) {
+  const long n = argc > 1 ? atol(argv[1]) : 400000;
+  check_mlp<3>(n);
+  report("mlp3");
+  check_mlp<5>(n);
+  report("mlp5");
+  return fail;
+}
