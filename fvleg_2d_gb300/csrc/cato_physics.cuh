@@ -1496,7 +1496,8 @@ __device__ __forceinline__ void flux_slau(const FluxConsts<R>& K, const Prim<R>&
 // One pair of the Roe pressure sensor, |b - a| / (min(b, a) + 1e-16) >= 1 (or NaN).  With
 // 0 < min <= max < 2 min the difference is below min, so the quotient is below 1 (FP64: the
 // difference is exact by Sterbenz's lemma and the rounded quotient of x < y is below 1; the
-// other types keep a margin for their rounding): five divisions per edge are left out.
+// other types keep a margin for their rounding, max < 1.99 min): five divisions per edge are left
+// out.
 template <typename R> __device__ __forceinline__ bool roe_sensor_slow(R a, R b) {
   const R ratio = Num<R>::div(rabs(b - a), rmin(b, a) + R(1e-16));
   return !lt(ratio, R(1));
@@ -1513,13 +1514,13 @@ template <> __device__ __forceinline__ bool roe_sensor<double>(double a, double 
   return roe_sensor_f64(a, b);
 }
 template <> __device__ __forceinline__ bool roe_sensor<float>(float a, float b) {
-  const float lo = fminf(a, b), hi = fmaxf(a, b);
-  if (lo > 1e-25f && hi < 1.99f * lo) return false;
+  const float lo = fminf(a, b);  // (the number if the other is a NaN, which the sum keeps)
+  if (lo > 1e-25f && a + b < 2.99f * lo) return false;
   return roe_sensor_slow<float>(a, b);
 }
 template <> __device__ __forceinline__ bool roe_sensor<df>(df a, df b) {
-  const float lo = fminf(a.hi, b.hi), hi = fmaxf(a.hi, b.hi);
-  if (lo > 1e-25f && hi < 1.99f * lo) return false;
+  const float lo = fminf(a.hi, b.hi);
+  if (lo > 1e-25f && a.hi + b.hi < 2.99f * lo) return false;
   return roe_sensor_slow<df>(a, b);
 }
 // half(s) - x; FP32 as one FMA of the halved sum

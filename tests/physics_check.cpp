@@ -1,4 +1,4 @@
-// Host check of the FP64 stage arithmetic (cato_physics.cuh): the same source as the device code,
+// Host check of the stage arithmetic (cato_physics.cuh): the same source as the device code,
 // compiled for the host with the device intrinsics spelled out below.  Each family compares a
 // routine that leaves work out, or does it on the integer pipe, with the general form it stands
 // for, bit for bit (any NaN equals any NaN).
@@ -124,11 +124,29 @@ template <int ORDER> static void check_mlp(long n) {
     }
 }
 
+// the Roe pressure sensor that divides only where the pressures are far apart, in every type
+static void check_roe_sensor(long n) {
+  for (const auto& r : kRanges)
+    for (long i = 0; i < n; ++i) {
+      double q[2];
+      stencil(r.kind, std::max(r.lo, -60), std::min(r.hi, 60), q);
+      if (r.kind == 1) q[1] = std::copysign(q[1], q[0]);
+      const float f[2] = {(float)q[0], (float)q[1]};
+      ++tested;
+      const bool ok = roe_sensor<double>(q[0], q[1]) == roe_sensor_slow<double>(q[0], q[1]) &&
+                      roe_sensor<float>(f[0], f[1]) == roe_sensor_slow<float>(f[0], f[1]) &&
+                      roe_sensor<df>(df(q[0]), df(q[1])) == roe_sensor_slow<df>(df(q[0]), df(q[1]));
+      if (!ok && bad++ < 3) printf("roe_sensor %.17g %.17g\n", q[0], q[1]);
+    }
+}
+
 int main(int argc, char** argv) {
   const long n = argc > 1 ? atol(argv[1]) : 400000;
   check_mlp<3>(n);
   report("mlp3");
   check_mlp<5>(n);
   report("mlp5");
+  check_roe_sensor(n);
+  report("roe_sensor");
   return fail;
 }

@@ -1,4 +1,4 @@
-"""The FP64 stage arithmetic (fvleg_2d_gb300/csrc/cato_physics.cuh) compiled for the host with g++:
+"""The stage arithmetic (fvleg_2d_gb300/csrc/cato_physics.cuh) compiled for the host with g++:
 the routines that leave work out against the general forms they stand for, bit for bit, over
 ordinary and extreme values (tests/physics_check.cpp)."""
 import os
@@ -30,7 +30,7 @@ def families(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("family", ["mlp3", "mlp5"])
+@pytest.mark.parametrize("family", ["mlp3", "mlp5", "roe_sensor"])
 def test_bit_identical_to_the_general_form(families, family):
     tested, bad, log = families[family]
     assert tested >= 1_000_000 and bad == 0, log
