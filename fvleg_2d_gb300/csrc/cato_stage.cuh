@@ -317,7 +317,7 @@ __device__ __forceinline__ void load_src(const StageArgs& A, int sx, int row, Ro
   const size_t idx = (size_t)sy * A.pitch + sx;
   const double* const* src = A.Pin[0] ? A.Pin : A.Uk;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) s.c[k] = __ldg(src[k] + idx);
+  for (int k = 0; k < 4; ++k) s.c[k] = load_global(src[k] + idx);
 }
 
 template <typename R> __device__ __forceinline__ R from_double(double x);
@@ -424,7 +424,7 @@ __device__ __forceinline__ void load_operands(const StageArgs& A, size_t cidx, d
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     ua[k] = A.Ua[k] ? A.Ua[k][cidx] : 0.0;  // may alias Uo: plain load, read before write
-    uk[k] = (A.kind == 1) ? __ldg(A.Uk[k] + cidx) : 0.0;
+    uk[k] = (A.kind == 1) ? load_global(A.Uk[k] + cidx) : 0.0;
   }
 }
 
@@ -986,7 +986,7 @@ __device__ __forceinline__ void edge_tile(const StageArgs& A, const FluxConsts<R
       const Geom cg = cell_geom(A.G, gx, j);
       if constexpr (Prec<R>::kind == 2) C.set_row(A, j);
       const double ua = A.Ua[k] ? A.Ua[k][cidx] : 0.0;
-      const double uk = A.kind == 1 ? __ldg(A.Uk[k] + cidx) : 0.0;
+      const double uk = A.kind == 1 ? load_global(A.Uk[k] + cidx) : 0.0;
       const R* fj = sfy + ((j - y0 + 1) % (RW + 1) * 4 + k) * T + t;
       const R* fjm = sfy + ((j - y0) % (RW + 1) * 4 + k) * T + t;
       const double u = combine_var<R>(A, C, cg, Rcp<double>(cg.vol, cg.vol_y62), k, cidx, ua, uk,
