@@ -25,10 +25,13 @@ struct StepCtl {
 // Programmatic dependent launch: a kernel of a step is set up while its predecessor drains and
 // waits here, before its first access to memory, until the predecessor's results are complete.
 // Its blocks start when all of the predecessor's have passed launch_next or ended.  The FP32
-// kernels call it at the end of their march; the edge-parallel kernels do not: blocks that start
-// while others still run are placed unevenly, and a grid of about one block per SM then has two on
-// some (FP64 400 x 40: 54.0 us a step without the call, 62.3 with it, 62.0 with plain launches;
-// FP32 64 x 48: 17.9 us with it, 28.7 with plain launches).  No-ops in a plain launch.
+// kernel of a single grid calls it after its tile; the edge-parallel kernels do not: blocks that
+// start while others still run are placed unevenly, and a grid of about one block per SM then has
+// two on some (FP64 400 x 40: 54.0 us a step without the call, 62.3 with it, 62.0 with plain
+// launches; FP32 64 x 48: 17.9 us with it, 28.7 with plain launches).  Nor do the persistent batch
+// kernels: from within a tile the call would let the next stage's blocks wait on the SMs while the
+// queue still has items (served mix 131.0 us a step without it, 130.6 with it after the first
+// tile).  No-ops in a plain launch.
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void launch_next() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -685,7 +685,6 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, const FluxConsts<
       update_cell<EXT>(A, K, C, gx, j, cidx, ua, uk, Fi, Fim, Fj, Fjm);
     }
   }
-  launch_next();
   reduce_column(A, C);
 }
 
@@ -866,7 +865,6 @@ __device__ __forceinline__ void stage_tile_tvd(const StageArgs& A, const FluxCon
       for (int k = 0; k < 4; ++k) Fb[k] = Ft[k];
     }
   }
-  launch_next();
   reduce_column(A, C);
 }
 
@@ -1053,6 +1051,7 @@ __global__ void __maxnreg__(f32_regs(FLUX, RECON))
   if (A.active && *A.active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   tile_of<NG, FLUX, RECON, EXT>(A, K, blockIdx.x, blockIdx.y, smem_raw);
+  launch_next();
 }
 
 // FP64 and double-float: the edge-parallel tile, with a register budget per kernel variant.

@@ -19,3 +19,12 @@ def test_overlapped_kernels_use_no_read_only_loads():
         code = _code(name)
         for word in ("__ldg", "ld.global.nc", "__restrict__", "ldcs("):
             assert word not in code, (name, word)
+
+
+def test_tiles_do_not_launch_the_next_kernel():
+    # a persistent kernel makes many tiles: the trigger belongs after its last one
+    for name in ("cato_stage.cuh", "cato_batch.cuh"):
+        code = _code(name)
+        for m in re.finditer(r"launch_next\(\)", code):
+            before = code[:m.start()]
+            assert before.rfind("__global__") > before.rfind("__device__"), (name, before[-300:])
