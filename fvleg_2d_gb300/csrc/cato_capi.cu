@@ -1225,27 +1225,14 @@ int cato_gpu_run_timed(cato_handle* h, int64_t n_steps, float* total_ms, float* 
   return status_code(h->ctl_host->status);
 }
 
-// The launch shape of a plan (CTA width incl. the halo, rows per CTA).  The edge-parallel kernels
-// take half the width in columns (32 .. 128) and march in blocks of up to 4 rows.
-static StageShape plan_of(const cato_handle* h, int threads, int rows, int variant) {
-  StageShape s;
-  s.variant = variant;
-  s.rows = rows;
-  s.width = s.threads = threads;
-  if (h->cfg.precision != CATO_MIXED) {
-    s.threads = threads / 64 * 32;
-    s.block = std::min(rows, s.threads > 64 ? 2 : 4);
-    s.warps = 2 * s.block + 1;
-  }
-  return s;
-}
-
 int cato_gpu_set_plan(cato_handle* h, int32_t threads, int32_t rows_per_cta) {
   if (!h) return CATO_ERR_ARG;
   if (threads < 64 || threads > 256 || threads % 32 != 0 || rows_per_cta < 1 ||
       threads - 2 * h->ng < 1)
     return fail(h, CATO_ERR_ARG, "invalid plan");
-  h->plan = plan_of(h, threads, rows_per_cta, h->plan.variant);
+  const int variant = h->plan.variant;
+  h->plan = plan_shape(h->ni, h->nj, h->ng, h->cfg.precision, threads, rows_per_cta);
+  h->plan.variant = variant;
   return CATO_OK;
 }
 
@@ -1277,9 +1264,8 @@ int cato_gpu_tune(cato_handle* h, int32_t steps, int32_t* steps_taken, float* be
   for (int v = 0; v < nvar; ++v) {
     for (int width : {p0.width, 256}) {
       for (int rows : {p0.rows, half_rows, quarter_rows}) {
-        StageShape q = p0;
+        StageShape q = plan_shape(h->ni, h->nj, h->ng, h->cfg.precision, width, rows);
         q.variant = v;
-        if (width != p0.width || rows != p0.rows) q = plan_of(h, width, rows, v);
         bool dup = false;
         for (const StageShape& x : cands)
           dup |= x.width == q.width && x.rows == q.rows && x.variant == q.variant;

@@ -7,6 +7,7 @@
 #include <atomic>
 
 #include "cato_batch.cuh"
+#include "cato_shape.h"
 #include "cato_stage.cuh"
 
 namespace cato {
@@ -24,17 +25,6 @@ inline int launch_device() {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -1;
   return dev;
 }
-
-// The shape of a single-grid launch: CTA columns incl. the x-halo, rows marched per CTA, and for
-// the edge-parallel kernels (FP64, double-float) the rows of a block and the register budget.
-struct StageShape {
-  int width = 128;  // the plan's CTA width, as the caller knows it
-  int threads = 128;
-  int rows = 64;
-  int block = 4;
-  int warps = 9;    // blockDim.y of the edge-parallel kernels, at least 2 block + 1
-  int variant = 0;
-};
 
 // Raises kernel's dynamic shared-memory limit once per device.
 template <typename F>

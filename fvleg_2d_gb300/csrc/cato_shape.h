@@ -1,0 +1,80 @@
+// cato_shape.h -- the launch shapes of the stage kernels as functions of the grid: the rules only, so
+// that a host test can read them without CUDA.
+#pragma once
+
+#include <algorithm>
+
+#include "../../include/cato_gpu.h"
+
+namespace cato {
+
+// The shape of a single-grid launch: CTA columns incl. the x-halo, rows marched per CTA, and for
+// the edge-parallel kernels (FP64, double-float) the rows of a block and the register budget.
+struct StageShape {
+  int width = 128;  // the plan's CTA width, as the caller knows it
+  int threads = 128;
+  int rows = 64;
+  int block = 4;
+  int warps = 9;    // blockDim.y of the edge-parallel kernels, at least 2 block + 1
+  int variant = 0;
+};
+
+// Default single-grid launch shape.
+//
+// FP32 strips of 64 columns: as many rows per CTA (32 .. 1) as leave the GPU about full; a strip
+// of r rows pays for r + 1.5 of them, and more than 32 leave a long last wave (3000 x 2010 Roe:
+// 772 us a step at 32 rows, 1022 at 64 rows of 128 columns; 4096^2 HLLC 1257 and 1279). Best of 1
+// .. 64 rows: 64 x 48 and 200^2: 1 row, 300^2: 1 or 2 (24.6 and 25.9 us, 32.5 at 4), 512^2: 4,
+// 1024^2: 16.
+//
+// Edge-parallel tiles (FP64, double-float).  While they leave SMs idle the chain of a block is the
+// time of the launch: 32 columns in the split form with a single block of 1 row (64 x 48 HLLC:
+// 40 us a step, 54 in the unsplit form) or 2 rows (128 x 100: 59 us, 62 unsplit at 4 rows), then a
+// single unsplit block of 4 (200^2: 116 us, 149 with 64 columns).  From two tiles per SM on 64
+// columns, blocks of 4 rows and as many blocks per CTA as leave about four waves of the two resident
+// CTAs (1024^2: 1735 us at 8 rows, 1790 at 32; 4096^2: 24.0 ms at 32 rows, 25.3 at 8).  With two ghost
+// columns a side a little later (256^2: 170 us, 191 with 64 columns; Roe 239 and 251, double-float 69
+// and 78); with three, 32 columns lose more to the halo (SLAU + MLP5 357 and 344).
+constexpr int kSMs = 152;
+inline long long tiles_of(int ni, int nj, int ng, int columns, int rows) {
+  const int W = columns - 2 * ng;
+  return (long long)((ni + W - 1) / W) * ((nj + rows - 1) / rows);
+}
+
+// The shape of a plan (CTA width incl. the halo, rows per CTA), as cato_gpu_set_plan takes it and
+// cato_gpu_get_plan gives it; every shape is one of these.  The edge-parallel kernels take half the width in columns (32 .. 128)
+// and march in blocks of up to 4 rows.
+inline StageShape plan_shape(int ni, int nj, int ng, int precision, int width, int rows) {
+  StageShape s;
+  s.rows = rows;
+  s.width = s.threads = width;
+  if (precision == CATO_MIXED) return s;
+  s.threads = width / 64 * 32;
+  s.block = std::min(rows, s.threads > 64 ? 2 : 4);
+  s.warps = 2 * s.block + 1;
+  // the split form, where a CTA is a single block of 1 or 2 rows and SMs stay idle
+  if (s.threads == 32 && rows == 1 && tiles_of(ni, nj, ng, 32, 1) <= kSMs) s.warps = 12;
+  if (s.threads == 32 && rows == 2 && tiles_of(ni, nj, ng, 32, 2) <= 2 * kSMs + 16) s.warps = 10;
+  return s;
+}
+
+inline StageShape default_shape(int ni, int nj, int ng, int precision) {
+  auto tiles = [&](int columns, int rows) { return tiles_of(ni, nj, ng, columns, rows); };
+  auto plan = [&](int width, int rows) { return plan_shape(ni, nj, ng, precision, width, rows); };
+  if (precision == CATO_MIXED) {
+    int rows = 32;
+    while (rows > 2 && tiles(64, rows) < 7LL * kSMs) rows /= 2;
+    if (tiles(64, 2) < 3LL * kSMs) rows = 1;  // 200^2: 20.4 us a step, 23.0 at 2 rows
+    return plan(64, rows);
+  }
+  for (int rows : {1, 2}) {
+    const StageShape s = plan(64, rows);
+    if (s.warps > 2 * s.block + 1) return s;
+  }
+  if (tiles(64, 4) < (ng == 2 ? 7LL * kSMs / 3 : 2LL * kSMs)) return plan(64, 4);
+  int rows = 32;
+  while (rows > 4 && tiles(64, rows) < 7LL * kSMs) rows /= 2;
+  return plan(128, rows);
+}
+
+}  // namespace cato

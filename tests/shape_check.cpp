@@ -1,0 +1,16 @@
+// The launch shape rules (cato_shape.h) as C functions for the tests.
+#include "../fvleg_2d_gb300/csrc/cato_shape.h"
+
+static void put(const cato::StageShape& s, int* out) {
+  const int v[6] = {s.width, s.threads, s.rows, s.block, s.warps, s.variant};
+  for (int k = 0; k < 6; ++k) out[k] = v[k];
+}
+
+extern "C" {
+void default_shape(int ni, int nj, int ng, int precision, int* out) {
+  put(cato::default_shape(ni, nj, ng, precision), out);
+}
+void plan_shape(int ni, int nj, int ng, int precision, int width, int rows, int* out) {
+  put(cato::plan_shape(ni, nj, ng, precision, width, rows), out);
+}
+}

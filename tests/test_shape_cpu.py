@@ -1,0 +1,47 @@
+"""The launch shape rules (fvleg_2d_gb300/csrc/cato_shape.h), compiled for the host."""
+import ctypes
+import os
+import random
+import shutil
+import subprocess
+from collections import namedtuple
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+FP64, MIXED, MIXED_DF = 0, 1, 2
+Shape = namedtuple("Shape", "width threads rows block warps variant")
+GRIDS = [(64, 48), (128, 100), (200, 200), (256, 256), (400, 40), (448, 40), (512, 512), (1024, 1024),
+         (4096, 4096), (3, 3), (5000, 3), (3, 5000), (100, 2000)]
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("g++ not available")
+    so = str(tmp_path_factory.mktemp("shape") / "libshape.so")
+    subprocess.run([gxx, "-O1", "-std=c++17", "-shared", "-fPIC",
+                    os.path.join(HERE, "shape_check.cpp"), "-o", so], check=True)
+    return ctypes.CDLL(so)
+
+
+def _call(fn, *args):
+    out = (ctypes.c_int * 6)()
+    fn(*args, out)
+    return Shape(*out)
+
+
+def _grids():
+    rng = random.Random(3)
+    return GRIDS + [(int(2 ** rng.uniform(1.6, 13)), int(2 ** rng.uniform(1.6, 13)))
+                    for _ in range(300)]
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED, MIXED_DF])
+@pytest.mark.parametrize("ng", [2, 3])
+def test_a_plan_survives_get_and_set(rules, precision, ng):
+    for ni, nj in _grids():
+        d = _call(rules.default_shape, ni, nj, ng, precision)
+        p = _call(rules.plan_shape, ni, nj, ng, precision, d.width, d.rows)
+        assert p == d, (ni, nj)
