@@ -105,11 +105,11 @@ cudaError_t launch_stage_one(const StageShape& s, bool warm, cudaStream_t stream
     }
     return launch_strip<NG, FLUX, RECON, true>(s, warm, stream, A, K);
   } else {
-    const bool split = EdgeShape{s.threads, s.block, s.warps}.split();
+    const StageForm form = stage_form(s, Prec<R>::kind == 0 ? CATO_FP64 : CATO_MIXED_DF);
     if (warm) {
       cudaError_t e = launch_edge<R, NG, FLUX, RECON, edge_regs(0), true>(s, true, stream, A, K);
       if (e != cudaSuccess) return e;
-    } else if (split && s.variant == 0) {
+    } else if (form.split) {
       return launch_edge<R, NG, FLUX, RECON, edge_regs(0), true>(s, false, stream, A, K);
     }
     if constexpr (Prec<R>::kind == 0) {
@@ -118,9 +118,9 @@ cudaError_t launch_stage_one(const StageShape& s, bool warm, cudaStream_t stream
         if (e == cudaSuccess)
           e = launch_edge<R, NG, FLUX, RECON, edge_regs(2)>(s, true, stream, A, K);
         if (e != cudaSuccess) return e;
-      } else if (s.variant == 1) {
+      } else if (form.variant == 1) {
         return launch_edge<R, NG, FLUX, RECON, edge_regs(1)>(s, false, stream, A, K);
-      } else if (s.variant == 2) {
+      } else if (form.variant == 2) {
         return launch_edge<R, NG, FLUX, RECON, edge_regs(2)>(s, false, stream, A, K);
       }
     }

@@ -19,6 +19,17 @@ struct StageShape {
   int variant = 0;
 };
 
+// The kernel of a shape: the FP64 register budget (the other types have one kernel, whatever budget
+// was set) and the split form, which FP64 has at the default budget only.
+struct StageForm {
+  int variant;
+  bool split;
+};
+inline StageForm stage_form(const StageShape& s, int precision) {
+  const int variant = precision == CATO_FP64 ? s.variant : 0;
+  return {variant, precision != CATO_MIXED && variant == 0 && s.warps > 2 * s.block + 1};
+}
+
 // Default single-grid launch shape.
 //
 // FP32 strips of 64 columns: as many rows per CTA (32 .. 1) as leave the GPU about full; a strip

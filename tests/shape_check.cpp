@@ -10,6 +10,15 @@ extern "C" {
 void default_shape(int ni, int nj, int ng, int precision, int* out) {
   put(cato::default_shape(ni, nj, ng, precision), out);
 }
+// the register budget the kernel is launched with, and whether it is the split one
+void launched_form(int ni, int nj, int ng, int precision, int width, int rows, int variant,
+                   int* out) {
+  cato::StageShape s = cato::plan_shape(ni, nj, ng, precision, width, rows);
+  s.variant = variant;
+  const cato::StageForm f = cato::stage_form(s, precision);
+  out[0] = f.variant;
+  out[1] = f.split;
+}
 void plan_shape(int ni, int nj, int ng, int precision, int width, int rows, int* out) {
   put(cato::plan_shape(ni, nj, ng, precision, width, rows), out);
 }

@@ -45,3 +45,21 @@ def test_a_plan_survives_get_and_set(rules, precision, ng):
         d = _call(rules.default_shape, ni, nj, ng, precision)
         p = _call(rules.plan_shape, ni, nj, ng, precision, d.width, d.rows)
         assert p == d, (ni, nj)
+
+
+def test_the_register_budget_is_ignored_outside_fp64(rules):
+    for ni, nj in GRIDS:
+        for precision in (FP64, MIXED, MIXED_DF):
+            d = _call(rules.default_shape, ni, nj, 2, precision)
+            forms = [_call2(rules.launched_form, ni, nj, 2, precision, d.width, d.rows, v)
+                     for v in (0, 1, 2)]
+            if precision == FP64:
+                assert [v for v, _ in forms] == [0, 1, 2]
+            else:
+                assert forms[0] == forms[1] == forms[2] and forms[0][0] == 0, (ni, nj)
+
+
+def _call2(fn, *args):
+    out = (ctypes.c_int * 2)()
+    fn(*args, out)
+    return tuple(out)
