@@ -72,11 +72,16 @@ inline StageShape plan_shape(int ni, int nj, int ng, int precision, int width, i
 inline StageShape default_shape(int ni, int nj, int ng, int precision) {
   auto tiles = [&](int columns, int rows) { return tiles_of(ni, nj, ng, columns, rows); };
   auto plan = [&](int width, int rows) { return plan_shape(ni, nj, ng, precision, width, rows); };
+  // a launch has at most 65535 tiles along j: taller grids (2 M rows at 32) take taller tiles
+  auto fit = [&](int rows) {
+    while ((nj + rows - 1) / rows > 65535) rows *= 2;
+    return rows;
+  };
   if (precision == CATO_MIXED) {
     int rows = 32;
     while (rows > 2 && tiles(64, rows) < 7LL * kSMs) rows /= 2;
     if (tiles(64, 2) < 3LL * kSMs) rows = 1;  // 200^2: 20.4 us a step, 23.0 at 2 rows
-    return plan(64, rows);
+    return plan(64, fit(rows));
   }
   for (int rows : {1, 2}) {
     const StageShape s = plan(64, rows);
@@ -85,7 +90,7 @@ inline StageShape default_shape(int ni, int nj, int ng, int precision) {
   if (tiles(64, 4) < (ng == 2 ? 7LL * kSMs / 3 : 2LL * kSMs)) return plan(64, 4);
   int rows = 32;
   while (rows > 4 && tiles(64, rows) < 7LL * kSMs) rows /= 2;
-  return plan(128, rows);
+  return plan(128, fit(rows));
 }
 
 }  // namespace cato

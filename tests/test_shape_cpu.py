@@ -63,3 +63,10 @@ def _call2(fn, *args):
     out = (ctypes.c_int * 2)()
     fn(*args, out)
     return tuple(out)
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED, MIXED_DF])
+@pytest.mark.parametrize("ni,nj", [(2, 2_097_121), (3, 4_194_240), (64, 2_100_000), (3, 1 << 30)])
+def test_tall_grids_fit_the_launch_limit(rules, precision, ni, nj):
+    d = _call(rules.default_shape, ni, nj, 2, precision)
+    assert -(-nj // d.rows) <= 65535, d
