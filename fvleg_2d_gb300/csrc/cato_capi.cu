@@ -1254,25 +1254,8 @@ int cato_gpu_tune(cato_handle* h, int32_t steps, int32_t* steps_taken, float* be
   if (steps_taken) *steps_taken = 0;
   if (!h->uploaded) return fail(h, CATO_ERR_STATE, "no state uploaded");
   if (h->exchange) return refuse_exchange(h, "cato_gpu_tune");
-  // candidates: the current plan and the widest one, each with the current, half and a quarter of
-  // the rows per CTA (down to 8), and with every FP64 register budget
   const StageShape p0 = h->plan;
-  std::vector<StageShape> cands;
-  const int half_rows = p0.rows <= 8 ? p0.rows : std::max(8, p0.rows / 2);
-  const int quarter_rows = p0.rows <= 8 ? p0.rows : std::max(8, p0.rows / 4);
-  const int nvar = h->cfg.precision == CATO_FP64 ? 3 : 1;
-  for (int v = 0; v < nvar; ++v) {
-    for (int width : {p0.width, 256}) {
-      for (int rows : {p0.rows, half_rows, quarter_rows}) {
-        StageShape q = plan_shape(h->ni, h->nj, h->ng, h->cfg.precision, width, rows);
-        q.variant = v;
-        bool dup = false;
-        for (const StageShape& x : cands)
-          dup |= x.width == q.width && x.rows == q.rows && x.variant == q.variant;
-        if (!dup && q.width - 2 * h->ng <= h->ni + 2 * h->ng) cands.push_back(q);
-      }
-    }
-  }
+  const std::vector<StageShape> cands = tune_shapes(h->ni, h->nj, h->ng, h->cfg.precision, p0);
   StageShape best = p0;
   float best_t = INFINITY;
   int taken = 0;

@@ -3,6 +3,7 @@
 #pragma once
 
 #include <algorithm>
+#include <vector>
 
 #include "../../include/cato_gpu.h"
 
@@ -91,6 +92,33 @@ inline StageShape default_shape(int ni, int nj, int ng, int precision) {
   int rows = 32;
   while (rows > 4 && tiles(64, rows) < 7LL * kSMs) rows /= 2;
   return plan(128, fit(rows));
+}
+
+// The candidates of a tuning run: the current plan and the widest one, each with the current, half
+// and a quarter of the rows per CTA (down to 8), and with every FP64 register budget; none wider
+// than the grid with its halo.
+inline std::vector<StageShape> tune_shapes(int ni, int nj, int ng, int precision,
+                                           const StageShape& current) {
+  std::vector<StageShape> out;
+  const int r = current.rows;
+  const int half_rows = r <= 8 ? r : std::max(8, r / 2);
+  const int quarter_rows = r <= 8 ? r : std::max(8, r / 4);
+  const int nvar = precision == CATO_FP64 ? 3 : 1;
+  for (int v = 0; v < nvar; ++v) {
+    for (int width : {current.width, 256}) {
+      for (int rows : {r, half_rows, quarter_rows}) {
+        StageShape q = plan_shape(ni, nj, ng, precision, width, rows);
+        q.variant = v;
+        bool dup = false;
+        for (const StageShape& x : out)
+          dup |= x.width == q.width && x.rows == q.rows && x.variant == q.variant;
+        // (the current plan by its columns: a width of 128 is 64 columns in FP64)
+        const int span = width == current.width ? q.threads : width;
+        if (!dup && span - 2 * ng <= ni + 2 * ng) out.push_back(q);
+      }
+    }
+  }
+  return out;
 }
 
 }  // namespace cato

@@ -22,4 +22,13 @@ void launched_form(int ni, int nj, int ng, int precision, int width, int rows, i
 void plan_shape(int ni, int nj, int ng, int precision, int width, int rows, int* out) {
   put(cato::plan_shape(ni, nj, ng, precision, width, rows), out);
 }
+int tune_shapes(int ni, int nj, int ng, int precision, int width, int rows, int* out) {
+  const auto c = cato::tune_shapes(
+      ni, nj, ng, precision, cato::plan_shape(ni, nj, ng, precision, width, rows));
+  for (const auto& s : c) {
+    put(s, out);
+    out += 6;
+  }
+  return (int)c.size();
+}
 }

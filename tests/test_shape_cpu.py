@@ -70,3 +70,19 @@ def _call2(fn, *args):
 def test_tall_grids_fit_the_launch_limit(rules, precision, ni, nj):
     d = _call(rules.default_shape, ni, nj, 2, precision)
     assert -(-nj // d.rows) <= 65535, d
+
+
+def _tune(rules, ni, nj, ng, precision, width, rows):
+    out = (ctypes.c_int * 512)()
+    n = rules.tune_shapes(ni, nj, ng, precision, width, rows, out)
+    return [Shape(*out[6 * k:6 * k + 6]) for k in range(n)]
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED, MIXED_DF])
+@pytest.mark.parametrize("ni,nj", [(60, 5000), (100, 2000), (119, 900), (96, 104), (700, 500)])
+def test_the_default_plan_is_a_tuning_candidate(rules, precision, ni, nj):
+    d = _call(rules.default_shape, ni, nj, 2, precision)
+    shapes = _tune(rules, ni, nj, 2, precision, d.width, d.rows)
+    assert d in shapes
+    assert {s.variant for s in shapes} == ({0, 1, 2} if precision == FP64 else {0})
+    assert len(set(shapes)) == len(shapes)
