@@ -86,6 +86,7 @@ struct cato_handle {
   double* src_field = nullptr;
   int* src_dep = nullptr;
   int src_parity = 0;
+  int sms = 0;  // of the device the handle was made on
   StageShape plan;
   FluxConsts<double> K64{};
   FluxConsts<float> K32{};
@@ -159,7 +160,8 @@ static void fill_consts(cato_handle* h) {
 }
 
 static void default_plan(cato_handle* h) {
-  h->plan = default_shape(h->ni, h->nj, h->ng, h->cfg.precision);
+  h->sms = sm_count();
+  h->plan = default_shape(h->sms, h->ni, h->nj, h->ng, h->cfg.precision);
 }
 
 static StageArgs base_args(cato_handle* h) {
@@ -1231,7 +1233,7 @@ int cato_gpu_set_plan(cato_handle* h, int32_t threads, int32_t rows_per_cta) {
       threads - 2 * h->ng < 1)
     return fail(h, CATO_ERR_ARG, "invalid plan");
   const int variant = h->plan.variant;
-  h->plan = plan_shape(h->ni, h->nj, h->ng, h->cfg.precision, threads, rows_per_cta);
+  h->plan = plan_shape(h->sms, h->ni, h->nj, h->ng, h->cfg.precision, threads, rows_per_cta);
   h->plan.variant = variant;
   return CATO_OK;
 }
@@ -1255,7 +1257,8 @@ int cato_gpu_tune(cato_handle* h, int32_t steps, int32_t* steps_taken, float* be
   if (!h->uploaded) return fail(h, CATO_ERR_STATE, "no state uploaded");
   if (h->exchange) return refuse_exchange(h, "cato_gpu_tune");
   const StageShape p0 = h->plan;
-  const std::vector<StageShape> cands = tune_shapes(h->ni, h->nj, h->ng, h->cfg.precision, p0);
+  const std::vector<StageShape> cands =
+      tune_shapes(h->sms, h->ni, h->nj, h->ng, h->cfg.precision, p0);
   StageShape best = p0;
   float best_t = INFINITY;
   int taken = 0;

@@ -26,6 +26,15 @@ inline int launch_device() {
   return dev;
 }
 
+// SMs of the current device (1 when it cannot be read)
+inline int sm_count() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    (void)cudaGetLastError();
+  return n > 0 ? n : 1;
+}
+
 // Raises kernel's dynamic shared-memory limit once per device.
 template <typename F>
 inline cudaError_t allow_smem(PerDevice& attr, int dev, F* kernel, size_t bytes) {

@@ -118,7 +118,7 @@ extern "C" int cato_gpu_solve_noalloc(const cato_config* cfg, double* rho, doubl
   // flux constants, uniform geometry and launch shape: those a handle derives from cfg
   const FluxConsts<double> K = flux_consts_of(*cfg);
   const Geom G = uniform_geom(cfg->dx, cfg->dy);
-  const StageShape shape = default_shape(ni, nj, ng, cfg->precision);
+  const StageShape shape = default_shape(sm_count(), ni, nj, ng, cfg->precision);
 
   StageArgs A;
   std::memset(&A, 0, sizeof(A));

@@ -31,7 +31,30 @@ inline StageForm stage_form(const StageShape& s, int precision) {
   return {variant, precision != CATO_MIXED && variant == 0 && s.warps > 2 * s.block + 1};
 }
 
-// Default single-grid launch shape.
+// tiles of columns (incl. the halo) x rows
+inline long long tiles_of(int ni, int nj, int ng, int columns, int rows) {
+  const int W = columns - 2 * ng;
+  return (long long)((ni + W - 1) / W) * ((nj + rows - 1) / rows);
+}
+
+// The shape of a plan (CTA width incl. the halo, rows per CTA), as cato_gpu_set_plan takes it and
+// cato_gpu_get_plan gives it; every shape is one of these.  The edge-parallel kernels take half the
+// width in columns (32 .. 128) and march in blocks of up to 4 rows.
+inline StageShape plan_shape(int sms, int ni, int nj, int ng, int precision, int width, int rows) {
+  StageShape s;
+  s.rows = rows;
+  s.width = s.threads = width;
+  if (precision == CATO_MIXED) return s;
+  s.threads = width / 64 * 32;
+  s.block = std::min(rows, s.threads > 64 ? 2 : 4);
+  s.warps = 2 * s.block + 1;
+  // the split form, where a CTA is a single block of 1 or 2 rows and SMs stay idle
+  if (s.threads == 32 && rows == 1 && tiles_of(ni, nj, ng, 32, 1) <= sms) s.warps = 12;
+  if (s.threads == 32 && rows == 2 && tiles_of(ni, nj, ng, 32, 2) <= 2 * sms + 16) s.warps = 10;
+  return s;
+}
+
+// Default single-grid launch shape, for a GPU of sms SMs (measured on 152).
 //
 // FP32 strips of 64 columns: as many rows per CTA (32 .. 1) as leave the GPU about full; a strip
 // of r rows pays for r + 1.5 of them, and more than 32 leave a long last wave (3000 x 2010 Roe:
@@ -41,38 +64,19 @@ inline StageForm stage_form(const StageShape& s, int precision) {
 //
 // Edge-parallel tiles (FP64, double-float).  While they leave SMs idle the chain of a block is the
 // time of the launch: 32 columns in the split form with a single block of 1 row (64 x 48 HLLC:
-// 40 us a step, 54 in the unsplit form) or 2 rows (128 x 100: 59 us, 62 unsplit at 4 rows), then a
-// single unsplit block of 4 (200^2: 116 us, 149 with 64 columns).  From two tiles per SM on 64
+// 40 us a step, 54 in the unsplit form) or 2 rows (128 x 100: 59 us, 62 unsplit at 4 rows; a little
+// beyond two tiles per SM too, where 4 rows give a few SMs a second tile: 392 x 44 to 448 x 40, 308
+// to 320 tiles, HLLC 70 to 72 us, 77 to 79 at 4 rows, double-float 37 and 35), then a single
+// unsplit block of 4 (200^2: 116 us, 149 with 64 columns).  From two tiles per SM on 64
 // columns, blocks of 4 rows and as many blocks per CTA as leave about four waves of the two resident
 // CTAs (1024^2: 1735 us at 8 rows, 1790 at 32; 4096^2: 24.0 ms at 32 rows, 25.3 at 8).  With two ghost
 // columns a side a little later (256^2: 170 us, 191 with 64 columns; Roe 239 and 251, double-float 69
 // and 78); with three, 32 columns lose more to the halo (SLAU + MLP5 357 and 344).
-constexpr int kSMs = 152;
-inline long long tiles_of(int ni, int nj, int ng, int columns, int rows) {
-  const int W = columns - 2 * ng;
-  return (long long)((ni + W - 1) / W) * ((nj + rows - 1) / rows);
-}
-
-// The shape of a plan (CTA width incl. the halo, rows per CTA), as cato_gpu_set_plan takes it and
-// cato_gpu_get_plan gives it; every shape is one of these.  The edge-parallel kernels take half the width in columns (32 .. 128)
-// and march in blocks of up to 4 rows.
-inline StageShape plan_shape(int ni, int nj, int ng, int precision, int width, int rows) {
-  StageShape s;
-  s.rows = rows;
-  s.width = s.threads = width;
-  if (precision == CATO_MIXED) return s;
-  s.threads = width / 64 * 32;
-  s.block = std::min(rows, s.threads > 64 ? 2 : 4);
-  s.warps = 2 * s.block + 1;
-  // the split form, where a CTA is a single block of 1 or 2 rows and SMs stay idle
-  if (s.threads == 32 && rows == 1 && tiles_of(ni, nj, ng, 32, 1) <= kSMs) s.warps = 12;
-  if (s.threads == 32 && rows == 2 && tiles_of(ni, nj, ng, 32, 2) <= 2 * kSMs + 16) s.warps = 10;
-  return s;
-}
-
-inline StageShape default_shape(int ni, int nj, int ng, int precision) {
+inline StageShape default_shape(int sms, int ni, int nj, int ng, int precision) {
   auto tiles = [&](int columns, int rows) { return tiles_of(ni, nj, ng, columns, rows); };
-  auto plan = [&](int width, int rows) { return plan_shape(ni, nj, ng, precision, width, rows); };
+  auto plan = [&](int width, int rows) {
+    return plan_shape(sms, ni, nj, ng, precision, width, rows);
+  };
   // a launch has at most 65535 tiles along j: taller grids (2 M rows at 32) take taller tiles
   auto fit = [&](int rows) {
     while ((nj + rows - 1) / rows > 65535) rows *= 2;
@@ -80,24 +84,24 @@ inline StageShape default_shape(int ni, int nj, int ng, int precision) {
   };
   if (precision == CATO_MIXED) {
     int rows = 32;
-    while (rows > 2 && tiles(64, rows) < 7LL * kSMs) rows /= 2;
-    if (tiles(64, 2) < 3LL * kSMs) rows = 1;  // 200^2: 20.4 us a step, 23.0 at 2 rows
+    while (rows > 2 && tiles(64, rows) < 7LL * sms) rows /= 2;
+    if (tiles(64, 2) < 3LL * sms) rows = 1;  // 200^2: 20.4 us a step, 23.0 at 2 rows
     return plan(64, fit(rows));
   }
   for (int rows : {1, 2}) {
     const StageShape s = plan(64, rows);
     if (s.warps > 2 * s.block + 1) return s;
   }
-  if (tiles(64, 4) < (ng == 2 ? 7LL * kSMs / 3 : 2LL * kSMs)) return plan(64, 4);
+  if (tiles(64, 4) < (ng == 2 ? 7LL * sms / 3 : 2LL * sms)) return plan(64, 4);
   int rows = 32;
-  while (rows > 4 && tiles(64, rows) < 7LL * kSMs) rows /= 2;
+  while (rows > 4 && tiles(64, rows) < 7LL * sms) rows /= 2;
   return plan(128, fit(rows));
 }
 
 // The candidates of a tuning run: the current plan and the widest one, each with the current, half
 // and a quarter of the rows per CTA (down to 8), and with every FP64 register budget; none wider
 // than the grid with its halo.
-inline std::vector<StageShape> tune_shapes(int ni, int nj, int ng, int precision,
+inline std::vector<StageShape> tune_shapes(int sms, int ni, int nj, int ng, int precision,
                                            const StageShape& current) {
   std::vector<StageShape> out;
   const int r = current.rows;
@@ -107,7 +111,7 @@ inline std::vector<StageShape> tune_shapes(int ni, int nj, int ng, int precision
   for (int v = 0; v < nvar; ++v) {
     for (int width : {current.width, 256}) {
       for (int rows : {r, half_rows, quarter_rows}) {
-        StageShape q = plan_shape(ni, nj, ng, precision, width, rows);
+        StageShape q = plan_shape(sms, ni, nj, ng, precision, width, rows);
         q.variant = v;
         bool dup = false;
         for (const StageShape& x : out)

@@ -7,24 +7,24 @@ static void put(const cato::StageShape& s, int* out) {
 }
 
 extern "C" {
-void default_shape(int ni, int nj, int ng, int precision, int* out) {
-  put(cato::default_shape(ni, nj, ng, precision), out);
+void default_shape(int sms, int ni, int nj, int ng, int precision, int* out) {
+  put(cato::default_shape(sms, ni, nj, ng, precision), out);
 }
 // the register budget the kernel is launched with, and whether it is the split one
-void launched_form(int ni, int nj, int ng, int precision, int width, int rows, int variant,
+void launched_form(int sms, int ni, int nj, int ng, int precision, int width, int rows, int variant,
                    int* out) {
-  cato::StageShape s = cato::plan_shape(ni, nj, ng, precision, width, rows);
+  cato::StageShape s = cato::plan_shape(sms, ni, nj, ng, precision, width, rows);
   s.variant = variant;
   const cato::StageForm f = cato::stage_form(s, precision);
   out[0] = f.variant;
   out[1] = f.split;
 }
-void plan_shape(int ni, int nj, int ng, int precision, int width, int rows, int* out) {
-  put(cato::plan_shape(ni, nj, ng, precision, width, rows), out);
+void plan_shape(int sms, int ni, int nj, int ng, int precision, int width, int rows, int* out) {
+  put(cato::plan_shape(sms, ni, nj, ng, precision, width, rows), out);
 }
-int tune_shapes(int ni, int nj, int ng, int precision, int width, int rows, int* out) {
+int tune_shapes(int sms, int ni, int nj, int ng, int precision, int width, int rows, int* out) {
   const auto c = cato::tune_shapes(
-      ni, nj, ng, precision, cato::plan_shape(ni, nj, ng, precision, width, rows));
+      sms, ni, nj, ng, precision, cato::plan_shape(sms, ni, nj, ng, precision, width, rows));
   for (const auto& s : c) {
     put(s, out);
     out += 6;

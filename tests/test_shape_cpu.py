@@ -10,6 +10,7 @@ import pytest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 FP64, MIXED, MIXED_DF = 0, 1, 2
+SMS = 152
 Shape = namedtuple("Shape", "width threads rows block warps variant")
 GRIDS = [(64, 48), (128, 100), (200, 200), (256, 256), (400, 40), (448, 40), (512, 512), (1024, 1024),
          (4096, 4096), (3, 3), (5000, 3), (3, 5000), (100, 2000)]
@@ -42,16 +43,16 @@ def _grids():
 @pytest.mark.parametrize("ng", [2, 3])
 def test_a_plan_survives_get_and_set(rules, precision, ng):
     for ni, nj in _grids():
-        d = _call(rules.default_shape, ni, nj, ng, precision)
-        p = _call(rules.plan_shape, ni, nj, ng, precision, d.width, d.rows)
+        d = _call(rules.default_shape, SMS, ni, nj, ng, precision)
+        p = _call(rules.plan_shape, SMS, ni, nj, ng, precision, d.width, d.rows)
         assert p == d, (ni, nj)
 
 
 def test_the_register_budget_is_ignored_outside_fp64(rules):
     for ni, nj in GRIDS:
         for precision in (FP64, MIXED, MIXED_DF):
-            d = _call(rules.default_shape, ni, nj, 2, precision)
-            forms = [_call2(rules.launched_form, ni, nj, 2, precision, d.width, d.rows, v)
+            d = _call(rules.default_shape, SMS, ni, nj, 2, precision)
+            forms = [_call2(rules.launched_form, SMS, ni, nj, 2, precision, d.width, d.rows, v)
                      for v in (0, 1, 2)]
             if precision == FP64:
                 assert [v for v, _ in forms] == [0, 1, 2]
@@ -68,21 +69,31 @@ def _call2(fn, *args):
 @pytest.mark.parametrize("precision", [FP64, MIXED, MIXED_DF])
 @pytest.mark.parametrize("ni,nj", [(2, 2_097_121), (3, 4_194_240), (64, 2_100_000), (3, 1 << 30)])
 def test_tall_grids_fit_the_launch_limit(rules, precision, ni, nj):
-    d = _call(rules.default_shape, ni, nj, 2, precision)
+    d = _call(rules.default_shape, SMS, ni, nj, 2, precision)
     assert -(-nj // d.rows) <= 65535, d
 
 
 def _tune(rules, ni, nj, ng, precision, width, rows):
     out = (ctypes.c_int * 512)()
-    n = rules.tune_shapes(ni, nj, ng, precision, width, rows, out)
+    n = rules.tune_shapes(SMS, ni, nj, ng, precision, width, rows, out)
     return [Shape(*out[6 * k:6 * k + 6]) for k in range(n)]
 
 
 @pytest.mark.parametrize("precision", [FP64, MIXED, MIXED_DF])
 @pytest.mark.parametrize("ni,nj", [(60, 5000), (100, 2000), (119, 900), (96, 104), (700, 500)])
 def test_the_default_plan_is_a_tuning_candidate(rules, precision, ni, nj):
-    d = _call(rules.default_shape, ni, nj, 2, precision)
+    d = _call(rules.default_shape, SMS, ni, nj, 2, precision)
     shapes = _tune(rules, ni, nj, 2, precision, d.width, d.rows)
     assert d in shapes
     assert {s.variant for s in shapes} == ({0, 1, 2} if precision == FP64 else {0})
     assert len(set(shapes)) == len(shapes)
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED, MIXED_DF])
+def test_shapes_follow_the_number_of_sms(rules, precision):
+    # a grid of half the columns of tiles on half the SMs takes the same shape
+    for tiles in (2, 4, 10, 40, 300):
+        a, b = (_call(rules.default_shape, n * SMS, 60 * tiles * n, 120, 2, precision) for n in (1, 2))
+        assert a == b, tiles
+    shapes = {_call(rules.default_shape, n, 400, 200, 2, precision) for n in (20, 152, 1000)}
+    assert len(shapes) > 1
