@@ -183,30 +183,12 @@ static int rebuild(cato_batch* b) {
     BK(cudaGetDevice(&dev));
     BK(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev));
   }
-  // Rows per tile, at most the plan's.  FP32 strips hide their latency with neighbours: the most
-  // rows that leave five tiles per SM (served stream, 1.1 M cells: 1.93 ms per 16 steps at 8 rows,
-  // 3.06 at 32).  The edge-parallel tiles fill an SM with two: what counts is the share of the
-  // busiest SM, its tiles times the rows they hold and the edges they repeat (16 steps of an FP64
-  // sweep of 0.29 M cells: 19.9 ms at 4 rows with 9 tiles on an SM, 24.4 at 16 rows with 3; MLP5,
-  // 16 grids up to 512^2: 21.7 ms at 24 rows with 2, 25.0 at 16 with 3), over the multiples of four.
-  auto n_tiles = [&](int r) {
-    long long n = 0;
-    for (int i : order) {
-      const InstDesc& d = b->h_descs[i];
-      const int W = tile_columns(b) - 2 * d.ng, rr = std::min(r, d.nj);
-      n += (long long)((d.ni + W - 1) / W) * ((d.nj + rr - 1) / rr);
-    }
-    return n;
-  };
-  int tile_rows = b->rows;
-  if (b->prec == CATO_MIXED) {
-    while (tile_rows > 4 && n_tiles(tile_rows) < 5LL * b->sms)
-      tile_rows = std::max(4, tile_rows / 2);
-  } else {
-    auto share = [&](int r) { return (double)((n_tiles(r) + b->sms - 1) / b->sms) * (r + 1.2); };
-    for (int r = (tile_rows - 1) / 4 * 4; r >= 4; r -= 4)
-      if (share(r) < share(tile_rows)) tile_rows = r;
+  std::vector<BatchGrid> grids;
+  for (int i : order) {
+    const InstDesc& d = b->h_descs[i];
+    grids.push_back({d.ni, d.nj, tile_columns(b) - 2 * d.ng});
   }
+  const int tile_rows = batch_rows(b->sms, b->prec, b->rows, grids);
   b->tile_rows = tile_rows;
   for (int i : order) {
     const InstDesc& d = b->h_descs[i];

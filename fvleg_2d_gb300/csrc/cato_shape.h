@@ -125,4 +125,45 @@ inline std::vector<StageShape> tune_shapes(int sms, int ni, int nj, int ng, int 
   return out;
 }
 
+// Rows per tile of a batch, at most the plan's, for grids of ni x nj cells in strips of W columns.
+// FP32 strips hide their latency with neighbours: the most rows that leave five tiles per SM (served
+// stream, 1.1 M cells: 1.93 ms per 16 steps at 8 rows, 3.06 at 32).  The edge-parallel tiles fill an
+// SM with two: what counts is the share of the busiest SM, its tiles times their rows and 1.2 more
+// for what a tile repeats, its ghost rows and lowest edges (one wave of 304 tiles of 4 to 32 rows
+// takes k (r + c), c = 0.8 for FP64 HLLC and Roe, 1.1 with MLP5, 1.6 for double-float; 16 steps of
+// an FP64 sweep of 0.29 M cells: 19.9 ms at 4 rows with 9 tiles on an SM, 24.4 at 16 rows with 3;
+// MLP5, 16 grids up to 512^2: 21.7 ms at 24 rows with 2, 25.0 at 16 with 3), over the multiples of
+// four up to the tallest grid.
+struct BatchGrid {
+  int ni, nj, W;
+};
+inline int batch_rows(int sms, int precision, int plan_rows, const std::vector<BatchGrid>& grids) {
+  auto n_tiles = [&](int r) {
+    long long n = 0;
+    for (const BatchGrid& g : grids) {
+      const int rr = std::min(r, g.nj);
+      n += (long long)((g.ni + g.W - 1) / g.W) * ((g.nj + rr - 1) / rr);
+    }
+    return n;
+  };
+  int rows = plan_rows;
+  if (precision == CATO_MIXED) {
+    while (rows > 4 && n_tiles(rows) < 5LL * sms) rows = std::max(4, rows / 2);
+    return rows;
+  }
+  auto share = [&](int r) { return (double)((n_tiles(r) + sms - 1) / sms) * (r + 1.2); };
+  int tallest = 1;
+  for (const BatchGrid& g : grids) tallest = std::max(tallest, g.nj);
+  rows = std::min(rows, (int)(((long long)tallest + 3) / 4 * 4));
+  double least = share(rows);
+  for (int r = (rows - 1) / 4 * 4; r >= 4; r -= 4) {
+    const double x = share(r);
+    if (x < least) {
+      least = x;
+      rows = r;
+    }
+  }
+  return rows;
+}
+
 }  // namespace cato

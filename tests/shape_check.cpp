@@ -31,4 +31,9 @@ int tune_shapes(int sms, int ni, int nj, int ng, int precision, int width, int r
   }
   return (int)c.size();
 }
+int batch_rows(int sms, int precision, int plan_rows, int n, int W, const int* ni, const int* nj) {
+  std::vector<cato::BatchGrid> g;
+  for (int k = 0; k < n; ++k) g.push_back({ni[k], nj[k], W});
+  return cato::batch_rows(sms, precision, plan_rows, g);
+}
 }

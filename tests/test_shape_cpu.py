@@ -97,3 +97,18 @@ def test_shapes_follow_the_number_of_sms(rules, precision):
         assert a == b, tiles
     shapes = {_call(rules.default_shape, n, 400, 200, 2, precision) for n in (20, 152, 1000)}
     assert len(shapes) > 1
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED_DF])
+def test_batch_rows_are_bounded_by_the_tallest_grid(rules, precision):
+    rng = random.Random(5)
+    grids = [(rng.randint(8, 512), rng.randint(8, 512)) for _ in range(2000)]
+    ni = (ctypes.c_int * len(grids))(*(g[0] for g in grids))
+    nj = (ctypes.c_int * len(grids))(*(g[1] for g in grids))
+    for n in (1, 3, 40, 2000):
+        tall = -(-max(nj[:n]) // 4) * 4
+        # a search over every multiple of four up to 2^31 would not end
+        rows = [rules.batch_rows(SMS, precision, plan, n, 60, ni, nj)
+                for plan in (tall, tall + 1, 100_000, 2**31 - 1)]
+        assert len(set(rows)) == 1 and 4 <= rows[0] <= tall, (n, rows)
+    assert rules.batch_rows(SMS, precision, 3, 40, 60, ni, nj) == 3
