@@ -140,6 +140,99 @@ static void check_roe_sensor(long n) {
     }
 }
 
+// the TVD2 edge values that divide only where the ratio itself is needed
+static void check_tvd2(long n) {
+  for (const auto& r : kRanges)
+    for (long i = 0; i < n; ++i) {
+      double q[4];
+      stencil(r.kind, r.lo, r.hi, q);
+      const int lim = (int)(i % 3);
+      const EdgePair a = recon_tvd2_f64(lim, q[0], q[1], q[2], q[3]);
+      EdgePair b;
+      recon_tvd2<double>(lim, q[0], q[1], q[2], q[3], b.L, b.R);
+      ++tested;
+      if (same(a.L, b.L) && same(a.R, b.R)) continue;
+      if (bad++ < 3)
+        printf("tvd2 limiter %d %.17g %.17g %.17g %.17g: %.17g %.17g, general form %.17g %.17g\n", lim,
+               q[0], q[1], q[2], q[3], a.L, a.R, b.L, b.R);
+    }
+}
+
+// a bit pattern: the exponents 0 to 2047 in turn, either sign, and significands at random, near
+// either end, or with few bits set
+static uint64_t pattern(long i) {
+  constexpr uint64_t frac = 0x000fffffffffffffULL;
+  uint64_t m = rng() & frac;
+  switch (rng() % 5) {
+    case 0: m &= 0xfff; break;
+    case 1: m = frac - (m & 0xfff); break;
+    case 2: m = (rng() & 1) ? 0 : frac; break;
+    case 3: m = (1ULL << (rng() % 52)) | (1ULL << (rng() % 52)); break;
+    default: break;
+  }
+  return ((rng() & 1) << 63) | ((uint64_t)(i & 2047) << 52) | m;
+}
+
+static void check_sums(long n, bool one) {
+  for (long i = 0; i < 10 * n; ++i) {
+    uint64_t u = pattern(i);
+    if (one && i % 2) u = (u & 0x000fffffffffffffULL) | ((uint64_t)(988 + i / 2 % 40) << 52);
+    const double x = bit_cast<double>(u), y = one ? 1.0 + x : x + 1e-16;
+    bool ok;
+    const uint64_t r = one ? intdiv::one_plus_bits(u, ok) : intdiv::add_1em16_bits(u, ok);
+    if (!ok) continue;
+    ++tested;
+    if (r == bit_cast<uint64_t>(y)) continue;
+    if (bad++ < 3) printf("%a: %a, sum %a\n", x, bit_cast<double>(r), y);
+  }
+}
+
+static void check_to_df(long n) {
+  for (long i = 0; i < 10 * n; ++i) {
+    const double d = bit_cast<double>(pattern(i));
+    const df a = to_df(d), b = to_df_any(d);
+    ++tested;
+    if (same(a.hi, b.hi) && same(a.lo, b.lo)) continue;
+    if (bad++ < 3) printf("to_df %a: %a %a, general form %a %a\n", d, a.hi, a.lo, b.hi, b.lo);
+  }
+}
+
+// exact but for denormals, which become zeros
+static void check_f2d(long n) {
+  for (long i = 0; i < 10 * n; ++i) {
+    uint32_t u = (uint32_t)rng();
+    if (i % 4 == 1) u = (u & 0x80000000u) | ((uint32_t)(i / 4 % 256) << 23);
+    if (i % 4 == 2) u |= 0x007fffffu;
+    if (i % 4 == 3) u = (u & 0x80000007u) + ((uint32_t)(rng() % 4 * 85) << 23);
+    const float f = bit_cast<float>(u);
+    const double d = std::fabs(f) < FLT_MIN ? std::copysign(0.0, f) : (double)f;
+    ++tested;
+    if (!same(f2d_int(f), d) && bad++ < 3) printf("f2d_int %a: %a\n", f, f2d_int(f));
+  }
+}
+
+// normal operands with a normal quotient (one just below the normal range can round into it)
+static void check_div_normal(long n) {
+  auto normal = [](double x) { return std::isnormal(x); };
+  auto in_range = [](double q) { return q >= 2.0 * DBL_MIN && q <= DBL_MAX; };
+  for (long i = 0; i < 5 * n; ++i) {
+    double x[4];
+    for (double& v : x) v = bit_cast<double>(pattern((long)(rng() % 2048)));
+    if (i % 2)
+      for (double& v : x) {
+        int e;
+        v = std::ldexp(std::frexp(v, &e), (int)(rng() % 60) - 30);
+      }
+    if (!normal(x[0]) || !normal(x[1]) || !normal(x[2]) || !normal(x[3])) continue;
+    const double q = std::fabs(x[0] / x[1]), p = std::fabs(x[2] / x[3]);
+    if (!in_range(q) || !in_range(p)) continue;
+    const D2 two = div_normal2(x[0], x[1], x[2], x[3]);
+    ++tested;
+    const bool ok = same(div_normal(x[0], x[1]), q) && same(two.x, q) && same(two.y, p);
+    if (!ok && bad++ < 3) printf("div_normal %a / %a, %a / %a\n", x[0], x[1], x[2], x[3]);
+  }
+}
+
 int main(int argc, char** argv) {
   const long n = argc > 1 ? atol(argv[1]) : 400000;
   check_mlp<3>(n);
@@ -148,5 +241,17 @@ int main(int argc, char** argv) {
   report("mlp5");
   check_roe_sensor(n);
   report("roe_sensor");
+  check_tvd2(n);
+  report("tvd2");
+  check_sums(n, false);
+  report("add_1em16");
+  check_sums(n, true);
+  report("one_plus");
+  check_to_df(n);
+  report("to_df");
+  check_f2d(n);
+  report("f2d_int");
+  check_div_normal(n);
+  report("div_normal");
   return fail;
 }
