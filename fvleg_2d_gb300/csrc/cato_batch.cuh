@@ -60,7 +60,6 @@ __device__ __forceinline__ void batch_stage_args(InstDesc* d, const BatchStageAr
   A.status = &d->ctl.status;
   A.gamma = d->gamma;
   A.bc_p = d->bc_p;
-  A.cfl = d->cfl;
   A.G = d->G;
   // single-handle features the batch does not carry (configurations are rejected at add)
   A.pbc_edge = nullptr;

@@ -179,7 +179,6 @@ static StageArgs base_args(cato_handle* h) {
   A.status = &h->ctl->status;
   A.gamma = h->cfg.gamma;
   A.bc_p = h->cfg.bc_pressure;
-  A.cfl = h->cfg.cfl;
   A.G = h->G;
   return A;
 }

@@ -134,7 +134,6 @@ extern "C" int cato_gpu_solve_noalloc(const cato_config* cfg, double* rho, doubl
   A.status = reinterpret_cast<int*>(ctl + 2);
   A.gamma = cfg->gamma;
   A.bc_p = cfg->bc_pressure;
-  A.cfl = cfg->cfl;
   A.G = G;
   for (int k = 0; k < 4; ++k) {
     A.Pin[k] = prim[k];

@@ -959,14 +959,6 @@ static __device__ __noinline__ DfPair recon_tvd2_df(int lim, df qm1, df q0, df q
   return e;
 }
 
-template <>
-__device__ __forceinline__ void recon_tvd2<df>(int lim, df qm1, df q0, df qp1, df qp2, df& L,
-                                               df& Rr) {
-  const DfPair e = recon_tvd2_df(lim, qm1, q0, qp1, qp2);
-  L = e.L;
-  Rr = e.R;
-}
-
 // One side of the MLP limiter: the slope phi * dq, phi = max(0, min(alpha r, alpha, beta)),
 // for r = d0 / dq > 0 (the caller handles r <= 0).  min(alpha r, alpha) dq = alpha mq with
 // mq = (|d0| < |dq| ? d0 : dq) = min(r, 1) dq; beta dq is bdq.  dq is the own-side difference
@@ -1072,20 +1064,6 @@ static __device__ __noinline__ DfPair recon_mlp_df_ool(df qm2, df qm1, df q0, df
   DfPair e;
   recon_mlp_df<ORDER>(qm2, qm1, q0, qp1, qp2, qp3, t0p, t0m, t1p, t1m, e.L, e.R);
   return e;
-}
-template <>
-__device__ __forceinline__ void recon_mlp<df, 3>(df qm2, df qm1, df q0, df qp1, df qp2, df qp3,
-                                                 df t0p, df t0m, df t1p, df t1m, df& L, df& Rr) {
-  const DfPair e = recon_mlp_df_ool<3>(qm2, qm1, q0, qp1, qp2, qp3, t0p, t0m, t1p, t1m);
-  L = e.L;
-  Rr = e.R;
-}
-template <>
-__device__ __forceinline__ void recon_mlp<df, 5>(df qm2, df qm1, df q0, df qp1, df qp2, df qp3,
-                                                 df t0p, df t0m, df t1p, df t1m, df& L, df& Rr) {
-  const DfPair e = recon_mlp_df_ool<5>(qm2, qm1, q0, qp1, qp2, qp3, t0p, t0m, t1p, t1m);
-  L = e.L;
-  Rr = e.R;
 }
 
 // ---------------------------------------------------------------------------------------------

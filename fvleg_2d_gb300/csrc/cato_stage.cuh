@@ -51,7 +51,7 @@ struct StageArgs {
   unsigned long long* dt_min;  // bits of the smallest positive dt candidate (atomicMin)
   int* status;
   // physics
-  double gamma, cfl;
+  double gamma;
   double bc_p;             // outlet pressure (CATO_BC_OUTLET)
   // +x pressure input (CATO_BC_PRESSURE_INPUT): the ghost state (rho, u, p; v = 0) of rows
   // -pbc_ng .. nj+pbc_ng-1, written for this stage by pbc_edge_kernel
