@@ -1034,18 +1034,20 @@ constexpr bool batch_tvd_tile_of(int flux, int recon) {
 // Registers per thread of the FP32 kernels.
 // Single grids: HLLC, Roe and AUSM+-up with the TVD2 tile at 104 (the compiler's 113 to 135 leave
 // four 128-thread CTAs on an SM; 4096^2 HLLC 1469 -> 1307 us a step), the others the compiler's
-// choice, where a cap changes which products the assembler fuses and with it the rounding.
+// choice, where a cap changes which products the assembler fuses and with it the rounding.  Roe
+// with the rectilinear, source and pressure-input code spills at 104 and takes 128 (layered
+// 1500 x 1040: 261 us a step, 287 at 104, 255 uncapped; 3000 x 2010: 765, 862 and 922).
 // Batches: the general tile at 64 (+4.5 % on the batched workload), the TVD2 tile at 128.
-constexpr int f32_regs(int flux, int recon) {
+constexpr int f32_regs(int flux, int recon, bool ext) {
   const bool capped = flux == FLUX_HLLC || flux == FLUX_ROE || flux == FLUX_AUSM_UP;
-  return recon == 0 && capped ? 104 : 255;
+  return recon != 0 || !capped ? 255 : (ext && flux == FLUX_ROE ? 128 : 104);
 }
 constexpr int f32_batch_regs(int flux, int recon) {
   return batch_tvd_tile_of(flux, recon) ? 128 : 64;
 }
 
 template <int NG, int FLUX, int RECON, bool EXT>
-__global__ void __maxnreg__(f32_regs(FLUX, RECON))
+__global__ void __maxnreg__(f32_regs(FLUX, RECON, EXT))
     stage_kernel(const StageArgs A, const FluxConsts<float> K) {
   wait_previous();
   if (A.active && *A.active == 0) return;
