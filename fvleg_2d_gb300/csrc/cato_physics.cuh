@@ -781,7 +781,7 @@ static __device__ __noinline__ EdgePair recon_mlp_f64(double qm2, double qm1, do
     const float toth = __fdividef(s ? fn[0] : fn[1], s ? fe[0] : fe[1]);
     const float at = __fdividef(2.0f * fmaxf(1.0f, rf) * (1.0f + fmaxf(0.0f, toth * fx * if0)),
                                 1.0f + town);
-    const bool known = sure && at >= 0.0f && fabsf(toth * if0) < 1e24f && fabsf(fx * if0) < 1e24f;
+    const bool known = sure && at >= 0.0f && fmaxf(toth, fabsf(fx)) * fabsf(if0) < 1e24f;
     const float lo = known ? fmaxf(1.0f, fminf(2.0f, at * 0.999f)) : 1.0f;
     const float hi = known ? fmaxf(1.0f, fminf(2.0f, at * 1.001f)) : 2.0f;
     const float db = ORDER == 5 && fabsf(fy * ifq) >= 1e24f ? INFINITY : 1e-3f * bm;
