@@ -18,7 +18,7 @@ def test_result_is_independent_of_the_shape(precision, ni, nj, limiter, flux):
     cfg = _cfg(ni, nj, limiter, flux, precision)
     prims = random_prims(cfg, np.random.default_rng(ni * 100 + nj))
     states = []
-    for plan in (None, (64, 1), (64, 2), (96, 3), (128, 7), (256, 30)):
+    for plan in (None, (64, 1), (64, 2), (96, 3), (128, 7), (192, 5), (224, 9), (256, 30)):
         f = Fluid(cfg).initialize(*prims)
         if plan:
             f.set_plan(*plan)
