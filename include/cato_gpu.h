@@ -290,7 +290,7 @@ int cato_gpu_run_timed(cato_handle* h, int64_t n_steps, float* total_ms, float* 
 /* Work decomposition of the stage kernel (the autotuner's knobs): CTA width `threads` (a
  * multiple of 32 in [64, 256], including 2*n_ghost halo columns; the FP64 and double-float
  * kernels, which put several warps on a column, take half of it in columns) and rows marched per
- * CTA. */
+ * CTA.  Setting what cato_gpu_get_plan gives keeps the launch as it is. */
 int cato_gpu_set_plan(cato_handle* h, int32_t threads, int32_t rows_per_cta);
 int cato_gpu_get_plan(const cato_handle* h, int32_t* threads, int32_t* rows_per_cta);
 
