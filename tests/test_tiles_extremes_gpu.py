@@ -48,3 +48,38 @@ def test_wide_magnitudes_equal_the_oracle(oracle, limiter, lo, hi):
     got = FluxSolver(cfg).solve(*[p.copy(order="F") for p in prims])
     for k in range(4):
         np.testing.assert_array_equal(got[k], want[k])
+
+
+@pytest.mark.parametrize("limiter", ["superbee", "van_leer", "MLP3", "MLP5"])
+@pytest.mark.parametrize("flux", ["AUSMPW+", "SLAU2", "SD-SLAU", "Roe", "AUSM+-up", "M-AUSMPW+"])
+@pytest.mark.parametrize("width", [2, 10, 60])
+def test_wild_states_equal_the_oracle(oracle, limiter, flux, width):
+    # magnitudes 2^-width .. 2^width next to each other: negative edge pressures, NaN, overflow
+    cfg = _cfg(97, 61, limiter, flux)
+    g = cfg.ghost_layers()
+    rng = np.random.default_rng(width)
+    prims = []
+    for k in range(4):
+        d = np.exp2(rng.uniform(-width, width, (cfg.ni, cfg.nj)))
+        if k in (1, 2):
+            d *= rng.choice([-1.0, 1.0, 0.0], d.shape, p=[0.4, 0.4, 0.2])
+        d[20:50, 10:40] = d[20, 10]  # a flat stretch
+        a = np.zeros(cfg.halo_shape, order="F")
+        a[g:g + cfg.ni, g:g + cfg.nj] = d
+        prims.append(a)
+    ref = oracle.OracleFluid(cfg)
+    ref.set_primitive(*prims)
+    f = Fluid(cfg).initialize(*prims)
+    want_code = ref.integrate(1e-6)
+    _, code = f.integrate(1e-6)
+    want, got = ref.state(), f.state(FIELDS)
+    f.close()
+    assert code == want_code
+    for k in FIELDS:
+        np.testing.assert_array_equal(got[k], want[k], err_msg=k)
+    for a in prims:  # and a residual with a NaN and an infinity among the values
+        a[g + 5, g + 7], a[g + 60, g + 30] = np.nan, np.inf
+    want = oracle.solve(cfg, *[p.copy(order="F") for p in prims])
+    got = FluxSolver(cfg).solve(*[p.copy(order="F") for p in prims])
+    for k in range(4):
+        np.testing.assert_array_equal(got[k], want[k])
